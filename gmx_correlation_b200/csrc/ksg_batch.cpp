@@ -214,6 +214,8 @@ gc_status autotune(BatchPlan& bp)
     for (auto& gp : bp.groups)
     {
         BatchGroup& g    = *gp;
+        if (g.fl.row_walk) // one shape: nothing to tune
+            continue;
         float      best = 1e30f;
         WalkConfig best_cfg;
         for (const WalkConfig& c : walk_candidates(g.maxT))

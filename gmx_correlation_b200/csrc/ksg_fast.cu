@@ -40,21 +40,11 @@
 #include "gc_common.cuh"
 #include "gc_internal.h"
 #include "ksg_exact_query.cuh"
+#include "ksg_device.cuh"
 #include "ksg_fast.h"
 #include "row_sort.cuh"
 
 namespace gc {
-
-__device__ __forceinline__ float dist3f(const float4 a, const float4 b)
-{
-    return fmaxf(fmaxf(fabsf(a.x - b.x), fabsf(a.y - b.y)), fabsf(a.z - b.z));
-}
-
-__device__ __forceinline__ double dist3d(const double* __restrict__ X64, int atom, int T, int i, int j)
-{
-    const double* r = X64 + (size_t)atom * 3 * T;
-    return fmax(fmax(fabs(r[i] - r[j]), fabs(r[T + i] - r[T + j])), fabs(r[2 * T + i] - r[2 * T + j]));
-}
 
 // One warp per atom: component midranges c = (min + max) / 2 (for the
 // min-shifted rows kraskov_prepare makes, max / 2), centred FP32 coordinates
@@ -88,21 +78,6 @@ __global__ void ksg_x32_kernel(const double* __restrict__ X64, int natoms, int T
         eps_atom[a] = __double2float_ru(R * (1.0 + 0x1p-40) * 0x1p-21) + 1e-30f;
 }
 
-// The descriptor owning task t: the largest d with prefix[d] <= t.
-__device__ __forceinline__ int batch_desc(const long long* __restrict__ prefix, int n, long long t)
-{
-    int lo = 0, hi = n - 1;
-    while (lo < hi)
-    {
-        const int mid = (lo + hi + 1) >> 1;
-        if (prefix[mid] <= t)
-            lo = mid;
-        else
-            hi = mid - 1;
-    }
-    return lo;
-}
-
 // One CTA per (atom, query) of the launch's query blocks: the row's T-1
 // marginal distances (self excluded), sorted ascending with their frames
 // (sort_row).
@@ -128,22 +103,6 @@ __global__ void __launch_bounds__(THREADS) ksg_rows_kernel(WalkBatch B)
 
 namespace {
 
-// One lane's view of a transposed sorted row (see WalkParams).
-struct LaneRow
-{
-    const float*    S;
-    const uint16_t* P;
-    size_t          gstride; // elements between consecutive 4-entry groups
-
-    __device__ __forceinline__ float  s(int m) const { return S[(size_t)(m >> 2) * gstride + (m & 3)]; }
-    __device__ __forceinline__ int    j(int m) const { return P[(size_t)(m >> 2) * gstride + (m & 3)]; }
-    __device__ __forceinline__ float4 s4(int g) const
-    {
-        return *reinterpret_cast<const float4*>(S + (size_t)g * gstride);
-    }
-    __device__ __forceinline__ uint2 j4(int g) const { return *reinterpret_cast<const uint2*>(P + (size_t)g * gstride); }
-};
-
 // Entry q (0..3) of a 4-entry group: its distance and its frame.
 __device__ __forceinline__ float f4get(const float4& v, int q)
 {
@@ -153,12 +112,6 @@ __device__ __forceinline__ float f4get(const float4& v, int q)
 __device__ __forceinline__ unsigned u2get16(const uint2& v, int q)
 {
     return q < 2 ? ((v.x >> (16 * q)) & 0xFFFFu) : ((v.y >> (16 * (q - 2))) & 0xFFFFu);
-}
-
-__device__ __forceinline__ LaneRow lane_row(const WalkParams& p, int atom, int iq)
-{
-    const size_t base = ((size_t)atom * (p.Lpad >> 2) * p.Qp + iq) * 4;
-    return LaneRow{p.S + base, p.P + base, (size_t)p.Qp * 4};
 }
 
 // Four independent binary searches advanced together, so their loads
@@ -201,16 +154,6 @@ __device__ __forceinline__ double dist3r(const double* __restrict__ r, int T, do
 constexpr int kScanCap = 1024; // row entries a backward scan may visit
 constexpr int kAmbCap  = 8;    // ambiguous entries ordered in FP64
 
-// Hand-over causes (WalkParams::reasons index).
-enum
-{
-    kReasonRange    = 2, // k-th value beyond the histogram's two octaves
-    kReasonBand     = 3, // band larger than kBandCap or inconsistent with the histogram
-    kReasonAmbig    = 4, // ambiguous set inconsistent or larger than kAmbCap
-    kReasonScan     = 5, // backward scan for the maxima exceeded kScanCap
-    kReasonPrefix   = 6  // count band reaches beyond the walked prefix
-};
-
 } // namespace
 
 namespace {
@@ -244,8 +187,10 @@ __device__ __forceinline__ LaneSetup lane_setup(const WalkParams& p, int a1, int
     u.o              = u.wx ? a2 : a1;
     u.rw             = u.wx ? ra : rb;
     u.ro             = u.wx ? rb : ra;
-    u.L              = u.wx ? Ra : Rb;
-    u.Lb             = __float_as_uint(u.L);
+    // bucket edges are multiples of 2^shift float ulps, the same for every
+    // pair: the lower bound is rounded down to one
+    u.Lb             = __float_as_uint(u.wx ? Ra : Rb) >> p.shift << p.shift;
+    u.L              = __uint_as_float(u.Lb);
     u.X32w           = u.wx ? xa : xb;
     u.X32o           = u.wx ? xb : xa;
     u.xw             = u.X32w[i];
@@ -302,14 +247,6 @@ __device__ __forceinline__ bool next_task(const WalkBatch& B, long long total, l
     tk.c                 = (int)(lt / p.pair_count);
     task_pair(p, (long)(lt - (long long)tk.c * p.pair_count), tk);
     return true;
-}
-
-// Walk result of one (pair, query): bucket of the k-th value, the number of
-// entries below that bucket, the walked length, and a hand-over cause.
-__device__ __forceinline__ unsigned long long pack_walk(int bstar, int prefix, int m_end, int reason)
-{
-    return (unsigned long long)(bstar & 0xFF) | ((unsigned long long)(prefix & 0xFFFF) << 8) |
-           ((unsigned long long)(m_end & 0xFFFF) << 24) | ((unsigned long long)(reason & 0xFF) << 40);
 }
 
 } // namespace

@@ -19,6 +19,13 @@ constexpr int kWalkBuckets = 128;      // per-lane histogram buckets
 #ifndef GC_BAND_CAP
 #define GC_BAND_CAP 20 // a build-time setting for timing other capacities
 #endif
+constexpr int kRwChunk     = 128;       // row walk: row entries staged at a time
+constexpr int kRwHistBytes  = kWalkBuckets * 32; // row walk: a warp's histogram
+constexpr int kRwStageBytes = kRwChunk * 5;      // row walk: a warp's staged entries
+constexpr int kRwMaxOffset  = 128; // row walk: largest window offset the 256 codes of a tile cover
+constexpr int kRwMaxAtoms   = 4096; // row walk: atoms the per-query ordering takes
+// Row walk: bytes of the code tile of T frames.
+__host__ __device__ inline size_t rw_tile_bytes(int T) { return ((size_t)T * 32 + 127) & ~(size_t)127; }
 constexpr int kBandCap     = GC_BAND_CAP; // band entries kept per lane
 constexpr int kBandSlotBytes = 14;     // v, s, d (f32), row position in its range (u16)
 constexpr uint32_t kHandOver = 0xFFFFFFFFu; // cnt value of a query handed to the exact kernel
@@ -52,6 +59,10 @@ struct WalkParams
     // (GC_VARIANT_HBM_GATHER: the walk reads the other marginal here)
     float* U;
     int    Tpad;
+    // full pair matrices walked row by row (row_walk.cuh): the block's atoms
+    // by ascending k-th distance, [Q][natoms] (atom, code of that distance);
+    // null where the walk with one query per lane runs
+    uint2* order;
 };
 
 // One launch over the query blocks of several trajectories (or of one): the
@@ -63,6 +74,8 @@ struct WalkBatch
     const long long*    rprefix; // [n + 1] row-sort tasks: natoms * Q per descriptor
     const long long*    wprefix; // [n + 1] walk tasks: ceil(groups / chunk) * pairs
     const long long*    fprefix; // [n + 1] finish tasks: query groups * pairs
+    const long long*    qprefix; // [n + 1] queries (row walk only)
+    const long long*    uprefix; // [n + 1] row-walk tasks: Q * ceil(natoms / 32)
     int                 n;
     int                 maxT;    // largest frame count (shared-memory layout)
     int                 maxK;    // largest k
@@ -95,6 +108,11 @@ cudaError_t launch_ksg_walk(const WalkBatch& b, int warps, bool staged, int sms,
                             bool gather_u = false, bool double_buffer = false);
 // Warps per CTA the double-buffered walk leaves room for (0: its rows do not fit).
 int walk_max_db_warps(int maxT);
+// The row walk (row_walk.cuh) of descriptors with an order array; queries:
+// qprefix[n], maxn: the most atoms of a descriptor.
+cudaError_t launch_ksg_row_walk(const WalkBatch& b, long long queries, int maxn, int sms, cudaStream_t s);
+// Warps per CTA of the row walk (0: the tile of maxT frames does not fit) and CTAs per SM.
+int row_walk_warps(int maxT, int* ctas);
 cudaError_t launch_ksg_finish(const WalkBatch& b, int sms, cudaStream_t s);
 // Exact FP64 statistics for every queued hand-over of the batch's
 // descriptors, then for any hand-over mark a queue could not hold (a scan of

@@ -29,6 +29,15 @@ int ksg_block_queries(int natoms, int T, double budget, int quantum, double extr
     return (int)q;
 }
 
+// The row walk holds 32 pairs of one atom in a warp: below 24 atoms most of
+// its lanes are idle; its window index 0 counts up to k - 1 entries in a byte;
+// its tile and a few warps' histograms have to fit in shared memory.
+static bool row_walk_fits(int natoms, int T, int k)
+{
+    int ctas = 0;
+    return natoms >= 24 && natoms <= gc::kRwMaxAtoms && k < 256 && gc::row_walk_warps(T, &ctas) > 0;
+}
+
 gc_status KsgTraj::create(int n, int nframes, int k, long pb, long pc, const int64_t* lst, const int2* d_ab, int q,
                           int tile, bool unsorted_rows, bool own_rows)
 {
@@ -71,6 +80,11 @@ gc_status KsgTraj::create(int n, int nframes, int k, long pb, long pc, const int
     GC_TRY(hq_len.alloc(1));
     GC_TRY(walk_elems.alloc(1));
     GC_TRY(reasons.alloc(8));
+    // the row walk takes whole pair lists (see row_walk_fits)
+    if (!lst && pb == 0 && pc == (long)n * (n - 1) / 2 && !unsorted_rows && row_walk_fits(n, nframes, k))
+        GC_TRY(order.alloc((size_t)Q * natoms));
+    else
+        order.reset();
     pair_tile = 0;
     return set_pair_tile(tile);
 }
@@ -137,6 +151,7 @@ WalkParams KsgTraj::desc(const double* X, uint32_t* cnt, int* status, int b) con
     w.reasons    = reasons.p;
     w.U          = U.p;
     w.Tpad       = Tpad;
+    w.order      = order.p;
     return w;
 }
 
@@ -172,15 +187,25 @@ gc_status KsgLaunch::build(const std::vector<std::vector<WalkParams>>& wave_desc
     std::vector<long long>  pre;
     std::vector<size_t>     dofs, pofs;
     int                     maxT = 0, maxK = 0;
+    row_walk  = !cfg.gather_u;
+    max_atoms = 0;
+    for (const auto& wv : wave_descs)
+        for (const WalkParams& d : wv)
+        {
+            row_walk  = row_walk && d.order != nullptr;
+            max_atoms = std::max(max_atoms, d.natoms);
+        }
     for (const auto& wv : wave_descs)
     {
         dofs.push_back(all.size());
         pofs.push_back(pre.size());
         long long r = 0, w = 0, f = 0;
-        std::vector<long long> rp{0}, wp{0}, fp{0};
+        std::vector<long long> rp{0}, wp{0}, fp{0}, qp{0}, up{0};
         for (const WalkParams& d : wv)
         {
             all.push_back(d);
+            qp.push_back(qp.back() + d.Q);
+            up.push_back(up.back() + (long long)d.Q * ((d.natoms + 31) / 32));
             maxT                 = std::max(maxT, d.T);
             maxK                 = std::max(maxK, d.K);
             const long long grp  = (d.Q + 31) / 32;
@@ -195,6 +220,8 @@ gc_status KsgLaunch::build(const std::vector<std::vector<WalkParams>>& wave_desc
         pre.insert(pre.end(), rp.begin(), rp.end());
         pre.insert(pre.end(), wp.begin(), wp.end());
         pre.insert(pre.end(), fp.begin(), fp.end());
+        pre.insert(pre.end(), qp.begin(), qp.end());
+        pre.insert(pre.end(), up.begin(), up.end());
     }
     const size_t tofs = all.size();
     all.insert(all.end(), traj_descs.begin(), traj_descs.end());
@@ -205,6 +232,7 @@ gc_status KsgLaunch::build(const std::vector<std::vector<WalkParams>>& wave_desc
     GC_TRY_CUDA(cudaMemcpy(prefix.p, pre.data(), sizeof(long long) * pre.size(), cudaMemcpyHostToDevice));
     waves.clear();
     wave_rows.clear();
+    wave_queries.clear();
     for (size_t v = 0; v < wave_descs.size(); ++v)
     {
         const int  n = (int)wave_descs[v].size();
@@ -213,6 +241,8 @@ gc_status KsgLaunch::build(const std::vector<std::vector<WalkParams>>& wave_desc
         b.rprefix  = prefix.p + pofs[v];
         b.wprefix  = b.rprefix + (n + 1);
         b.fprefix  = b.wprefix + (n + 1);
+        b.qprefix  = b.fprefix + (n + 1);
+        b.uprefix  = b.qprefix + (n + 1);
         b.n        = n;
         b.maxT     = maxT;
         b.maxK     = maxK;
@@ -220,6 +250,7 @@ gc_status KsgLaunch::build(const std::vector<std::vector<WalkParams>>& wave_desc
         b.counter  = counters.p + 2 * v;
         waves.push_back(b);
         wave_rows.push_back(pre[pofs[v] + n]);
+        wave_queries.push_back(pre[pofs[v] + 3 * ((size_t)n + 1) + n]);
     }
     fix      = WalkBatch{};
     fix.d    = descs.p + tofs;
@@ -239,8 +270,14 @@ gc_status KsgLaunch::enqueue(int sms, cudaStream_t s, int first_wave, int last_w
     for (int v = first_wave; v <= last_wave; ++v)
     {
         GC_TRY_CUDA(launch_ksg_rows(waves[(size_t)v], wave_rows[(size_t)v], s));
-        GC_TRY_CUDA(launch_ksg_walk(waves[(size_t)v], cfg.walk_warps, cfg.staged, sms, s, cfg.gather_u,
-                                    cfg.double_buf));
+        if (row_walk)
+        {
+            GC_TRY_CUDA(launch_ksg_row_walk(waves[(size_t)v], wave_queries[(size_t)v], max_atoms, sms, s));
+            ++launches;
+        }
+        else
+            GC_TRY_CUDA(launch_ksg_walk(waves[(size_t)v], cfg.walk_warps, cfg.staged, sms, s, cfg.gather_u,
+                                        cfg.double_buf));
         GC_TRY_CUDA(launch_ksg_finish(waves[(size_t)v], sms, s));
         launches += 3;
     }

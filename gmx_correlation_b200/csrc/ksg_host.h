@@ -43,6 +43,7 @@ struct KsgTraj
     PoolBuf<int>                pair_order;
     PoolBuf<float>              U; // unsorted distance rows (GC_VARIANT_HBM_GATHER only)
     int                         Tpad = 0;
+    PoolBuf<uint2>              order; // the row walk's atom order (empty where it does not run)
 
     // Sizes the workspace for query blocks of Q frames (a multiple of 32, or T).
     // own_rows false: the sorted rows live elsewhere (a batch's shared arena)
@@ -77,8 +78,11 @@ struct KsgLaunch
     DevBuf<unsigned long long> counters;
     std::vector<WalkBatch>     waves;
     std::vector<long long>     wave_rows;
+    std::vector<long long>     wave_queries; // row walk: queries of the wave
     WalkBatch                  fix{};
     WalkConfig                 cfg;
+    bool                       row_walk = false; // the wave's walk is launch_ksg_row_walk
+    int                        max_atoms = 0;
     int                        launches = 0;
 
     gc_status build(const std::vector<std::vector<WalkParams>>& wave_descs, const std::vector<WalkParams>& traj_descs,
