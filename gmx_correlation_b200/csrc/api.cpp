@@ -358,7 +358,7 @@ gc_status plan_run(gc_ksg_plan* p, const double* d_xyz, double* d_pair_mi, cudaS
             p->launches += 1;
         }
         GC_TRY_CUDA(cudaEventRecord(p->ev1, s));
-        gc::launch_ksg_finalize(p->cnt.p, p->pair_count, p->T, p->K, p->psi.p, d_pair_mi, s,
+        gc::launch_ksg_finalize(p->cnt.p, p->pair_count, p->T, p->K, p->psi.p, d_pair_mi, p->sms, s,
                                 p->wide ? p->cnt.p + (size_t)p->T * p->pair_count : nullptr);
         p->launches += 1;
     }
@@ -779,7 +779,7 @@ gc_status gc_ksg_pair(const double* rows6, int nframes, int k, const double* psi
     GC_TRY_CUDA(cudaMemcpyAsync(d_X.p, rows6 + (size_t)3 * T, sizeof(double) * 3 * T, cudaMemcpyHostToDevice, ss.s));
     GC_TRY_CUDA(cudaMemcpyAsync(d_psi.p, psi, sizeof(double) * (T + 1), cudaMemcpyHostToDevice, ss.s));
     gc::launch_ksg_exact(d_X.p, T, k, 0, 1, d_cnt.p, ss.s, nullptr, wide ? d_cnt.p + T : nullptr);
-    gc::launch_ksg_finalize(d_cnt.p, 1, T, k, d_psi.p, d_mi.p, ss.s, wide ? d_cnt.p + T : nullptr);
+    gc::launch_ksg_finalize(d_cnt.p, 1, T, k, d_psi.p, d_mi.p, 148, ss.s, wide ? d_cnt.p + T : nullptr);
     GC_TRY_CUDA(cudaGetLastError());
     GC_TRY_CUDA(cudaMemcpyAsync(mi, d_mi.p, sizeof(double), cudaMemcpyDeviceToHost, ss.s));
     GC_TRY_CUDA(cudaStreamSynchronize(ss.s));

@@ -120,7 +120,7 @@ gc_status te_enqueue_all(void* ctx, cudaStream_t s)
         GC_TRY(g->enqueue(bp.sms, s));
     for (auto& ip : bp.items)
         if (ip->active)
-            GC_TRY_CUDA(gc::launch_te_reduce(ip->tt->cnt.p, ip->natoms, ip->tt->Nv, ip->K, ip->tt->psi.p, ip->te.p, s));
+            GC_TRY_CUDA(gc::launch_te_reduce(ip->tt->cnt.p, ip->natoms, ip->tt->Nv, ip->K, ip->tt->psi.p, ip->te.p, bp.sms, s));
     GC_TRY_CUDA(cudaGetLastError());
     return GC_OK;
 }

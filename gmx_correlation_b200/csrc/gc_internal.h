@@ -42,7 +42,7 @@ void launch_ksg_exact(const double* X, int T, int K, long pair_begin, long pair_
 
 // MI per pair from the per-query counts, summed in frame order as mir_xnyn does.
 void launch_ksg_finalize(const uint32_t* cnt, long pair_count, int T, int K, const double* psi,
-                         double* pair_mi, cudaStream_t s, const uint32_t* cnt_y = nullptr);
+                         double* pair_mi, int sms, cudaStream_t s, const uint32_t* cnt_y = nullptr);
 
 // ---- Transfer entropy ------------------------------------------------------
 // xyz [natoms][T][3] -> XT [3*natoms][T] (component-major copy, raw values),

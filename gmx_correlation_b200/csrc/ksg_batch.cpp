@@ -190,7 +190,7 @@ gc_status enqueue_all(BatchPlan& bp, cudaStream_t s)
     for (auto& g : bp.groups)
         GC_TRY(g->fl.enqueue(bp.sms, s));
     for (auto& b : bp.t)
-        gc::launch_ksg_finalize(b->cnt.p, b->pairs, b->T, b->K, b->psi.p, b->mi.p, s);
+        gc::launch_ksg_finalize(b->cnt.p, b->pairs, b->T, b->K, b->psi.p, b->mi.p, bp.sms, s);
     GC_TRY_CUDA(cudaGetLastError());
     return GC_OK;
 }

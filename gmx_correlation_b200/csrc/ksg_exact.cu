@@ -18,6 +18,7 @@
 #include "gc_common.cuh"
 #include "gc_internal.h"
 #include "ksg_exact_query.cuh"
+#include "ordered_sum.cuh"
 
 namespace gc {
 
@@ -178,48 +179,25 @@ __global__ void __launch_bounds__(kExactWarps * 32)
 // MI = psi[N] + (psi[K] - 1/K) - (1/N) * sum_i (psi[n_x,i] + psi[n_y,i]),
 // summed over i in frame order (lib/kraskov.cpp:1262, :1303-1318).
 // cnt_y != nullptr: wide counts (n_x in cnt, n_y in cnt_y, 32 bits each).
-__global__ void ksg_finalize_kernel(const uint32_t* __restrict__ cnt, const uint32_t* __restrict__ cnt_y,
-                                    long pair_count, int T, int K, const double* __restrict__ psi,
-                                    double* __restrict__ pair_mi)
+__global__ void __launch_bounds__(kSumThreads)
+    ksg_finalize_kernel(const uint32_t* __restrict__ cnt, const uint32_t* __restrict__ cnt_y, long pair_count, int T,
+                        int K, int P, const double* __restrict__ psi, double* __restrict__ pair_mi)
 {
-    const long p = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    if (p >= pair_count)
-        return;
-    if (cnt_y)
+    const long   p0   = (long)blockIdx.x * P;
+    const int    live = (int)min((long)P, pair_count - p0);
+    const size_t base = (size_t)p0 * T;
+    const double s    = ordered_sums(P, live, T, [&](int p, int f) {
+        const size_t at = base + (size_t)p * T + f;
+        if (cnt_y)
+            return __dadd_rn(psi[cnt[at]], psi[cnt_y[at]]);
+        const uint32_t c = cnt[at];
+        return __dadd_rn(psi[c & 0xFFFFu], psi[c >> 16]);
+    });
+    if ((int)threadIdx.x < live)
     {
-        double s = 0.0;
-        for (int i = 0; i < T; ++i)
-            s = __dadd_rn(s, __dadd_rn(psi[cnt[(size_t)p * T + i]], psi[cnt_y[(size_t)p * T + i]]));
-        const double phiK = __dsub_rn(psi[K], __ddiv_rn(1.0, (double)K));
-        pair_mi[p]        = __dsub_rn(__dadd_rn(psi[T], phiK), __ddiv_rn(s, (double)T));
-        return;
+        const double phiK         = __dsub_rn(psi[K], __ddiv_rn(1.0, (double)K));
+        pair_mi[p0 + threadIdx.x] = __dsub_rn(__dadd_rn(psi[T], phiK), __ddiv_rn(s, (double)T));
     }
-    // 16 frames' counts and digamma terms are fetched together; the sum
-    // itself stays sequential in frame order
-    double s = 0.0;
-    int    i = 0;
-    for (; i + 16 <= T; i += 16)
-    {
-        uint32_t c[16];
-        double   term[16];
-#pragma unroll
-        for (int u = 0; u < 16; ++u)
-            c[u] = cnt[(size_t)p * T + i + u];
-#pragma unroll
-        for (int u = 0; u < 16; ++u)
-            term[u] = __dadd_rn(psi[c[u] & 0xFFFFu], psi[c[u] >> 16]);
-#pragma unroll
-        for (int u = 0; u < 16; ++u)
-            s = __dadd_rn(s, term[u]);
-    }
-    for (; i < T; ++i)
-    {
-        const uint32_t c = cnt[(size_t)p * T + i];
-        s                = __dadd_rn(s, __dadd_rn(psi[c & 0xFFFFu], psi[c >> 16]));
-    }
-    const double phiK = __dsub_rn(psi[K], __ddiv_rn(1.0, (double)K));
-    const double dxy2 = __ddiv_rn(s, (double)T);
-    pair_mi[p]        = __dsub_rn(__dadd_rn(psi[T], phiK), dxy2);
 }
 
 void launch_ksg_prepare(const double* xyz, int natoms, int T, double* X, int* status, cudaStream_t s)
@@ -256,10 +234,11 @@ void launch_ksg_exact(const double* X, int T, int K, long pair_begin, long pair_
 }
 
 void launch_ksg_finalize(const uint32_t* cnt, long pair_count, int T, int K, const double* psi,
-                         double* pair_mi, cudaStream_t s, const uint32_t* cnt_y)
+                         double* pair_mi, int sms, cudaStream_t s, const uint32_t* cnt_y)
 {
-    ksg_finalize_kernel<<<(unsigned)((pair_count + 127) / 128), 128, 0, s>>>(cnt, cnt_y, pair_count, T, K, psi,
-                                                                            pair_mi);
+    const int P = sums_per_cta(pair_count, sms);
+    ksg_finalize_kernel<<<(unsigned)((pair_count + P - 1) / P), kSumThreads, 0, s>>>(cnt, cnt_y, pair_count, T, K, P,
+                                                                                    psi, pair_mi);
 }
 
 } // namespace gc

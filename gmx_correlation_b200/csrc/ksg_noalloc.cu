@@ -135,7 +135,7 @@ extern "C" gc_status gc_ksg_pair_mi_noalloc(const double* d_xyz, int natoms, int
         noalloc_psi_kernel<<<1, 1, 0, s>>>(psi, nframes);
         gc::launch_ksg_prepare(d_xyz, natoms, nframes, X, status, s);
         gc::launch_ksg_exact(X, nframes, k, 0, npairs, cnt, s);
-        gc::launch_ksg_finalize(cnt, npairs, nframes, k, psi, d_pair_mi, s);
+        gc::launch_ksg_finalize(cnt, npairs, nframes, k, psi, d_pair_mi, 148, s);
         e = cudaGetLastError();
     }
     int st = 0;

@@ -361,7 +361,7 @@ gc_status gc_te_plan_run(gc_te_plan* p, const double* d_xyz, double* d_te, void*
     {
         GC_TRY(p->tl.enqueue(p->sms, s));
         GC_TRY_CUDA(cudaEventRecord(p->ev1, s));
-        GC_TRY_CUDA(gc::launch_te_reduce(p->tt.cnt.p, n, p->Nv, p->K, p->tt.psi.p, d_te, s));
+        GC_TRY_CUDA(gc::launch_te_reduce(p->tt.cnt.p, n, p->Nv, p->K, p->tt.psi.p, d_te, p->sms, s));
         p->launches += p->tl.launches + 1;
     }
     else

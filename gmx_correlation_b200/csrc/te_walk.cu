@@ -34,6 +34,7 @@
 #include "gc_common.cuh"
 #include "gc_internal.h"
 #include "ksg_fast.h"
+#include "ordered_sum.cuh"
 #include "row_sort.cuh"
 #include "te_exact_query.cuh"
 #include "te_walk.h"
@@ -1115,43 +1116,30 @@ __global__ void __launch_bounds__(256) te_fixup_scan_kernel(TeBatch B)
 // te_sum += psi_k + psi[n_xp + 1] - psi[n_xfxp + 1] - psi[n_ypxp + 1] with
 // the counts clamped to N_valid, in query order; te_sum / N_valid
 // (lib/transfer_entropy.cpp:188-204).  cnt is pair-major [q][Nv].
-__global__ void te_reduce_kernel(const uint2* __restrict__ cnt, int natoms, int Nv, int K,
-                                 const double* __restrict__ psi, double* __restrict__ te_mat)
+__global__ void __launch_bounds__(kSumThreads)
+    te_reduce_kernel(const uint2* __restrict__ cnt, int natoms, int Nv, int K, int P, const double* __restrict__ psi,
+                     double* __restrict__ te_mat)
 {
-    const long npairs = (long)natoms * (natoms - 1);
-    const long q      = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    if (q >= npairs)
-        return;
-    const uint2* c   = cnt + (size_t)q * Nv;
-    const double pk  = psi[K];
-    double       sum = 0.0;
-    auto term = [&](uint2 v) {
-        const int xp = min((int)(v.x & 0xFFFFu), Nv);
-        const int xf = min((int)(v.x >> 16), Nv);
-        const int yp = min((int)v.y, Nv);
+    const long   npairs = (long)natoms * (natoms - 1);
+    const long   q0     = (long)blockIdx.x * P;
+    const int    live   = (int)min((long)P, npairs - q0);
+    const uint2* c      = cnt + (size_t)q0 * Nv;
+    const double pk     = psi[K];
+    const double sum    = ordered_sums(P, live, Nv, [&](int p, int f) {
+        const uint2 v  = c[(size_t)p * Nv + f];
+        const int   xp = min((int)(v.x & 0xFFFFu), Nv);
+        const int   xf = min((int)(v.x >> 16), Nv);
+        const int   yp = min((int)v.y, Nv);
         return __dsub_rn(__dsub_rn(__dadd_rn(pk, psi[xp + 1]), psi[xf + 1]), psi[yp + 1]);
-    };
-    int i = 0;
-    for (; i + 8 <= Nv; i += 8)
+    });
+    if ((int)threadIdx.x < live)
     {
-        uint2  v[8];
-        double t[8];
-#pragma unroll
-        for (int u = 0; u < 8; ++u)
-            v[u] = c[i + u];
-#pragma unroll
-        for (int u = 0; u < 8; ++u)
-            t[u] = term(v[u]);
-#pragma unroll
-        for (int u = 0; u < 8; ++u)
-            sum = __dadd_rn(sum, t[u]);
+        const long q  = q0 + threadIdx.x;
+        const int  a1 = (int)(q / (natoms - 1));
+        const int  rr = (int)(q - (long)a1 * (natoms - 1));
+        const int  a2 = rr < a1 ? rr : rr + 1;
+        te_mat[(size_t)a1 * natoms + a2] = __ddiv_rn(sum, (double)Nv);
     }
-    for (; i < Nv; ++i)
-        sum = __dadd_rn(sum, term(c[i]));
-    const int a1 = (int)(q / (natoms - 1));
-    const int rr = (int)(q - (long)a1 * (natoms - 1));
-    const int a2 = rr < a1 ? rr : rr + 1;
-    te_mat[(size_t)a1 * natoms + a2] = __ddiv_rn(sum, (double)Nv);
 }
 
 // ---------------------------------------------------------------------------
@@ -1249,11 +1237,12 @@ cudaError_t launch_te_fixup(const TeBatch& b, int sms, cudaStream_t s)
     return cudaGetLastError();
 }
 
-cudaError_t launch_te_reduce(const uint2* cnt, int natoms, int Nv, int K, const double* psi, double* te_mat,
+cudaError_t launch_te_reduce(const uint2* cnt, int natoms, int Nv, int K, const double* psi, double* te_mat, int sms,
                              cudaStream_t s)
 {
     const long npairs = (long)natoms * (natoms - 1);
-    te_reduce_kernel<<<(unsigned)((npairs + 127) / 128), 128, 0, s>>>(cnt, natoms, Nv, K, psi, te_mat);
+    const int  P      = sums_per_cta(npairs, sms);
+    te_reduce_kernel<<<(unsigned)((npairs + P - 1) / P), kSumThreads, 0, s>>>(cnt, natoms, Nv, K, P, psi, te_mat);
     return cudaGetLastError();
 }
 

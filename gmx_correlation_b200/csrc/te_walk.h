@@ -81,7 +81,7 @@ cudaError_t launch_te_count(const TeBatch& b, int warps, bool staged, int sms, c
 cudaError_t launch_te_fixup(const TeBatch& b, int sms, cudaStream_t s);
 // te[a1 * natoms + a2] = mean over qi of psi[k] + psi[n_xp + 1] - psi[n_xfxp + 1]
 // - psi[n_ypxp + 1], summed in query order (lib/transfer_entropy.cpp:195-204).
-cudaError_t launch_te_reduce(const uint2* cnt, int natoms, int Nv, int K, const double* psi, double* te_mat,
+cudaError_t launch_te_reduce(const uint2* cnt, int natoms, int Nv, int K, const double* psi, double* te_mat, int sms,
                              cudaStream_t s);
 
 } // namespace gc
