@@ -158,6 +158,7 @@ struct gc_ksg_plan
     cudaStream_t stream = nullptr;
     PoolBuf<double>   X, psi;
     PoolBuf<uint32_t> cnt;
+    PoolBuf<double>  brute; // scratch of the FP32 brute force (trajectories too long for sorted rows)
     DevBuf<int>      status;
     DevBuf<int2>     pair_ab; // explicit pair list as (a1, a2), empty for a range
     int              launches = 0;
@@ -280,8 +281,12 @@ gc_status gc_ksg_plan_create(int natoms, int nframes, int k, const gc_opts* opts
     GC_TRY(p->status.alloc(1));
     GC_TRY_CUDA(cudaDeviceGetAttribute(&p->sms, cudaDevAttrMultiProcessorCount, p->device));
     // The fast path sorts each marginal row in shared memory (<= 16384
-    // frames); longer trajectories use the exact kernels throughout.
+    // frames); longer trajectories use brute force, FP32 with FP64 repair
+    // (8 atoms x 20,001 frames, k = 50: 29 ms, the exact FP64 kernel 282 ms)
+    // unless the FP64 path is asked for.
     p->fast = o.path != GC_PATH_EXACT_FP64 && nframes - 1 <= 16384 && pc > 0;
+    if (!p->fast && o.path != GC_PATH_EXACT_FP64)
+        GC_TRY(p->brute.alloc(gc::ksg_brute_scratch(natoms) / sizeof(double) + 1));
     const std::vector<double> psi = digamma_table(nframes);
     GC_TRY_CUDA(cudaMemcpy(p->psi.p, psi.data(), sizeof(double) * psi.size(), cudaMemcpyHostToDevice));
     if (o.pair_list && pc > 0)
@@ -350,6 +355,12 @@ gc_status plan_run(gc_ksg_plan* p, const double* d_xyz, double* d_pair_mi, cudaS
             GC_TRY(p->ft.clear(s));
             GC_TRY(p->fl.enqueue(p->sms, s));
             p->launches += 1 + p->fl.launches;
+        }
+        else if (p->brute.p)
+        {
+            gc::launch_ksg_brute(p->X.p, p->natoms, p->T, p->K, p->pair_begin, p->pair_count, p->cnt.p, p->brute.p, p->sms,
+                                 s, p->pair_ab.p, p->wide ? p->cnt.p + (size_t)p->T * p->pair_count : nullptr);
+            p->launches += 2;
         }
         else
         {
@@ -768,8 +779,11 @@ gc_status gc_ksg_pair(const double* rows6, int nframes, int k, const double* psi
     GC_TRY(ss.init(o.stream));
     // Two-atom system whose single pair (1, 0) has a1 = atom 1: the
     // x-marginal (first three rows, the grid's first axis) goes to atom 1.
-    DevBuf<double>   d_X, d_psi, d_mi;
+    int cur = 0;
+    GC_TRY_CUDA(cudaGetDevice(&cur));
+    DevBuf<double>   d_X, d_psi, d_mi, d_brute;
     DevBuf<uint32_t> d_cnt;
+    GC_TRY(d_brute.alloc(gc::ksg_brute_scratch(2) / sizeof(double) + 1));
     GC_TRY(d_X.alloc((size_t)6 * T));
     GC_TRY(d_psi.alloc((size_t)T + 1));
     GC_TRY(d_mi.alloc(1));
@@ -778,8 +792,13 @@ gc_status gc_ksg_pair(const double* rows6, int nframes, int k, const double* psi
     GC_TRY_CUDA(cudaMemcpyAsync(d_X.p + (size_t)3 * T, rows6, sizeof(double) * 3 * T, cudaMemcpyHostToDevice, ss.s));
     GC_TRY_CUDA(cudaMemcpyAsync(d_X.p, rows6 + (size_t)3 * T, sizeof(double) * 3 * T, cudaMemcpyHostToDevice, ss.s));
     GC_TRY_CUDA(cudaMemcpyAsync(d_psi.p, psi, sizeof(double) * (T + 1), cudaMemcpyHostToDevice, ss.s));
-    gc::launch_ksg_exact(d_X.p, T, k, 0, 1, d_cnt.p, ss.s, nullptr, wide ? d_cnt.p + T : nullptr);
-    gc::launch_ksg_finalize(d_cnt.p, 1, T, k, d_psi.p, d_mi.p, 148, ss.s, wide ? d_cnt.p + T : nullptr);
+    int sms = 148;
+    GC_TRY_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, cur));
+    if (o.path == GC_PATH_EXACT_FP64)
+        gc::launch_ksg_exact(d_X.p, T, k, 0, 1, d_cnt.p, ss.s, nullptr, wide ? d_cnt.p + T : nullptr);
+    else
+        gc::launch_ksg_brute(d_X.p, 2, T, k, 0, 1, d_cnt.p, d_brute.p, sms, ss.s, nullptr, wide ? d_cnt.p + T : nullptr);
+    gc::launch_ksg_finalize(d_cnt.p, 1, T, k, d_psi.p, d_mi.p, sms, ss.s, wide ? d_cnt.p + T : nullptr);
     GC_TRY_CUDA(cudaGetLastError());
     GC_TRY_CUDA(cudaMemcpyAsync(mi, d_mi.p, sizeof(double), cudaMemcpyDeviceToHost, ss.s));
     GC_TRY_CUDA(cudaStreamSynchronize(ss.s));

@@ -40,6 +40,13 @@ void launch_ksg_check_rows(const double* X, long n, int* status, cudaStream_t s)
 void launch_ksg_exact(const double* X, int T, int K, long pair_begin, long pair_count, uint32_t* cnt,
                       cudaStream_t s, const int2* pair_ab = nullptr, uint32_t* cnt_y = nullptr);
 
+// The same counts by FP32 brute force with FP64 repair (any frame count).
+// scratch: ksg_brute_scratch(natoms) bytes of device memory, 8-byte aligned.
+size_t ksg_brute_scratch(int natoms);
+void launch_ksg_brute(const double* X, int natoms, int T, int K, long pair_begin, long pair_count, uint32_t* cnt,
+                      void* scratch, int sms, cudaStream_t s, const int2* pair_ab = nullptr,
+                      uint32_t* cnt_y = nullptr);
+
 // MI per pair from the per-query counts, summed in frame order as mir_xnyn does.
 void launch_ksg_finalize(const uint32_t* cnt, long pair_count, int T, int K, const double* psi,
                          double* pair_mi, int sms, cudaStream_t s, const uint32_t* cnt_y = nullptr);

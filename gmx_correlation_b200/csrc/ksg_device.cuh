@@ -48,6 +48,11 @@ __device__ __forceinline__ LaneRow lane_row(const WalkParams& p, int atom, int i
     return LaneRow{p.S + base, p.P + base, (size_t)p.Qp * 4};
 }
 
+__device__ __forceinline__ double dist3r(const double* __restrict__ r, int T, double q0, double q1, double q2, int j)
+{
+    return fmax(fmax(fabs(q0 - r[j]), fabs(q1 - r[T + j])), fabs(q2 - r[2 * T + j]));
+}
+
 // Hand-over causes (WalkParams::reasons index).
 enum
 {

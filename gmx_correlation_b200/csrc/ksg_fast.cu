@@ -146,11 +146,6 @@ __device__ __forceinline__ void row_bounds4(const LaneRow (&r)[4], int (&lo)[4],
     }
 }
 
-__device__ __forceinline__ double dist3r(const double* __restrict__ r, int T, double q0, double q1, double q2, int j)
-{
-    return fmax(fmax(fabs(q0 - r[j]), fabs(q1 - r[T + j])), fabs(q2 - r[2 * T + j]));
-}
-
 constexpr int kScanCap = 1024; // row entries a backward scan may visit
 constexpr int kAmbCap  = 8;    // ambiguous entries ordered in FP64
 

@@ -4,9 +4,9 @@
 // code, or a caller on a latency-critical path where an allocation (and the
 // implicit device synchronisation cudaFree brings) is not acceptable.
 //
-// The exact FP64 KSG pipeline (the same kernels as gc_ksg_matrix's exact
-// path: normalisation, neighbour statistics, frame-ordered MI reduction)
-// runs with every piece of scratch memory taken from one fixed array,
+// The brute-force KSG pipeline (the kernels gc_ksg_matrix runs on
+// trajectories too long for sorted rows: normalisation, FP32 neighbour
+// statistics with FP64 repair, frame-ordered MI reduction) runs with every piece of scratch memory taken from one fixed array,
 // g_noalloc_scratch, that lives for the life of the process on every device
 // that loads this library.  The caller passes device pointers for the
 // coordinates and the pair MI output.
@@ -51,7 +51,8 @@ constexpr size_t kOffX      = 0;                                                
 constexpr size_t kOffCnt    = kOffX + align256(sizeof(double) * 3 * kNoAllocMaxAtoms * kNoAllocMaxFrames);
 constexpr size_t kOffPsi    = kOffCnt + align256(sizeof(uint32_t) * kMaxPairs * kNoAllocMaxFrames);
 constexpr size_t kOffStatus = kOffPsi + align256(sizeof(double) * (kNoAllocMaxFrames + 1));
-constexpr size_t kScratchBytes = kOffStatus + 256;
+constexpr size_t kOffBrute  = kOffStatus + 256;                                        // ksg_brute_scratch(64)
+constexpr size_t kScratchBytes = kOffBrute + align256(kNoAllocMaxAtoms * (3 * sizeof(double) + sizeof(float)));
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
 
@@ -60,15 +61,26 @@ std::mutex    g_setup_mutex;
 void*         g_scratch_addr[kMaxDevices] = {};
 
 // psi[0] = 0, psi[1] = -0.57721566490153, psi[n+1] = psi[n] + 1/n, in the
-// reference's sequential order (lib/kraskov.cpp:2217-2219).
-__global__ void noalloc_psi_kernel(double* psi, int N)
+// reference's sequential order (lib/kraskov.cpp:2217-2219).  One CTA: the
+// quotients by all threads, the sums by one (which took 40 us for 900 frames
+// when it divided as well).
+__global__ void __launch_bounds__(256) noalloc_psi_kernel(double* psi, int N)
 {
-    if (blockIdx.x != 0 || threadIdx.x != 0)
+    __shared__ double inv[kNoAllocMaxFrames + 1];
+    for (int n = threadIdx.x + 1; n < N; n += 256)
+        inv[n] = __ddiv_rn(1.0, (double)n);
+    __syncthreads();
+    if (threadIdx.x != 0)
         return;
-    psi[0] = 0.0;
-    psi[1] = -0.57721566490153;
+    double p = -0.57721566490153;
+    psi[0]   = 0.0;
+    psi[1]   = p;
+#pragma unroll 8
     for (int n = 1; n < N; ++n)
-        psi[n + 1] = __dadd_rn(psi[n], __ddiv_rn(1.0, (double)n));
+    {
+        p          = __dadd_rn(p, inv[n]);
+        psi[n + 1] = p;
+    }
 }
 
 // Records `msg` as the calling thread's gc_last_error() text and returns st.
@@ -129,13 +141,16 @@ extern "C" gc_status gc_ksg_pair_mi_noalloc(const double* d_xyz, int natoms, int
     cudaStream_t   s      = static_cast<cudaStream_t>(stream);
     const long     npairs = (long)natoms * (natoms - 1) / 2;
 
-    cudaError_t e = cudaMemsetAsync(status, 0, sizeof(int), s);
+    int         sms = 148;
+    cudaError_t e   = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess)
+        e = cudaMemsetAsync(status, 0, sizeof(int), s);
     if (e == cudaSuccess)
     {
-        noalloc_psi_kernel<<<1, 1, 0, s>>>(psi, nframes);
+        noalloc_psi_kernel<<<1, 256, 0, s>>>(psi, nframes);
         gc::launch_ksg_prepare(d_xyz, natoms, nframes, X, status, s);
-        gc::launch_ksg_exact(X, nframes, k, 0, npairs, cnt, s);
-        gc::launch_ksg_finalize(cnt, npairs, nframes, k, psi, d_pair_mi, 148, s);
+        gc::launch_ksg_brute(X, natoms, nframes, k, 0, npairs, cnt, b + kOffBrute, sms, s);
+        gc::launch_ksg_finalize(cnt, npairs, nframes, k, psi, d_pair_mi, sms, s);
         e = cudaGetLastError();
     }
     int st = 0;

@@ -1,0 +1,59 @@
+"""The row walk and the FP32 brute force at the sizes where they can go wrong,
+against the exact FP64 path: blocks of 32 atoms and their remainders, tiles of
+the shortest and longest rows, the smallest and largest k, bucket windows far
+apart, duplicated frames and exact ties; frames around the staged chunk and
+the row sort's limit.  Both sides count the same neighbours and add the same
+table entries in the same order, so every value is equal, bit for bit."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _traj(kind, n, T, seed):
+    from gmx_correlation_b200.synth import synth_traj
+    rng = np.random.default_rng(seed)
+    x = synth_traj(n, T, 6, 0.08, seed=seed, fp32=True)
+    if kind == "ties":  # a coarse lattice: many equal distances
+        x = np.round(x * 40.0) / 40.0 + 0.0
+    elif kind == "duplicates":  # a third of the frames repeat frame 0
+        x[:, rng.choice(T, T // 3, replace=False)] = x[:, :1]
+    elif kind == "tails":  # atoms with rare large excursions: k-th distances of very different size
+        x[::3] *= 1.0 + 200.0 * (rng.random((len(x[::3]), T, 1)) < 4.0 / T)
+    return x
+
+
+@pytest.mark.parametrize("n,T,k,kind", [
+    (24, 40, 1, "smooth"), (24, 40, 39, "smooth"), (31, 97, 5, "smooth"), (32, 129, 7, "ties"),
+    (33, 128, 20, "smooth"), (64, 300, 10, "duplicates"), (65, 257, 12, "smooth"), (66, 500, 100, "tails"),
+    (40, 1300, 254, "smooth"), (25, 2049, 60, "ties"), (24, 6040, 30, "smooth"), (24, 6060, 30, "smooth"),
+    (97, 400, 4, "tails"),
+])
+def test_row_walk_equals_exact(gc, n, T, k, kind):
+    x = _traj(kind, n, T, seed=n + T)
+    a, ax, ay = gc.kraskov_corrmatrix(x, k, detail=True)
+    b, bx, by = gc.kraskov_corrmatrix(x, k, path=gc.PATH_EXACT_FP64, detail=True)
+    np.testing.assert_array_equal(ax, bx)
+    np.testing.assert_array_equal(ay, by)
+    np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("T,k,kind", [
+    (20, 1, "smooth"), (33, 32, "smooth"), (500, 10, "ties"), (700, 40, "duplicates"), (2047, 100, "smooth"),
+    (2048, 300, "smooth"), (2049, 6, "tails"), (4097, 50, "smooth"), (5000, 4999, "smooth"),
+])
+def test_single_pair_equals_exact(gc, T, k, kind):
+    x = _traj(kind, 2, T, seed=T)
+    X, psi, _ = gc.kraskov_prepare(x)
+    assert gc.kraskov_wrap(X, psi, 1, 0, k) == gc.kraskov_corrmatrix(x, k, path=gc.PATH_EXACT_FP64)[1, 0]
+
+
+@pytest.mark.parametrize("n,T,k,kind", [(3, 16386, 20, "smooth"), (4, 16500, 3, "tails"), (2, 17000, 900, "smooth"),
+                                        (2, 16400, 15, "ties")])
+def test_long_rows_equal_exact(gc, n, T, k, kind):
+    x = _traj(kind, n, T, seed=n)
+    a, ax, ay = gc.kraskov_corrmatrix(x, k, detail=True)
+    b, bx, by = gc.kraskov_corrmatrix(x, k, path=gc.PATH_EXACT_FP64, detail=True)
+    np.testing.assert_array_equal(ax, bx)
+    np.testing.assert_array_equal(ay, by)
+    np.testing.assert_array_equal(a, b)
