@@ -706,59 +706,58 @@ __global__ void __launch_bounds__(kFinishWarps * 32, 1) ksg_finish_kernel(WalkBa
                     nlo += v < elo;
                 };
                 // Both ranges by aligned 4-entry groups of the row (one 16-byte
-                // and one 8-byte load per group), kFinishRound groups per round
-                // (the loads of a round, then its gathers).  One group per round
-                // keeps the kernel at 96 registers, so a CTA holds 20 warps.
-                for (int g0 = mw0 >> 2; g0 * 4 < mw1; g0 += kFinishRound) // s in the band, d <= bandhi
+                // and one 8-byte load per group),
+                // the next group's loads in flight while this one gathers.
                 {
-                    float4 s4[kFinishRound];
-                    uint2  j4[kFinishRound];
-#pragma unroll
-                    for (int h = 0; h < kFinishRound; ++h)
-                        if ((g0 + h) * 4 < mw1)
-                        {
-                            s4[h] = rw.s4(g0 + h);
-                            j4[h] = rw.j4(g0 + h);
-                        }
-#pragma unroll
-                    for (int h = 0; h < kFinishRound; ++h)
+                    int    g  = min(mw0, Llen - 1) >> 2;
+                    float4 s4 = rw.s4(g);
+                    uint2  j4 = rw.j4(g);
+                    while (g * 4 < mw1) // s in the band, d <= bandhi
+                    {
+                        const int    gn = (g + 1) * 4 < mw1 ? g + 1 : g;
+                        const float4 ns = rw.s4(gn);
+                        const uint2  nj = rw.j4(gn);
 #pragma unroll
                         for (int q = 0; q < 4; ++q)
                         {
-                            const int   mm = (g0 + h) * 4 + q;
+                            const int   mm = g * 4 + q;
                             const bool  in = mm >= mw0 && mm < mw1;
-                            const int   j  = (int)u2get16(j4[h], q);
-                            const float sv = f4get(s4[h], q);
+                            const int   j  = (int)u2get16(j4, q);
+                            const float sv = f4get(s4, q);
                             const float dv = dist3f(xo, X32o[in ? j : 0]);
                             if (in && dv <= bandhi)
                                 add(fmaxf(sv, dv), sv, dv, mm - mw0);
                         }
+                        ++g;
+                        s4 = ns;
+                        j4 = nj;
+                    }
                 }
                 const int nW = nband; // band entries from the walked row come first
-                for (int g0 = mo0 >> 2; g0 * 4 < mo1; g0 += kFinishRound) // d in the band, s < inlo
                 {
-                    float4 d4[kFinishRound];
-                    uint2  j4[kFinishRound];
-#pragma unroll
-                    for (int h = 0; h < kFinishRound; ++h)
-                        if ((g0 + h) * 4 < mo1)
-                        {
-                            d4[h] = ro.s4(g0 + h);
-                            j4[h] = ro.j4(g0 + h);
-                        }
-#pragma unroll
-                    for (int h = 0; h < kFinishRound; ++h)
+                    int    g  = min(mo0, Llen - 1) >> 2;
+                    float4 d4 = ro.s4(g);
+                    uint2  j4 = ro.j4(g);
+                    while (g * 4 < mo1) // d in the band, s < inlo
+                    {
+                        const int    gn = (g + 1) * 4 < mo1 ? g + 1 : g;
+                        const float4 nd = ro.s4(gn);
+                        const uint2  nj = ro.j4(gn);
 #pragma unroll
                         for (int q = 0; q < 4; ++q)
                         {
-                            const int   mm = (g0 + h) * 4 + q;
+                            const int   mm = g * 4 + q;
                             const bool  in = mm >= mo0 && mm < mo1;
-                            const int   j  = (int)u2get16(j4[h], q);
-                            const float dv = f4get(d4[h], q);
+                            const int   j  = (int)u2get16(j4, q);
+                            const float dv = f4get(d4, q);
                             const float sv = dist3f(xw, X32w[in ? j : 0]);
                             if (in && sv < inlo)
                                 add(dv, sv, dv, mm - mo0);
                         }
+                        ++g;
+                        d4 = nd;
+                        j4 = nj;
+                    }
                 }
                 // frame of band entry e (for the FP64 paths)
                 auto band_frame = [&](int e) -> int {
