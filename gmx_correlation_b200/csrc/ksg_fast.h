@@ -83,12 +83,18 @@ struct WalkBatch
     unsigned long long* counter; // [2] walk and finish task counters, zero at launch
 };
 
-// Bucket width of the walk histogram for k: about 1.3/k of the value
-// (around eight entries per bucket near the k-th value), at least 2^17
-// ulps so that the 128 buckets span two octaves above the lower bound.
+// Bucket width of the walk histogram for k: about 0.33/k of the value (two or
+// three entries per bucket near the k-th value), between 2^17 ulps, so that
+// the 128 buckets span two octaves above the lower bound, and 2^21.  Four
+// times wider buckets, eight entries each, make the finish kernels enumerate
+// that many more: 64 x 500, k = 10: finish 552 -> 405 us, hand-overs 163 ->
+// 0; 150 x 4000, k = 10: 54.7 -> 33.1 ms; TE 40 x 700, k = 10: 705 -> 348 us.
+// Half the width again (2^17 ulps already at k = 10) gains 5-10% of the
+// finish and loses it in the walk; 2^16 ulps span one octave: 4% of the
+// queries at 100 x 4999, k = 100 lie beyond and the matrix takes 311 ms for 82.
 inline int walk_histogram_shift(int K)
 {
-    const double target = 24.0 + __builtin_log2(0.67 / (double)K);
+    const double target = 22.0 + __builtin_log2(0.67 / (double)K);
     int          s      = (int)(target + 0.5);
     return s < 17 ? 17 : (s > 21 ? 21 : s);
 }
