@@ -675,10 +675,9 @@ static gc_status gauss_like(const gc_traj_view* traj, const gc_opts* opts, doubl
     StreamScope ss;
     GC_TRY(ss.init(o.stream));
     const long     nb = (long)n * (n + 1) / 2;
-    DevBuf<double> d_xyz, d_XF, d_Z, d_zt, d_blk, d_mat;
+    DevBuf<double> d_xyz, d_Z, d_zt, d_blk, d_mat;
     DevBuf<int>    d_st;
     GC_TRY(d_xyz.alloc((size_t)n * T * 3));
-    GC_TRY(d_XF.alloc((size_t)n * T * 3));
     GC_TRY(d_blk.alloc((size_t)nb * 9));
     GC_TRY(d_mat.alloc((size_t)n * n));
     GC_TRY(d_st.alloc(1));
@@ -690,14 +689,13 @@ static gc_status gauss_like(const gc_traj_view* traj, const gc_opts* opts, doubl
     GC_TRY(upload_traj(traj, d_xyz.p, ss.s));
     GC_TRY_CUDA(cudaMemsetAsync(d_st.p, 0, sizeof(int), ss.s));
     GC_TRY_CUDA(cudaMemsetAsync(d_mat.p, 0, sizeof(double) * (size_t)n * n, ss.s));
-    gc::launch_frame_major(d_xyz.p, n, T, d_XF.p, d_st.p, ss.s);
-    const double* V = d_XF.p;
     if (mode == 1)
     {
-        gc::launch_copula(d_XF.p, n, T, d_zt.p, d_Z.p, ss.s);
-        V = d_Z.p;
+        gc::launch_copula(d_xyz.p, n, T, d_zt.p, d_Z.p, d_st.p, ss.s);
+        gc::launch_blocks(d_Z.p, true, n, T, d_blk.p, nullptr, ss.s);
     }
-    gc::launch_blocks(V, n, T, d_blk.p, ss.s);
+    else
+        gc::launch_blocks(d_xyz.p, false, n, T, d_blk.p, d_st.p, ss.s);
     const double log2pi = std::log(2.0 * 3.14159265358979323846);
     gc::launch_pair_logdet(d_blk.p, n, T, mode, log2pi, d_mat.p, ss.s);
     GC_TRY_CUDA(cudaGetLastError());

@@ -260,7 +260,7 @@ TeBatchPlan* g_te[kMaxDev] = {}; // the last batch per device (its blocks return
 struct GcmiItem
 {
     int                 natoms = 0, T = 0;
-    PoolBuf<double>     xyz, XF, Z, zt, blk, mat;
+    PoolBuf<double>     xyz, Z, zt, blk, mat;
     std::vector<double> host;
 };
 
@@ -292,9 +292,8 @@ gc_status gcmi_enqueue_all(void* ctx, cudaStream_t s)
     {
         GcmiItem& it = *bp.items[i];
         GC_TRY_CUDA(cudaMemsetAsync(it.mat.p, 0, sizeof(double) * (size_t)it.natoms * it.natoms, s));
-        gc::launch_frame_major(it.xyz.p, it.natoms, it.T, it.XF.p, bp.status.p + i, s);
-        gc::launch_copula(it.XF.p, it.natoms, it.T, it.zt.p, it.Z.p, s);
-        gc::launch_blocks(it.Z.p, it.natoms, it.T, it.blk.p, s);
+        gc::launch_copula(it.xyz.p, it.natoms, it.T, it.zt.p, it.Z.p, bp.status.p + i, s);
+        gc::launch_blocks(it.Z.p, true, it.natoms, it.T, it.blk.p, nullptr, s);
         gc::launch_pair_logdet(it.blk.p, it.natoms, it.T, 1, log2pi, it.mat.p, s);
     }
     GC_TRY_CUDA(cudaGetLastError());
@@ -433,7 +432,6 @@ gc_status gc_gcmi_batch(const gc_traj_view* trajs, int ntraj, const gc_opts* opt
             it.T         = trajs[i].nframes;
             const size_t c = (size_t)it.natoms * it.T * 3;
             GC_TRY(it.xyz.alloc(c));
-            GC_TRY(it.XF.alloc(c));
             GC_TRY(it.Z.alloc(c));
             GC_TRY(it.zt.alloc((size_t)it.T));
             GC_TRY(it.blk.alloc((size_t)it.natoms * (it.natoms + 1) / 2 * 9));

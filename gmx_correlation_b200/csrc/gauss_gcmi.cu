@@ -18,23 +18,6 @@
 
 namespace gc {
 
-__global__ void frame_major_kernel(const double* __restrict__ xyz, int natoms, int T, double* __restrict__ XF,
-                                   int* __restrict__ status)
-{
-    const long n  = (long)natoms * T * 3;
-    const int  nc = natoms * 3;
-    for (long idx = blockIdx.x * (long)blockDim.x + threadIdx.x; idx < n; idx += (long)gridDim.x * blockDim.x)
-    {
-        const long   a = idx / ((long)T * 3);
-        const long   r = idx - a * (long)T * 3;
-        const int    f = (int)(r / 3), d = (int)(r - (r / 3) * 3);
-        const double v = xyz[idx];
-        if (!isfinite(v))
-            atomicOr(status, kStatNonFinite);
-        XF[(size_t)f * nc + a * 3 + d] = v;
-    }
-}
-
 // gcmi_erfinv (lib/gcmi.cpp:26-79): Acklam's rational approximation of the
 // inverse normal CDF (published coefficients), mapped to erfinv, then one
 // Newton step with erf/exp.
@@ -99,42 +82,56 @@ constexpr int kCopulaSortMax = 16384;
 
 // One CTA per component: bitonic sort of (value, frame) in shared memory,
 // then midrank averaging of the probit scores over runs of equal values
-// (lib/gcmi.cpp:113-143).  Requires next_pow2(T) * 12 bytes of shared memory.
-__global__ void copula_kernel(const double* __restrict__ XF, int natoms, int T, int P,
-                              const double* __restrict__ zt, double* __restrict__ Z)
+// (lib/gcmi.cpp:113-143).  Requires next_pow2(T) * 12 bytes of shared memory
+// (P >= 64).  A warp's threads take 32 neighbouring pairs, so the steps of
+// stride 32 and below stay inside its 64 entries and need no CTA barrier (51
+// of the 66 steps at 2048 entries): 247 x 2000 copulas 150 -> 131 us.
+__global__ void __launch_bounds__(512) copula_kernel(const double* __restrict__ xyz, int T, int P,
+                                                     const double* __restrict__ zt, double* __restrict__ Z,
+                                                     int* __restrict__ status)
 {
     extern __shared__ unsigned char smem_raw[];
-    double* val = reinterpret_cast<double*>(smem_raw);
-    int*    idx = reinterpret_cast<int*>(val + P);
-    const int nc = natoms * 3, comp = blockIdx.x;
+    double*       val  = reinterpret_cast<double*>(smem_raw);
+    int*          idx  = reinterpret_cast<int*>(val + P);
+    const int     comp = blockIdx.x;
+    const double* src  = xyz + (size_t)(comp / 3) * T * 3 + comp % 3;
+    bool          bad  = false;
     for (int t = threadIdx.x; t < P; t += blockDim.x)
     {
-        val[t] = t < T ? XF[(size_t)t * nc + comp] : __longlong_as_double(0x7ff0000000000000LL);
+        const double v = t < T ? src[(size_t)t * 3] : __longlong_as_double(0x7ff0000000000000LL);
+        bad |= t < T && !isfinite(v);
+        val[t] = v;
         idx[t] = t < T ? t : -1;
     }
+    if (bad)
+        atomicOr(status, kStatNonFinite);
     __syncthreads();
     for (int k = 2; k <= P; k <<= 1)
         for (int j = k >> 1; j > 0; j >>= 1)
         {
-            for (int t = threadIdx.x; t < P; t += blockDim.x)
+            for (int p = threadIdx.x; p < P / 2; p += blockDim.x)
             {
-                const int u = t ^ j;
-                if (u > t)
+                const int    t = 2 * p - (p & (j - 1)), u = t + j; // pair p of the step
+                const bool   up = (t & k) == 0;
+                const double vt = val[t], vu = val[u];
+                if ((vt > vu) == up)
                 {
-                    const bool   up = (t & k) == 0;
-                    const double vt = val[t], vu = val[u];
-                    if ((vt > vu) == up)
-                    {
-                        val[t] = vu;
-                        val[u] = vt;
-                        const int it = idx[t];
-                        idx[t]       = idx[u];
-                        idx[u]       = it;
-                    }
+                    val[t] = vu;
+                    val[u] = vt;
+                    const int it = idx[t];
+                    idx[t]       = idx[u];
+                    idx[u]       = it;
                 }
             }
-            __syncthreads();
+            // the next step's entries: the warp's own while its stride (j / 2, or
+            // k for the next merge's first) is at most 32
+            if (j > 32 || (j == 1 && k > 32))
+                __syncthreads();
+            else
+                __syncwarp();
         }
+    __syncthreads();
+    double* z = Z + (size_t)comp * T;
     for (int r = threadIdx.x; r < T; r += blockDim.x)
     {
         if (r > 0 && val[r] == val[r - 1])
@@ -147,7 +144,7 @@ __global__ void copula_kernel(const double* __restrict__ XF, int natoms, int T, 
             avg = __dadd_rn(avg, zt[t]);
         avg = __ddiv_rn(avg, (double)(s - r));
         for (int t = r; t < s; ++t)
-            Z[(size_t)idx[t] * nc + comp] = avg;
+            z[idx[t]] = avg;
     }
 }
 
@@ -158,20 +155,24 @@ __global__ void copula_kernel(const double* __restrict__ XF, int natoms, int T, 
 // components); the component's values pass through shared memory in tiles.
 constexpr int kCopulaTile = 4096;
 
-__global__ void __launch_bounds__(256) copula_count_kernel(const double* __restrict__ XF, int natoms, int T,
-                                                           const double* __restrict__ zt, double* __restrict__ Z)
+__global__ void __launch_bounds__(256) copula_count_kernel(const double* __restrict__ xyz, int T,
+                                                           const double* __restrict__ zt, double* __restrict__ Z,
+                                                           int* __restrict__ status)
 {
     __shared__ double tile[kCopulaTile];
-    const int    nc   = natoms * 3, comp = blockIdx.y;
-    const int    f    = blockIdx.x * blockDim.x + threadIdx.x;
-    const double v    = f < T ? XF[(size_t)f * nc + comp] : 0.0;
-    int          lt = 0, eq = 0;
+    const int     comp = blockIdx.y;
+    const double* src  = xyz + (size_t)(comp / 3) * T * 3 + comp % 3;
+    const int     f    = blockIdx.x * blockDim.x + threadIdx.x;
+    const double  v    = f < T ? src[(size_t)f * 3] : 0.0;
+    if (!isfinite(v))
+        atomicOr(status, kStatNonFinite);
+    int lt = 0, eq = 0;
     for (int t0 = 0; t0 < T; t0 += kCopulaTile)
     {
         const int n = min(kCopulaTile, T - t0);
         __syncthreads(); // the previous tile is consumed
         for (int e = threadIdx.x; e < n; e += blockDim.x)
-            tile[e] = XF[(size_t)(t0 + e) * nc + comp];
+            tile[e] = src[(size_t)(t0 + e) * 3];
         __syncthreads();
         for (int e = 0; e < n; ++e)
         {
@@ -185,46 +186,139 @@ __global__ void __launch_bounds__(256) copula_count_kernel(const double* __restr
     double avg = 0.0;
     for (int t = lt; t < lt + eq; ++t)
         avg = __dadd_rn(avg, zt[t]);
-    Z[(size_t)f * nc + comp] = __ddiv_rn(avg, (double)eq);
+    Z[(size_t)comp * T + f] = __ddiv_rn(avg, (double)eq);
 }
 
-// Block b = hi*(hi+1)/2 + lo (lo <= hi): 9 co-moments summed over frames in order.
-__global__ void blocks_kernel(const double* __restrict__ V, int natoms, int T, double* __restrict__ blk)
+// Co-moment blocks b = hi (hi + 1) / 2 + lo (lo <= hi): 9 sums over frames in
+// order.  A CTA takes TILE x TILE atom pairs, ROWS hi atoms per thread (two
+// halve the shared-memory reads, which else take as long as the arithmetic);
+// the tile's 2 TILE atoms pass through shared memory 8 frames at a time, atoms side by side (the
+// lanes of a warp read neighbouring lo atoms and two hi atoms), copied
+// asynchronously three stages ahead.  SERIES: V holds each
+// component's series [3 natoms][T]; otherwise frames of xyz [natoms][T][3].
+//
+// Bound by the FP64 pipe (9 multiplications and 9 additions per pair and
+// frame, which the reference's rounding forbids to fuse) and, with few
+// tiles, by one SM's share of it: T * 72 cycles for a 16 x 16 tile.  One
+// thread per block reading frame-major rows from L2 took 570 us at 247 x 2000
+// and 1660 us at 600 x 4000, after a 54 us transposition; now
+// 190 and 1300 us (10 T FP64 operations/s).
+constexpr int kMomentFrames = 8; // frames per stage
+constexpr int kMomentStages = 4;
+
+template <int TILE, int ROWS, bool SERIES>
+__global__ void __launch_bounds__(TILE * TILE / ROWS) comoment_kernel(const double* __restrict__ V, int natoms, int T,
+                                                                      double* __restrict__ blk, int* __restrict__ status)
 {
-    const long nb = (long)natoms * (natoms + 1) / 2;
-    const long b  = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    if (b >= nb)
-        return;
-    long hi = (long)((sqrt(8.0 * (double)b + 1.0) - 1.0) * 0.5);
-    while (hi * (hi + 1) / 2 > b)
-        --hi;
-    while ((hi + 1) * (hi + 2) / 2 <= b)
-        ++hi;
-    const long lo = b - hi * (hi + 1) / 2;
-    const int  nc = natoms * 3;
-    double     acc[9];
+    constexpr int F = kMomentFrames, kThreads = TILE * TILE / ROWS, kElems = 2 * TILE * 3 * F, kRow = 2 * TILE + 1;
+    constexpr int kPer = kElems / kThreads;
+    static_assert(kElems % kThreads == 0, "whole elements per thread");
+    __shared__ double buf[kMomentStages][F * 3][kRow]; // [frame * 3 + component][lo atoms, hi atoms]
+    const int tid = threadIdx.x, tx = tid % TILE, ty = tid / TILE;
+    // tile pair index -> (th, tl), tl <= th
+    int th = (int)((sqrtf(8.0f * (float)blockIdx.x + 1.0f) - 1.0f) * 0.5f);
+    while (th * (th + 1) / 2 > (int)blockIdx.x)
+        --th;
+    while ((th + 1) * (th + 2) / 2 <= (int)blockIdx.x)
+        ++th;
+    const int tl = (int)blockIdx.x - th * (th + 1) / 2;
+    // this thread's elements of a stage: consecutive threads take consecutive
+    // addresses of one atom's frames
+    const double* src[kPer];
+    unsigned      dst[kPer];
+    int           fr[kPer];
 #pragma unroll
-    for (int e = 0; e < 9; ++e)
-        acc[e] = 0.0;
-    const double* pl = V + lo * 3;
-    const double* ph = V + hi * 3;
-    for (int f = 0; f < T; ++f)
+    for (int k = 0; k < kPer; ++k)
     {
-        const double l0 = pl[(size_t)f * nc], l1 = pl[(size_t)f * nc + 1], l2 = pl[(size_t)f * nc + 2];
-        const double h0 = ph[(size_t)f * nc], h1 = ph[(size_t)f * nc + 1], h2 = ph[(size_t)f * nc + 2];
-        acc[0] = __dadd_rn(acc[0], __dmul_rn(l0, h0));
-        acc[1] = __dadd_rn(acc[1], __dmul_rn(l0, h1));
-        acc[2] = __dadd_rn(acc[2], __dmul_rn(l0, h2));
-        acc[3] = __dadd_rn(acc[3], __dmul_rn(l1, h0));
-        acc[4] = __dadd_rn(acc[4], __dmul_rn(l1, h1));
-        acc[5] = __dadd_rn(acc[5], __dmul_rn(l1, h2));
-        acc[6] = __dadd_rn(acc[6], __dmul_rn(l2, h0));
-        acc[7] = __dadd_rn(acc[7], __dmul_rn(l2, h1));
-        acc[8] = __dadd_rn(acc[8], __dmul_rn(l2, h2));
+        const int e = tid + k * kThreads, at = e / (3 * F), r = e - at * 3 * F;
+        const int f = SERIES ? r % F : r / 3, d = SERIES ? r / F : r - r / 3 * 3;
+        const int a = min(at < TILE ? tl * TILE + at : th * TILE + at - TILE, natoms - 1);
+        src[k]      = SERIES ? V + ((size_t)a * 3 + d) * T + f : V + ((size_t)a * T + f) * 3 + d;
+        dst[k]      = (unsigned)__cvta_generic_to_shared(&buf[0][f * 3 + d][at]);
+        fr[k]       = f;
     }
+    const int chunks = (T + F - 1) / F;
+    auto      fetch  = [&](int c) {
+        if (c < chunks)
+        {
+            const unsigned stage = (unsigned)(c % kMomentStages) * (unsigned)sizeof(buf[0]);
 #pragma unroll
-    for (int e = 0; e < 9; ++e)
-        blk[b * 9 + e] = acc[e];
+            for (int k = 0; k < kPer; ++k)
+                if (c * F + fr[k] < T)
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst[k] + stage),
+                                 "l"(src[k] + (size_t)c * F * (SERIES ? 1 : 3))
+                                 : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    constexpr int kStep = TILE / ROWS; // a thread's hi atoms: ty, ty + kStep, ...
+    double        acc[ROWS][9];
+#pragma unroll
+    for (int h = 0; h < ROWS; ++h)
+#pragma unroll
+        for (int e = 0; e < 9; ++e)
+            acc[h][e] = 0.0;
+    bool bad = false;
+#pragma unroll
+    for (int c = 0; c < kMomentStages - 1; ++c)
+        fetch(c);
+    for (int c = 0; c < chunks; ++c)
+    {
+        // this thread's part of stage c has arrived, then everyone's; the stage
+        // fetched next was read in the round before the barrier
+        asm volatile("cp.async.wait_group %0;" ::"n"(kMomentStages - 2) : "memory");
+        __syncthreads();
+        fetch(c + kMomentStages - 1);
+        const double(*b)[kRow] = buf[c % kMomentStages];
+        const int n            = min(F, T - c * F);
+        // a frame's values are read while the frame before it is summed
+        double l[2][3], v[2][ROWS][3];
+        auto   read = [&](int f, int w) {
+#pragma unroll
+            for (int d = 0; d < 3; ++d)
+            {
+                l[w][d] = b[f * 3 + d][tx];
+#pragma unroll
+                for (int h = 0; h < ROWS; ++h)
+                    v[w][h][d] = b[f * 3 + d][TILE + ty + h * kStep];
+            }
+        };
+        read(0, 0);
+#pragma unroll
+        for (int f = 0; f < F; ++f)
+        {
+            if (f + 1 < F)
+                read(f + 1, (f + 1) & 1); // behind the last frame: stale values, not used
+            if (f < n)
+#pragma unroll
+                for (int h = 0; h < ROWS; ++h)
+#pragma unroll
+                    for (int r = 0; r < 3; ++r)
+#pragma unroll
+                        for (int d = 0; d < 3; ++d)
+                            acc[h][r * 3 + d] =
+                                __dadd_rn(acc[h][r * 3 + d], __dmul_rn(l[f & 1][r], v[f & 1][h][d]));
+        }
+        if (status && tl == th) // every atom is in one tile of the diagonal
+            for (int f = 0; f < n; ++f)
+#pragma unroll
+                for (int d = 0; d < 3; ++d)
+                    bad |= !isfinite(b[f * 3 + d][tx]);
+    }
+    if (status && bad)
+        atomicOr(status, kStatNonFinite);
+#pragma unroll
+    for (int h = 0; h < ROWS; ++h)
+    {
+        const int lo = tl * TILE + tx, hi = th * TILE + ty + h * kStep;
+        if (lo <= hi && hi < natoms)
+        {
+            double* o = blk + ((size_t)hi * (hi + 1) / 2 + lo) * 9;
+#pragma unroll
+            for (int e = 0; e < 9; ++e)
+                o[e] = acc[h][e];
+        }
+    }
 }
 
 // Determinant by LU with partial pivoting (lib/correlation_core.cpp:49-98,
@@ -346,33 +440,46 @@ __global__ void pair_logdet_kernel(const double* __restrict__ blk, int natoms, i
     mat[(size_t)lo * natoms + hi] = mi;
 }
 
-void launch_frame_major(const double* xyz, int natoms, int T, double* XF, int* status, cudaStream_t s)
-{
-    frame_major_kernel<<<1184, 256, 0, s>>>(xyz, natoms, T, XF, status);
-}
-
-void launch_copula(const double* XF, int natoms, int T, double* zt, double* Z, cudaStream_t s)
+void launch_copula(const double* xyz, int natoms, int T, double* zt, double* Z, int* status, cudaStream_t s)
 {
     probit_table_kernel<<<(T + 127) / 128, 128, 0, s>>>(T, zt);
     if (T > kCopulaSortMax)
     {
-        copula_count_kernel<<<dim3((unsigned)((T + 255) / 256), (unsigned)(natoms * 3)), 256, 0, s>>>(XF, natoms, T,
-                                                                                                     zt, Z);
+        copula_count_kernel<<<dim3((unsigned)((T + 255) / 256), (unsigned)(natoms * 3)), 256, 0, s>>>(xyz, T, zt, Z,
+                                                                                                     status);
         return;
     }
-    int P = 1;
+    int P = 64;
     while (P < T)
         P <<= 1;
     const size_t smem = (size_t)P * (sizeof(double) + sizeof(int));
     if (smem > 48 * 1024)
         cudaFuncSetAttribute(copula_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    copula_kernel<<<natoms * 3, 512, smem, s>>>(XF, natoms, T, P, zt, Z);
+    const int threads = P / 2 < 512 ? P / 2 : 512;
+    copula_kernel<<<natoms * 3, threads, smem, s>>>(xyz, T, P, zt, Z, status);
 }
 
-void launch_blocks(const double* V, int natoms, int T, double* blk, cudaStream_t s)
+void launch_blocks(const double* V, bool series, int natoms, int T, double* blk, int* status, cudaStream_t s)
 {
-    const long nb = (long)natoms * (natoms + 1) / 2;
-    blocks_kernel<<<(unsigned)((nb + 127) / 128), 128, 0, s>>>(V, natoms, T, blk);
+    // 16 x 16 tiles, or 8 x 8 where those would leave most SMs idle (fewer
+    // than 74 tiles, up to 180 atoms)
+    const long t16 = (natoms + 15) / 16, t8 = (natoms + 7) / 8;
+    if (t16 * (t16 + 1) / 2 >= 74)
+    {
+        const unsigned g = (unsigned)(t16 * (t16 + 1) / 2);
+        if (series)
+            comoment_kernel<16, 2, true><<<g, 128, 0, s>>>(V, natoms, T, blk, status);
+        else
+            comoment_kernel<16, 2, false><<<g, 128, 0, s>>>(V, natoms, T, blk, status);
+    }
+    else
+    {
+        const unsigned g = (unsigned)(t8 * (t8 + 1) / 2);
+        if (series)
+            comoment_kernel<8, 1, true><<<g, 64, 0, s>>>(V, natoms, T, blk, status);
+        else
+            comoment_kernel<8, 1, false><<<g, 64, 0, s>>>(V, natoms, T, blk, status);
+    }
 }
 
 void launch_pair_logdet(const double* blk, int natoms, int T, int mode, double log2pi, double* mat,

@@ -71,14 +71,14 @@ void launch_te_finalize(const uint2* cnt, int natoms, int T, int K, int lag, con
                         double* te_mat, cudaStream_t s, bool wide = false);
 
 // ---- Gaussian and copula MI ------------------------------------------------
-// xyz [natoms][T][3] -> XF [T][3*natoms] (frame-major), status on non-finite.
-void launch_frame_major(const double* xyz, int natoms, int T, double* XF, int* status, cudaStream_t s);
-// Copula transform (lib/gcmi.cpp:95-146) of XF into Z [T][3*natoms] (frame-major).
+// Copula transform (lib/gcmi.cpp:95-146) of xyz [natoms][T][3] into the
+// component series Z [3*natoms][T], status on non-finite.
 // zt: [T] probit table sqrt(2)*erfinv(2(t+0.5)/T - 1).
-void launch_copula(const double* XF, int natoms, int T, double* zt, double* Z, cudaStream_t s);
+void launch_copula(const double* xyz, int natoms, int T, double* zt, double* Z, int* status, cudaStream_t s);
 // 3x3 co-moment blocks of every atom pair lo <= hi, summed over frames in
-// order: blk[(hi*(hi+1)/2 + lo)*9 + r*3 + c] = sum_f V[f][lo*3+r] * V[f][hi*3+c].
-void launch_blocks(const double* V, int natoms, int T, double* blk, cudaStream_t s);
+// order: blk[(hi*(hi+1)/2 + lo)*9 + r*3 + c] = sum_f v(lo, r, f) * v(hi, c, f).
+// series: V [3*natoms][T], else V [natoms][T][3].  status (optional): non-finite values.
+void launch_blocks(const double* V, bool series, int natoms, int T, double* blk, int* status, cudaStream_t s);
 // Per pair MI from the blocks.  mode 0: Gaussian (cov = sum / T, entropy
 // form); mode 1: GCMI (cov = sum * (1.0/T), log-det form).  Writes the full
 // symmetric matrix with diagonal 2000.
