@@ -11,6 +11,7 @@
 #include "ksg_fast.h"
 #include "host_common.h"
 #include "ksg_host.h"
+#include "te_host.h"
 
 #include <cuda_runtime.h>
 
@@ -122,8 +123,43 @@ void gc::host::pool_give(void* p, size_t bytes)
         cudaFree(p);
 }
 
+namespace {
+constexpr size_t           kIdleStreams = 8;
+std::vector<cudaStream_t>* g_streams    = new std::vector<cudaStream_t>[64]; // under g_pool_mutex
+} // namespace
+
+cudaStream_t gc::host::stream_take(int device)
+{
+    if (device < 0 || device >= 64)
+        return nullptr;
+    std::lock_guard<std::mutex> lock(g_pool_mutex);
+    if (g_streams[device].empty())
+        return nullptr;
+    cudaStream_t s = g_streams[device].back();
+    g_streams[device].pop_back();
+    return s;
+}
+
+void gc::host::stream_give(int device, cudaStream_t s)
+{
+    if (device >= 0 && device < 64)
+    {
+        std::lock_guard<std::mutex> lock(g_pool_mutex);
+        if (g_streams[device].size() < kIdleStreams)
+        {
+            g_streams[device].push_back(s);
+            return;
+        }
+    }
+    cudaStreamDestroy(s);
+}
+
 void gc::host::pool_release()
 {
+    for (int d = 0; d < 64; ++d)
+        while (cudaStream_t s = stream_take(d))
+            cudaStreamDestroy(s);
+
     std::multimap<size_t, void*> all[64];
     {
         std::lock_guard<std::mutex> lock(g_pool_mutex);
@@ -159,8 +195,8 @@ struct gc_ksg_plan
     PoolBuf<double>   X, psi;
     PoolBuf<uint32_t> cnt;
     PoolBuf<double>  brute; // scratch of the FP32 brute force (trajectories too long for sorted rows)
-    DevBuf<int>      status;
-    DevBuf<int2>     pair_ab; // explicit pair list as (a1, a2), empty for a range
+    PoolBuf<int>     status;
+    PoolBuf<int2>    pair_ab; // explicit pair list as (a1, a2), empty for a range
     int              launches = 0;
     cudaEvent_t      ev0 = nullptr, ev1 = nullptr;
     cudaEvent_t      ev_done = nullptr; // recorded after the last kernel of a run, on the run's stream
@@ -391,10 +427,13 @@ gc_status gc_ksg_plan_run(gc_ksg_plan* p, const double* d_xyz, double* d_pair_mi
     return plan_run(p, d_xyz, d_pair_mi, stream ? (cudaStream_t)stream : p->stream);
 }
 
-gc_status gc_ksg_plan_sync(gc_ksg_plan* p)
+} // extern "C"
+
+namespace {
+
+// Waits for the plan's last run; stats: fetch its hand-over and walk figures.
+gc_status plan_sync(gc_ksg_plan* p, bool stats)
 {
-    if (!p)
-        return fail(GC_ERR_INVALID, "null plan");
     DeviceScope dev(p->device);
     GC_TRY(dev.st);
     // The run may have been ordered on a caller's stream: wait for its last
@@ -402,8 +441,9 @@ gc_status gc_ksg_plan_sync(gc_ksg_plan* p)
     GC_TRY_CUDA(cudaEventSynchronize(p->ev_done));
     int st = 0;
     GC_TRY_CUDA(cudaMemcpy(&st, p->status.p, sizeof(int), cudaMemcpyDeviceToHost));
-    p->handoffs = 0;
-    if (p->fast)
+    if (stats)
+        p->handoffs = 0;
+    if (stats && p->fast)
     {
         unsigned long long we = 0;
         GC_TRY_CUDA(cudaMemcpy(&we, p->ft.walk_elems.p, sizeof(we), cudaMemcpyDeviceToHost));
@@ -418,6 +458,17 @@ gc_status gc_ksg_plan_sync(gc_ksg_plan* p)
     }
     st &= ~gc::kStatFallback;
     return status_to_error(st);
+}
+
+} // namespace
+
+extern "C" {
+
+gc_status gc_ksg_plan_sync(gc_ksg_plan* p)
+{
+    if (!p)
+        return fail(GC_ERR_INVALID, "null plan");
+    return plan_sync(p, true);
 }
 
 long gc_ksg_plan_pairs(const gc_ksg_plan* p) { return p ? p->pair_count : 0; }
@@ -546,6 +597,7 @@ void gc_release_cache(void)
     for (gc_ksg_plan* p : plans)
         if (p)
             gc_ksg_plan_destroy(p);
+    gc::host::te_cache_release();
     gc::host::pool_release();
 }
 
@@ -598,7 +650,7 @@ gc_status ksg_matrix_impl(const gc_traj_view* traj, const double* X, const doubl
         GC_TRY_CUDA(cudaMemcpyAsync(plan->psi.p, psi_in, sizeof(double) * ((size_t)T + 1), cudaMemcpyHostToDevice, s));
         GC_TRY(plan_run(plan.get(), nullptr, plan->io_mi.p, s));
     }
-    GC_TRY(gc_ksg_plan_sync(plan.get()));
+    GC_TRY(plan_sync(plan.get(), false));
     std::vector<double> pm((size_t)pc);
     if (pc > 0)
         GC_TRY_CUDA(cudaMemcpy(pm.data(), plan->io_mi.p, sizeof(double) * pc, cudaMemcpyDeviceToHost));
@@ -672,11 +724,11 @@ static gc_status gauss_like(const gc_traj_view* traj, const gc_opts* opts, doubl
         return fail(GC_ERR_INVALID, "gauss_corrmatrix: empty trajectory");
     DeviceScope dev(o.device);
     GC_TRY(dev.st);
-    StreamScope ss;
+    const long      nb = (long)n * (n + 1) / 2;
+    PoolBuf<double> d_xyz, d_Z, d_zt, d_blk, d_mat;
+    PoolBuf<int>    d_st;
+    StreamScope     ss;
     GC_TRY(ss.init(o.stream));
-    const long     nb = (long)n * (n + 1) / 2;
-    DevBuf<double> d_xyz, d_Z, d_zt, d_blk, d_mat;
-    DevBuf<int>    d_st;
     GC_TRY(d_xyz.alloc((size_t)n * T * 3));
     GC_TRY(d_blk.alloc((size_t)nb * 9));
     GC_TRY(d_mat.alloc((size_t)n * n));
@@ -729,10 +781,10 @@ gc_status gc_ksg_prepare(const gc_traj_view* traj, const gc_opts* opts, double* 
         return fail(GC_ERR_INVALID, "kraskov_prepare: need at least one atom and two frames");
     DeviceScope dev(o.device);
     GC_TRY(dev.st);
-    StreamScope ss;
+    PoolBuf<double> d_xyz, d_X;
+    PoolBuf<int>    d_st;
+    StreamScope     ss;
     GC_TRY(ss.init(o.stream));
-    DevBuf<double> d_xyz, d_X;
-    DevBuf<int>    d_st;
     GC_TRY(d_xyz.alloc((size_t)n * T * 3));
     GC_TRY(d_X.alloc((size_t)n * T * 3));
     GC_TRY(d_st.alloc(1));
@@ -773,14 +825,14 @@ gc_status gc_ksg_pair(const double* rows6, int nframes, int k, const double* psi
     GC_TRY(validate_ksg(2, T, k, one, &pb, &pc));
     DeviceScope dev(o.device);
     GC_TRY(dev.st);
-    StreamScope ss;
-    GC_TRY(ss.init(o.stream));
     // Two-atom system whose single pair (1, 0) has a1 = atom 1: the
     // x-marginal (first three rows, the grid's first axis) goes to atom 1.
     int cur = 0;
     GC_TRY_CUDA(cudaGetDevice(&cur));
-    DevBuf<double>   d_X, d_psi, d_mi, d_brute;
-    DevBuf<uint32_t> d_cnt;
+    PoolBuf<double>   d_X, d_psi, d_mi, d_brute;
+    PoolBuf<uint32_t> d_cnt;
+    StreamScope       ss;
+    GC_TRY(ss.init(o.stream));
     GC_TRY(d_brute.alloc(gc::ksg_brute_scratch(2) / sizeof(double) + 1));
     GC_TRY(d_X.alloc((size_t)6 * T));
     GC_TRY(d_psi.alloc((size_t)T + 1));

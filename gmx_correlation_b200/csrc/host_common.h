@@ -144,16 +144,17 @@ struct PoolBuf
         reset();
         if (count == 0)
             count = 1;
-        size_t got = 0;
-        void*  q   = pool_take(count * sizeof(T), &got);
+        const size_t want = pool_round(count * sizeof(T)); // blocks have rounded sizes
+        size_t       got  = 0;
+        void*        q    = pool_take(want, &got);
         if (!q)
         {
-            got           = pool_round(count * sizeof(T));
+            got           = want;
             cudaError_t e = cudaMalloc(&q, got);
             if (e == cudaErrorMemoryAllocation)
             {
                 cudaGetLastError();
-                pool_release(); // free what the pool holds and try once more
+                gc_release_cache(); // free what idle plans and the pool hold and try once more
                 e = cudaMalloc(&q, got);
             }
             if (e != cudaSuccess)
@@ -235,10 +236,20 @@ inline gc_status status_to_error(int st)
     return GC_OK;
 }
 
+// Per-device list of idle non-blocking streams (at most 8 a device; more are
+// destroyed): creating and destroying one costs a call about 170 us.
+// pool_release destroys the idle ones.
+cudaStream_t stream_take(int device);          // an idle stream, or nullptr
+void         stream_give(int device, cudaStream_t s);
+
+// The stream of one synchronous call: the caller's, or one of its own.  On
+// every path out of the call the stream has drained before the buffers
+// declared ahead of the scope are returned to the pool.
 struct StreamScope
 {
-    cudaStream_t s     = nullptr;
-    bool         owned = false;
+    cudaStream_t s      = nullptr;
+    bool         owned  = false;
+    int          device = -1;
     gc_status    init(void* user)
     {
         if (user)
@@ -246,13 +257,21 @@ struct StreamScope
             s = (cudaStream_t)user;
             return GC_OK;
         }
-        GC_TRY_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+        GC_TRY_CUDA(cudaGetDevice(&device));
+        s = stream_take(device);
+        if (!s)
+            GC_TRY_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
         owned = true;
         return GC_OK;
     }
     ~StreamScope()
     {
-        if (owned && s)
+        if (!s)
+            return;
+        const cudaError_t e = cudaStreamSynchronize(s);
+        if (owned && e == cudaSuccess)
+            stream_give(device, s);
+        else if (owned)
             cudaStreamDestroy(s);
     }
 };

@@ -73,9 +73,9 @@ int ksg_block_queries(int natoms, int T, double budget, int quantum = 32, double
 // fix-up over one descriptor per trajectory.
 struct KsgLaunch
 {
-    DevBuf<WalkParams>         descs;
-    DevBuf<long long>          prefix;
-    DevBuf<unsigned long long> counters;
+    PoolBuf<WalkParams>         descs;
+    PoolBuf<long long>          prefix;
+    PoolBuf<unsigned long long> counters;
     std::vector<WalkBatch>     waves;
     std::vector<long long>     wave_rows;
     std::vector<long long>     wave_queries; // row walk: queries of the wave

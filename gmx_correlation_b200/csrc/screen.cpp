@@ -461,9 +461,14 @@ gc_status gc_screen_features(const gc_traj_view* traj, int k, const gc_opts* opt
     StreamScope ss;
     GC_TRY(ss.init(o.stream));
     const int      width = pca_mean ? gc::kScreenIn : gc::kScreenBase + gc::kScreenHist;
-    DevBuf<double> d_xyz;
-    DevBuf<float>  d_out, d_pca;
-    DevBuf<int2>   d_ab;
+    PoolBuf<double> d_xyz;
+    PoolBuf<float>  d_out, d_pca;
+    PoolBuf<int2>   d_ab;
+    struct Drain // the stream has drained before the buffers return to the pool
+    {
+        cudaStream_t s;
+        ~Drain() { cudaStreamSynchronize(s); }
+    } drain{ss.s};
     GC_TRY(d_xyz.alloc((size_t)traj->natoms * traj->nframes * 3));
     GC_TRY(d_out.alloc((size_t)std::max<long>(count, 1) * width));
     GC_TRY(upload_traj(traj, d_xyz.p, ss.s));
@@ -664,8 +669,13 @@ gc_status gc_ksg_screened(const gc_traj_view* traj, int k, gc_screen_model* m, c
         }
     } evg{ev};
 
-    DevBuf<double> d_xyz;
-    DevBuf<float>  d_F, d_Y, d_mean, d_sd;
+    PoolBuf<double> d_xyz, d_mi;
+    PoolBuf<float>  d_F, d_Y, d_mean, d_sd;
+    struct Drain // the stream has drained before the buffers return to the pool
+    {
+        cudaStream_t s;
+        ~Drain() { cudaStreamSynchronize(s); }
+    } drain{s};
     GC_TRY(d_xyz.alloc((size_t)n * T * 3));
     GC_TRY(d_F.alloc((size_t)P * gc::kScreenIn));
     GC_TRY(d_Y.alloc((size_t)P * m->members));
@@ -750,7 +760,6 @@ gc_status gc_ksg_screened(const gc_traj_view* traj, int k, gc_screen_model* m, c
             gc_ksg_plan* p;
             ~PlanGuard() { gc_ksg_plan_destroy(p); }
         } pg{plan};
-        DevBuf<double> d_mi;
         GC_TRY(d_mi.alloc(list.size()));
         GC_TRY_CUDA(cudaEventRecord(ev[3], s));
         GC_TRY(gc_ksg_plan_run(plan, d_xyz.p, d_mi.p, s));

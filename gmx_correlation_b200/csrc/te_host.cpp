@@ -281,7 +281,8 @@ struct gc_te_plan
     cudaEvent_t         ev0 = nullptr, ev1 = nullptr, ev_done = nullptr;
     gc::host::TeTraj    tt;
     gc::host::TeLaunch  tl;
-    DevBuf<int>         status;
+    PoolBuf<int>        status;
+    PoolBuf<double>     io_xyz, io_te; // gc_te_matrix staging of inputs and outputs
     int                 launches = 0;
     long                handoffs = 0;
     double              walk_mean = 0.0;
@@ -379,18 +380,24 @@ gc_status gc_te_plan_run(gc_te_plan* p, const double* d_xyz, double* d_te, void*
     return GC_OK;
 }
 
-gc_status gc_te_plan_sync(gc_te_plan* p)
+} // extern "C"
+
+namespace {
+
+// Waits for the plan's last run; stats: fetch its hand-over and walk figures.
+gc_status te_sync(gc_te_plan* p, bool stats)
 {
-    if (!p)
-        return fail(GC_ERR_INVALID, "null plan");
     DeviceScope dev(p->device);
     GC_TRY(dev.st);
     GC_TRY_CUDA(cudaEventSynchronize(p->ev_done));
     int st = 0;
     GC_TRY_CUDA(cudaMemcpy(&st, p->status.p, sizeof(int), cudaMemcpyDeviceToHost));
-    p->handoffs  = 0;
-    p->walk_mean = 0.0;
-    if (p->walk)
+    if (stats)
+    {
+        p->handoffs  = 0;
+        p->walk_mean = 0.0;
+    }
+    if (stats && p->walk)
     {
         unsigned rc[8] = {};
         GC_TRY_CUDA(cudaMemcpy(rc, p->tt.reasons.p, sizeof(rc), cudaMemcpyDeviceToHost));
@@ -401,6 +408,75 @@ gc_status gc_te_plan_sync(gc_te_plan* p)
         p->walk_mean = (double)we / ((double)p->npairs * p->Nv);
     }
     return status_to_error(st & gc::kStatNonFinite);
+}
+
+// One plan per device kept by gc_te_matrix for the next call of the same
+// shape (as gc_ksg_matrix keeps one); gc_release_cache frees it.  Plans whose
+// counts exceed 4 GiB are not kept.
+struct TeKey
+{
+    int  natoms = 0, nframes = 0, k = 0, lag = 0, path = 0;
+    bool operator==(const TeKey& o) const
+    {
+        return natoms == o.natoms && nframes == o.nframes && k == o.k && lag == o.lag && path == o.path;
+    }
+};
+constexpr int kTeCacheDevices = 64;
+std::mutex&   g_te_cache_mutex = *new std::mutex;
+gc_te_plan*   g_te_cache_plan[kTeCacheDevices] = {};
+TeKey         g_te_cache_key[kTeCacheDevices];
+
+gc_te_plan* te_cache_take(int dev, const TeKey& key)
+{
+    if (dev < 0 || dev >= kTeCacheDevices)
+        return nullptr;
+    std::lock_guard<std::mutex> lock(g_te_cache_mutex);
+    if (!g_te_cache_plan[dev] || !(g_te_cache_key[dev] == key))
+        return nullptr;
+    gc_te_plan* p        = g_te_cache_plan[dev];
+    g_te_cache_plan[dev] = nullptr;
+    return p;
+}
+
+void te_cache_put(int dev, const TeKey& key, gc_te_plan* p)
+{
+    gc_te_plan* old = p;
+    if (dev >= 0 && dev < kTeCacheDevices && (double)p->npairs * p->Nv * sizeof(uint2) <= 4.0 * (1 << 30))
+    {
+        std::lock_guard<std::mutex> lock(g_te_cache_mutex);
+        old                  = g_te_cache_plan[dev];
+        g_te_cache_plan[dev] = p;
+        g_te_cache_key[dev]  = key;
+    }
+    if (old)
+        gc_te_plan_destroy(old);
+}
+
+} // namespace
+
+void gc::host::te_cache_release()
+{
+    gc_te_plan* plans[kTeCacheDevices];
+    {
+        std::lock_guard<std::mutex> lock(g_te_cache_mutex);
+        for (int d = 0; d < kTeCacheDevices; ++d)
+        {
+            plans[d]           = g_te_cache_plan[d];
+            g_te_cache_plan[d] = nullptr;
+        }
+    }
+    for (gc_te_plan* p : plans)
+        if (p)
+            gc_te_plan_destroy(p);
+}
+
+extern "C" {
+
+gc_status gc_te_plan_sync(gc_te_plan* p)
+{
+    if (!p)
+        return fail(GC_ERR_INVALID, "null plan");
+    return te_sync(p, true);
 }
 
 long gc_te_plan_pairs(const gc_te_plan* p) { return p ? p->npairs : 0; }
@@ -500,19 +576,29 @@ gc_status gc_te_matrix(const gc_traj_view* traj, int k, int lag, const gc_opts* 
         return GC_OK;
     DeviceScope dev(o.device);
     GC_TRY(dev.st);
-    // declared before the plan, so the plan (which waits for its last run)
-    // is destroyed first and these blocks return to the pool idle
-    PoolBuf<double> d_xyz, d_te;
-    gc_te_plan*     raw = nullptr;
-    GC_TRY(gc_te_plan_create(n, T, k, lag, &o, &raw));
+    int cur = -1;
+    cudaGetDevice(&cur);
+    TeKey key;
+    key.natoms  = n;
+    key.nframes = T;
+    key.k       = k;
+    key.lag     = lag;
+    key.path    = o.path;
+    gc_te_plan* raw = te_cache_take(cur, key);
+    if (!raw)
+        GC_TRY(gc_te_plan_create(n, T, k, lag, &o, &raw));
+    // destroying the plan waits for its last run, so its blocks return idle
     std::unique_ptr<gc_te_plan, void (*)(gc_te_plan*)> plan(raw, gc_te_plan_destroy);
-    GC_TRY(d_xyz.alloc((size_t)n * T * 3));
-    GC_TRY(d_te.alloc((size_t)n * n));
+    if (!plan->io_xyz.p)
+        GC_TRY(plan->io_xyz.alloc((size_t)n * T * 3));
+    if (!plan->io_te.p)
+        GC_TRY(plan->io_te.alloc((size_t)n * n));
     cudaStream_t s = o.stream ? (cudaStream_t)o.stream : plan->stream;
-    GC_TRY(upload_traj(traj, d_xyz.p, s));
-    GC_TRY(gc_te_plan_run(plan.get(), d_xyz.p, d_te.p, s));
-    GC_TRY(gc_te_plan_sync(plan.get()));
-    GC_TRY_CUDA(cudaMemcpy(te, d_te.p, sizeof(double) * (size_t)n * n, cudaMemcpyDeviceToHost));
+    GC_TRY(upload_traj(traj, plan->io_xyz.p, s));
+    GC_TRY(gc_te_plan_run(plan.get(), plan->io_xyz.p, plan->io_te.p, s));
+    GC_TRY(te_sync(plan.get(), false));
+    GC_TRY_CUDA(cudaMemcpy(te, plan->io_te.p, sizeof(double) * (size_t)n * n, cudaMemcpyDeviceToHost));
+    te_cache_put(cur, key, plan.release());
     return GC_OK;
 }
 

@@ -48,6 +48,9 @@ struct TeTraj
     gc_status prepare(const double* d_xyz, int* status, cudaStream_t s) const;
 };
 
+// Frees the plan gc_te_matrix keeps per device.
+void te_cache_release();
+
 // Sorted rows of a TE query block: bytes per query of a trajectory.
 double te_row_bytes_per_query(int natoms, int Nv);
 
@@ -56,9 +59,9 @@ double te_row_bytes_per_query(int natoms, int Nv);
 // of the fix-up over one descriptor per trajectory.
 struct TeLaunch
 {
-    DevBuf<TeParams>           descs;
-    DevBuf<long long>          prefix;
-    DevBuf<unsigned long long> counters;
+    PoolBuf<TeParams>           descs;
+    PoolBuf<long long>          prefix;
+    PoolBuf<unsigned long long> counters;
     std::vector<TeBatch>       waves;
     std::vector<long long>     wave_rows;
     TeBatch                    fix{};
