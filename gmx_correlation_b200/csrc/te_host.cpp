@@ -101,6 +101,13 @@ gc_status TeTraj::create(int n, int nframes, int k, int lg, int q, bool own_rows
         GC_TRY(PM.alloc(rows));
     }
     GC_TRY(wres.alloc((size_t)Q * npairs));
+    orderG.reset();
+    orderM.reset();
+    if (te_row_walk_fits(n, Nv, k))
+    {
+        GC_TRY(orderG.alloc((size_t)Q * n));
+        GC_TRY(orderM.alloc((size_t)Q * n));
+    }
     const double hq_want = 0.01 * (double)npairs * Nv + 4096.0;
     hq_cap               = (unsigned)(hq_want < 16777216.0 ? hq_want : 16777216.0);
     GC_TRY(hq.alloc(hq_cap));
@@ -143,6 +150,8 @@ TeParams TeTraj::desc(int* status, int b) const
     d.status     = status;
     d.walk_elems = walk_elems.p;
     d.reasons    = reasons.p;
+    d.orderG     = orderG.p;
+    d.orderM     = orderM.p;
     return d;
 }
 
@@ -180,9 +189,13 @@ gc_status TeTraj::prepare(const double* d_xyz, int* status, cudaStream_t s) cons
 gc_status TeLaunch::build(const std::vector<std::vector<TeParams>>& wave_descs, const std::vector<TeParams>& traj_descs)
 {
     int maxT = 0, maxNv = 0, maxK = 0;
+    row_walk  = true;
+    max_atoms = 0;
     for (const auto& wv : wave_descs)
         for (const TeParams& d : wv)
         {
+            row_walk  = row_walk && d.orderG != nullptr;
+            max_atoms = std::max(max_atoms, d.natoms);
             maxT  = std::max(maxT, d.T);
             maxNv = std::max(maxNv, d.Nv);
             maxK  = std::max(maxK, d.K);
@@ -196,7 +209,7 @@ gc_status TeLaunch::build(const std::vector<std::vector<TeParams>>& wave_descs, 
     {
         dofs.push_back(all.size());
         pofs.push_back(pre.size());
-        std::vector<long long> rp{0}, wp{0}, fp{0};
+        std::vector<long long> rp{0}, wp{0}, fp{0}, qp{0}, up{0}, vp{0};
         for (const TeParams& d : wv)
         {
             all.push_back(d);
@@ -204,10 +217,17 @@ gc_status TeLaunch::build(const std::vector<std::vector<TeParams>>& wave_descs, 
             rp.push_back(rp.back() + 2LL * d.natoms * d.Q);
             wp.push_back(wp.back() + (grp + chunk - 1) / chunk * d.pair_count);
             fp.push_back(fp.back() + grp * d.pair_count);
+            const long long blocks = (long long)d.Q * ((d.natoms + 31) / 32);
+            qp.push_back(qp.back() + d.Q);
+            up.push_back(up.back() + 2 * blocks);
+            vp.push_back(vp.back() + blocks);
         }
         pre.insert(pre.end(), rp.begin(), rp.end());
         pre.insert(pre.end(), wp.begin(), wp.end());
         pre.insert(pre.end(), fp.begin(), fp.end());
+        pre.insert(pre.end(), qp.begin(), qp.end());
+        pre.insert(pre.end(), up.begin(), up.end());
+        pre.insert(pre.end(), vp.begin(), vp.end());
     }
     const size_t tofs = all.size();
     all.insert(all.end(), traj_descs.begin(), traj_descs.end());
@@ -218,6 +238,7 @@ gc_status TeLaunch::build(const std::vector<std::vector<TeParams>>& wave_descs, 
     GC_TRY_CUDA(cudaMemcpy(prefix.p, pre.data(), sizeof(long long) * pre.size(), cudaMemcpyHostToDevice));
     waves.clear();
     wave_rows.clear();
+    wave_queries.clear();
     for (size_t v = 0; v < wave_descs.size(); ++v)
     {
         const int n = (int)wave_descs[v].size();
@@ -226,6 +247,9 @@ gc_status TeLaunch::build(const std::vector<std::vector<TeParams>>& wave_descs, 
         b.rprefix = prefix.p + pofs[v];
         b.wprefix = b.rprefix + (n + 1);
         b.fprefix = b.wprefix + (n + 1);
+        b.qprefix = b.fprefix + (n + 1);
+        b.uprefix = b.qprefix + (n + 1);
+        b.vprefix = b.uprefix + (n + 1);
         b.n       = n;
         b.maxT    = maxT;
         b.maxNv   = maxNv;
@@ -234,6 +258,7 @@ gc_status TeLaunch::build(const std::vector<std::vector<TeParams>>& wave_descs, 
         b.counter = counters.p + 2 * v;
         waves.push_back(b);
         wave_rows.push_back(pre[pofs[v] + n]);
+        wave_queries.push_back(pre[pofs[v] + 3 * ((size_t)n + 1) + n]);
     }
     fix       = TeBatch{};
     fix.d     = descs.p + tofs;
@@ -251,13 +276,20 @@ gc_status TeLaunch::enqueue(int sms, cudaStream_t s)
         GC_TRY_CUDA(cudaMemsetAsync(counters.p, 0, sizeof(unsigned long long) * 2 * waves.size(), s));
     for (const TeBatch& w : waves)
     {
-        GC_TRY_CUDA(gc::launch_te_rows(w, wave_rows[(size_t)(&w - waves.data())], s));
-        GC_TRY_CUDA(gc::launch_te_walk(w, warps, staged, sms, s));
+        const size_t v = (size_t)(&w - waves.data());
+        GC_TRY_CUDA(gc::launch_te_rows(w, wave_rows[v], s));
+        if (row_walk)
+            GC_TRY_CUDA(gc::launch_te_row_walk(w, wave_queries[v], max_atoms, sms, s));
+        else
+            GC_TRY_CUDA(gc::launch_te_walk(w, warps, staged, sms, s));
         GC_TRY_CUDA(gc::launch_te_finish(w, sms, s));
         // the walk's task counter serves the count kernel
         GC_TRY_CUDA(cudaMemsetAsync(w.counter, 0, sizeof(unsigned long long), s));
-        GC_TRY_CUDA(gc::launch_te_count(w, warps, staged, sms, s));
-        launches += 4;
+        if (row_walk && te_row_count_fits(w.maxNv))
+            GC_TRY_CUDA(gc::launch_te_row_count(w, wave_queries[v], sms, s));
+        else
+            GC_TRY_CUDA(gc::launch_te_count(w, warps, staged, sms, s));
+        launches += row_walk ? 5 : 4;
     }
     if (fix.n > 0)
     {

@@ -30,6 +30,7 @@ struct TeTraj
     PoolBuf<unsigned long long> wres, hq, walk_elems;
     PoolBuf<unsigned>           hq_len, reasons;
     PoolBuf<int>                pair_order;
+    PoolBuf<uint2>              orderG, orderM; // the row walk's atom orders (empty where it does not run)
 
     // Q > 0: the walk's workspace for query blocks of Q queries; Q == 0: the
     // brute-force kernels' (coordinates, counts and digamma table only).
@@ -63,7 +64,9 @@ struct TeLaunch
     PoolBuf<long long>          prefix;
     PoolBuf<unsigned long long> counters;
     std::vector<TeBatch>       waves;
-    std::vector<long long>     wave_rows;
+    std::vector<long long>     wave_rows, wave_queries;
+    bool                       row_walk = false; // walk and count by rows (te_row_walk.cu)
+    int                        max_atoms = 0;
     TeBatch                    fix{};
     int                        warps = 0;
     bool                       staged = false;

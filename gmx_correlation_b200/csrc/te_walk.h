@@ -48,6 +48,9 @@ struct TeParams
     int*                status;
     unsigned long long* walk_elems; // optional: total walked row entries
     unsigned*           reasons;    // optional [8]: hand-overs by cause
+    // where the row walk runs (else null): the block's atoms by ascending k-th
+    // value of their G and of their M rows, [Q][natoms] (atom, bits of the value)
+    uint2 *orderG, *orderM;
 };
 
 constexpr uint32_t kTeHandOver = 0xFFFFFFFFu;
@@ -63,6 +66,9 @@ struct TeBatch
     const long long*    rprefix; // [n + 1] row-sort tasks: 2 * natoms * Q per descriptor
     const long long*    wprefix; // [n + 1] walk tasks: ceil(groups / chunk) * pairs
     const long long*    fprefix; // [n + 1] finish tasks: query groups * pairs
+    const long long*    qprefix; // [n + 1] queries
+    const long long*    uprefix; // [n + 1] row-walk tasks: 2 Q * ceil(natoms / 32)
+    const long long*    vprefix; // [n + 1] row-count tasks: Q * ceil(natoms / 32)
     int                 n;
     int                 maxT;  // largest frame count (shared-memory layout)
     int                 maxNv; // largest row length + 1
@@ -76,6 +82,14 @@ cudaError_t launch_te_walk(const TeBatch& b, int warps, bool staged, int sms, cu
 cudaError_t launch_te_finish(const TeBatch& b, int sms, cudaStream_t s);
 // n_ypxp of every (pair, query) the finish settled (its walk launch shape).
 cudaError_t launch_te_count(const TeBatch& b, int warps, bool staged, int sms, cudaStream_t s);
+// The walk and the count by rows (te_row_walk.cu) of descriptors with orders;
+// queries: qprefix[n], maxn: the most atoms of a descriptor.
+cudaError_t launch_te_row_walk(const TeBatch& b, long long queries, int maxn, int sms, cudaStream_t s);
+cudaError_t launch_te_row_count(const TeBatch& b, long long queries, int sms, cudaStream_t s);
+// Whether the walk takes a trajectory of this shape (as row_walk_fits), and
+// whether the count, with its 16-bit tile, does then (up to about 3,200 frames).
+bool te_row_walk_fits(int natoms, int Nv, int k);
+bool te_row_count_fits(int Nv);
 // Exact FP64 statistics of every queued hand-over of the trajectories'
 // descriptors, then of any mark a full queue could not hold.
 cudaError_t launch_te_fixup(const TeBatch& b, int sms, cudaStream_t s);

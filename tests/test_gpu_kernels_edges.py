@@ -38,6 +38,16 @@ def test_row_walk_equals_exact(gc, n, T, k, kind):
     np.testing.assert_array_equal(a, b)
 
 
+@pytest.mark.parametrize("n,T,k,lag,kind", [
+    (24, 40, 1, 1, "smooth"), (25, 60, 38, 5, "smooth"), (32, 130, 6, 0, "ties"), (33, 200, 12, 3, "smooth"),
+    (65, 150, 10, 1, "tails"), (40, 400, 9, 10, "duplicates"), (30, 1500, 100, 1, "smooth"),
+    (24, 900, 255, 2, "smooth"), (24, 800, 254, 2, "smooth"), (24, 6000, 20, 1, "smooth"),
+])
+def test_te_rows_equal_exact(gc, n, T, k, lag, kind):
+    x = _traj(kind, n, T, seed=n + T)
+    np.testing.assert_array_equal(gc.te_matrix(x, k, lag), gc.te_matrix(x, k, lag, path=gc.PATH_EXACT_FP64))
+
+
 @pytest.mark.parametrize("T,k,kind", [
     (20, 1, "smooth"), (33, 32, "smooth"), (500, 10, "ties"), (700, 40, "duplicates"), (2047, 100, "smooth"),
     (2048, 300, "smooth"), (2049, 6, "tails"), (4097, 50, "smooth"), (5000, 4999, "smooth"),
