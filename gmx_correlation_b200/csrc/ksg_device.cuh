@@ -59,7 +59,7 @@ enum
     kReasonRange    = 2, // k-th value beyond the histogram's two octaves
     kReasonBand     = 3, // band larger than kBandCap or inconsistent with the histogram
     kReasonAmbig    = 4, // ambiguous set inconsistent or larger than kAmbCap
-    kReasonScan     = 5, // backward scan for the maxima exceeded kScanCap
+    kReasonScan     = 5, // scan for the maxima or their counts exceeded kScanCap
     kReasonPrefix   = 6  // count band reaches beyond the walked prefix
 };
 

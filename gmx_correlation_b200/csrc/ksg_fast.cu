@@ -9,8 +9,9 @@
 //   ksg_x32_kernel    FP32 copy of the normalised coordinates, centred per
 //                     component, and a per-atom bound eps_a with
 //                     |d32 - d64| <= eps_a for every marginal distance.
-//   ksg_rows_kernel   per (atom, query): the T-1 marginal distances, sorted
-//                     ascending, with their frame indices (S rows, P rows).
+//   ksg_rows_kernel   per (atom, query): the T-1 marginal distances in the
+//                     order of narrow buckets, with their frames (S rows,
+//                     P rows; row_sort.cuh).
 //   ksg_walk_kernel   one pair per CTA task, 32 consecutive queries per warp,
 //                     one query per lane.  Each lane walks the sorted row of the
 //                     marginal whose k-th distance is larger, gathering the
@@ -25,9 +26,9 @@
 //                     decision is re-evaluated in FP64 on the reference's
 //                     normalised coordinates, with the reference's grid-scan
 //                     order deciding exact ties, so n_x and n_y equal the
-//                     reference's counts.  Counts come from binary search in
-//                     the sorted rows, with FP64 repair of the band around
-//                     eps_x / eps_y.
+//                     reference's counts.  A count is what lies before the
+//                     maximum's fine bucket plus that bucket's entries up to
+//                     it, in FP64 where others are within 2 eps of it.
 //   ksg_fixup_kernel  queries a lane hands over (k-th value outside the
 //                     histogram, oversized bands) are marked in the count
 //                     array and recomputed here by the exact FP64 code.
@@ -79,10 +80,10 @@ __global__ void ksg_x32_kernel(const double* __restrict__ X64, int natoms, int T
 }
 
 // One CTA per (atom, query) of the launch's query blocks: the row's T-1
-// marginal distances (self excluded), sorted ascending with their frames
+// marginal distances (self excluded) in bucket order with their frames
 // (sort_row).
 template <int THREADS, int R>
-__global__ void __launch_bounds__(THREADS) ksg_rows_kernel(WalkBatch B)
+__global__ void __launch_bounds__(THREADS, THREADS == 256 ? 6 : (THREADS == 512 ? 2 : 1)) ksg_rows_kernel(WalkBatch B)
 {
     // row blockIdx.x of the launch -> descriptor, atom, query of its block
     const long long   r   = blockIdx.x;
@@ -97,8 +98,8 @@ __global__ void __launch_bounds__(THREADS) ksg_rows_kernel(WalkBatch B)
     const float4      q   = xr[i];
     __shared__ RowSortShared<THREADS> sh;
     sort_row<THREADS, R>(
-        sh, T - 1, i, [&](int j) { return dist3f(q, xr[j]); }, w.S, w.P, ((size_t)a * (Lpad >> 2) * Qp + iq) * 4,
-        (size_t)Qp * 4, w.U ? w.U + ((size_t)a * Qp + iq) * w.Tpad : nullptr);
+        sh, T - 1, i, row_top(w.eps_atom[a]), [&](int j) { return dist3f(q, xr[j]); }, w.S, w.P,
+        ((size_t)a * (Lpad >> 2) * Qp + iq) * 4, (size_t)Qp * 4, w.U ? w.U + ((size_t)a * Qp + iq) * w.Tpad : nullptr);
 }
 
 namespace {
@@ -114,35 +115,31 @@ __device__ __forceinline__ unsigned u2get16(const uint2& v, int q)
     return q < 2 ? ((v.x >> (16 * q)) & 0xFFFFu) : ((v.y >> (16 * (q - 2))) & 0xFFFFu);
 }
 
-// Four independent binary searches advanced together, so their loads
-// overlap: lo[q] becomes the first position in [lo[q], hi[q]] of row r[q]
-// whose value is not < t[q] (strict[q]) / not <= t[q].
-__device__ __forceinline__ void row_bounds4(const LaneRow (&r)[4], int (&lo)[4], int (&hi)[4], const float (&t)[4],
-                                            const bool (&strict)[4])
+// Two independent binary searches advanced together, so their loads overlap:
+// lo[q] becomes the first position in [lo[q], hi[q]] of row r[q] whose value
+// is not < t.  Rows are in fine-bucket order, so t is the first value of a
+// fine bucket.
+__device__ __forceinline__ void row_bounds2(const LaneRow (&r)[2], int (&lo)[2], int (&hi)[2], float t)
 {
-    for (;;)
+    while (lo[0] < hi[0] || lo[1] < hi[1])
     {
-        int   mid[4];
-        float v[4];
-        bool  any = false;
+        int   mid[2];
+        float v[2];
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
+        for (int q = 0; q < 2; ++q)
         {
             mid[q] = (lo[q] + hi[q]) >> 1;
             v[q]   = lo[q] < hi[q] ? r[q].s(mid[q]) : 0.0f;
         }
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
+        for (int q = 0; q < 2; ++q)
             if (lo[q] < hi[q])
             {
-                if (strict[q] ? v[q] < t[q] : v[q] <= t[q])
+                if (v[q] < t)
                     lo[q] = mid[q] + 1;
                 else
                     hi[q] = mid[q];
-                any |= lo[q] < hi[q];
             }
-        if (!any)
-            break;
     }
 }
 
@@ -680,100 +677,114 @@ __global__ void __launch_bounds__(kFinishWarps * 32, 1) ksg_finish_kernel(WalkBa
             const float    ew = u.ew, eo = u.eo, e2 = u.e2;
             if (reason == 0)
             {
-                // ---- band: every entry with inlo <= v <= bandhi, from two row ranges
-                const float elo    = __uint_as_float(Lb + ((unsigned)bstar << shift));
-                const float ehi    = __uint_as_float(Lb + ((unsigned)(bstar + 1) << shift));
-                const float inlo   = __fsub_rd(elo, e2);
-                const float bandhi = __fadd_ru(ehi, e2);
-                if (m_end < Llen && rw.s(m_end) <= bandhi)
-                    reason = kReasonPrefix;
-                const LaneRow rr[4] = {rw, rw, ro, ro};
-                int           lo[4] = {0, 0, 0, 0}, hi[4] = {m_end, m_end, Llen, Llen};
-                const float   tt[4] = {inlo, bandhi, inlo, bandhi};
-                const bool    st[4] = {true, false, true, false};
-                row_bounds4(rr, lo, hi, tt, st);
-                const int mw0 = lo[0], mw1 = lo[1], mo0 = lo[2], mo1 = lo[3];
-                int       nband = 0, nlo = 0;
-                auto add = [&](float v, float sv, float dv, int off) {
-                    if (nband < kBandCap)
-                    {
-                        bv[nband * 32] = v;
-                        bs[nband * 32] = sv;
-                        bd[nband * 32] = dv;
-                        bo[nband * 32] = (uint16_t)off;
-                    }
-                    ++nband;
-                    nlo += v < elo;
-                };
-                // Both ranges by aligned 4-entry groups of the row (one 16-byte
-                // and one 8-byte load per group),
-                // the next group's loads in flight while this one gathers.
+                // ---- band: the joint values in the k-th value's bucket, from the
+                // bucket's entries of the two rows.  When the k-th value lies within
+                // 2 eps of the bucket's edges the band is taken again with 2 eps more
+                // on both sides (from whole fine buckets of each row).
+                const unsigned bhi = Lb + ((unsigned)(bstar + 1) << shift);
+                const float    elo = __uint_as_float(Lb + ((unsigned)bstar << shift)), ehi = __uint_as_float(bhi);
+                float          inlo = elo, bandhi = __uint_as_float(bhi - 1u); // the band [inlo, bandhi]
+                bool           wide = false;
+                // where the band's entries start and end in the rows, and those below
+                // the bucket end: the joint values below it lie below it in both rows,
+                // and the walk went beyond it
+                int   mw0 = 0, mo0 = 0, mw1 = 0, mo1 = 0;
+                int   below_w = min(prefix, Llen), below_o = below_w;
+                int   nband = 0, nW = 0, n_in = 0;
+                float lower = 0.0f, upper = 0.0f;
+                for (;;)
                 {
-                    int    g  = min(mw0, Llen - 1) >> 2;
-                    float4 s4 = rw.s4(g);
-                    uint2  j4 = rw.j4(g);
-                    while (g * 4 < mw1) // s in the band, d <= bandhi
+                    const LaneRow rr[2] = {rw, ro};
+                    int           lo[2] = {wide ? 0 : below_w, wide ? 0 : below_o};
+                    int           hi[2] = {wide ? below_w : m_end, wide ? below_o : Llen};
+                    row_bounds2(rr, lo, hi, fine_start(fmaxf(inlo, 0.0f)));
+                    mw0 = lo[0];
+                    mo0 = lo[1];
+                    if (!wide)
                     {
-                        const int    gn = (g + 1) * 4 < mw1 ? g + 1 : g;
-                        const float4 ns = rw.s4(gn);
-                        const uint2  nj = rw.j4(gn);
-#pragma unroll
-                        for (int q = 0; q < 4; ++q)
+                        below_w = mw0;
+                        below_o = mo0;
+                    }
+                    int nlo = 0;
+                    nband   = 0;
+                    auto add = [&](float v, float sv, float dv, int off) {
+                        if (nband < kBandCap)
                         {
-                            const int   mm = g * 4 + q;
-                            const bool  in = mm >= mw0 && mm < mw1;
-                            const int   j  = (int)u2get16(j4, q);
-                            const float sv = f4get(s4, q);
-                            const float dv = dist3f(xo, X32o[in ? j : 0]);
-                            if (in && dv <= bandhi)
-                                add(fmaxf(sv, dv), sv, dv, mm - mw0);
+                            bv[nband * 32] = v;
+                            bs[nband * 32] = sv;
+                            bd[nband * 32] = dv;
+                            bo[nband * 32] = (uint16_t)off;
                         }
-                        ++g;
-                        s4 = ns;
-                        j4 = nj;
-                    }
-                }
-                const int nW = nband; // band entries from the walked row come first
-                {
-                    int    g  = min(mo0, Llen - 1) >> 2;
-                    float4 d4 = ro.s4(g);
-                    uint2  j4 = ro.j4(g);
-                    while (g * 4 < mo1) // d in the band, s < inlo
+                        ++nband;
+                        nlo += v < elo;
+                    };
+                    // Both ranges by aligned 4-entry groups of the row (one 16-byte
+                    // and one 8-byte load per group), the next group's loads in flight
+                    // while this one gathers, until a group ends beyond bandhi's fine
+                    // bucket.  NaN behind the row: not in the band.
                     {
-                        const int    gn = (g + 1) * 4 < mo1 ? g + 1 : g;
-                        const float4 nd = ro.s4(gn);
-                        const uint2  nj = ro.j4(gn);
-#pragma unroll
-                        for (int q = 0; q < 4; ++q)
+                        int    g    = min(mw0, Llen - 1) >> 2;
+                        float4 s4   = rw.s4(g);
+                        uint2  j4   = rw.j4(g);
+                        bool   more = true;
+                        while (more) // s in the band, d <= bandhi
                         {
-                            const int   mm = g * 4 + q;
-                            const bool  in = mm >= mo0 && mm < mo1;
-                            const int   j  = (int)u2get16(j4, q);
-                            const float dv = f4get(d4, q);
-                            const float sv = dist3f(xw, X32w[in ? j : 0]);
-                            if (in && sv < inlo)
-                                add(dv, sv, dv, mm - mo0);
+                            more            = (g + 1) * 4 < Llen && fine_start(s4.w) <= bandhi;
+                            const int    gn = more ? g + 1 : g;
+                            const float4 ns = rw.s4(gn);
+                            const uint2  nj = rw.j4(gn);
+#pragma unroll
+                            for (int q = 0; q < 4; ++q)
+                            {
+                                const float sv = f4get(s4, q);
+                                const bool  in = sv >= inlo && sv <= bandhi;
+                                const int   j  = (int)u2get16(j4, q);
+                                const float dv = dist3f(xo, X32o[in ? j : 0]);
+                                if (in && dv <= bandhi)
+                                    add(fmaxf(sv, dv), sv, dv, g * 4 + q - mw0);
+                            }
+                            ++g;
+                            s4 = ns;
+                            j4 = nj;
                         }
-                        ++g;
-                        d4 = nd;
-                        j4 = nj;
+                        mw1 = min(g * 4, Llen);
                     }
-                }
-                // frame of band entry e (for the FP64 paths)
-                auto band_frame = [&](int e) -> int {
-                    return e < nW ? rw.j(mw0 + bo[e * 32]) : ro.j(mo0 + bo[e * 32]);
-                };
-                int       n_in = prefix - nlo; // #{v < inlo}
-                const int r    = K - n_in;     // 1-based rank of the k-th value in the band
-                if (!reason && (nband > kBandCap || r < 1 || r > nband))
-                    reason = kReasonBand;
-
-                // ---- the k-th FP32 value; certain members and the ambiguous set ---
-                unsigned amb  = 0u;
-                float    lower = 0.0f;
-                int      need  = 0;
-                if (!reason)
-                {
+                    nW = nband; // band entries from the walked row come first
+                    {
+                        int    g    = min(mo0, Llen - 1) >> 2;
+                        float4 d4   = ro.s4(g);
+                        uint2  j4   = ro.j4(g);
+                        bool   more = true;
+                        while (more) // d in the band, s < inlo
+                        {
+                            more            = (g + 1) * 4 < Llen && fine_start(d4.w) <= bandhi;
+                            const int    gn = more ? g + 1 : g;
+                            const float4 nd = ro.s4(gn);
+                            const uint2  nj = ro.j4(gn);
+#pragma unroll
+                            for (int q = 0; q < 4; ++q)
+                            {
+                                const float dv = f4get(d4, q);
+                                const bool  in = dv >= inlo && dv <= bandhi;
+                                const int   j  = (int)u2get16(j4, q);
+                                const float sv = dist3f(xw, X32w[in ? j : 0]);
+                                if (in && sv < inlo)
+                                    add(dv, sv, dv, g * 4 + q - mo0);
+                            }
+                            ++g;
+                            d4 = nd;
+                            j4 = nj;
+                        }
+                        mo1 = min(g * 4, Llen);
+                    }
+                    n_in        = prefix - nlo; // #{v < inlo}
+                    const int r = K - n_in;     // 1-based rank of the k-th value in the band
+                    if (nband > kBandCap || r < 1 || r > nband)
+                    {
+                        reason = kReasonBand;
+                        break;
+                    }
+                    // ---- the k-th FP32 value
                     float d32 = 0.0f;
                     for (int e = 0; e < nband; ++e)
                     {
@@ -790,8 +801,24 @@ __global__ void __launch_bounds__(kFinishWarps * 32, 1) ksg_finish_kernel(WalkBa
                             break;
                         }
                     }
-                    lower             = __fsub_rd(d32, e2);
-                    const float upper = __fadd_ru(d32, e2);
+                    lower = __fsub_rd(d32, e2);
+                    upper = __fadd_ru(d32, e2);
+                    if (wide || (lower >= inlo && upper <= bandhi))
+                        break;
+                    wide   = true;
+                    inlo   = __fsub_rd(elo, e2);
+                    bandhi = __fadd_ru(ehi, e2);
+                }
+                // frame of band entry e (for the FP64 paths)
+                auto band_frame = [&](int e) -> int {
+                    return e < nW ? rw.j(mw0 + bo[e * 32]) : ro.j(mo0 + bo[e * 32]);
+                };
+
+                // ---- certain members and the ambiguous set ------------------------
+                unsigned amb  = 0u;
+                int      need = 0;
+                if (!reason)
+                {
                     for (int e = 0; e < nband; ++e)
                     {
                         const float v = bv[e * 32];
@@ -804,14 +831,6 @@ __global__ void __launch_bounds__(kFinishWarps * 32, 1) ksg_finish_kernel(WalkBa
                     if (need < 1 || need > __popc(amb))
                         reason = kReasonAmbig;
                 }
-
-                // ---- marginal maxima over the members, then the counts -----------
-                // Fast path: when no other member lies within 2 eps below the
-                // FP32 maximum member of a marginal, that member holds the FP64
-                // maximum; when no other row entry lies within 2 eps of it
-                // either, its row position gives the count.  Otherwise every
-                // member within 2 eps gets an FP64 look and an FP64-repaired
-                // binary search counts.
                 const double* xa64 = p.X64 + (size_t)a1 * 3 * T;
                 const double* xb64 = p.X64 + (size_t)a2 * 3 * T;
                 const double* xw64 = wx ? xa64 : xb64;
@@ -853,6 +872,13 @@ __global__ void __launch_bounds__(kFinishWarps * 32, 1) ksg_finish_kernel(WalkBa
                         }
                     }
                 }
+
+                // ---- marginal maxima over the members, then the counts -----------
+                // The FP32 maximum member's own fine bucket (and any other within
+                // 2 eps of it) is looked through: its entries up to the maximum plus
+                // everything before it is the count, unless another entry of the row
+                // lies within 2 eps.  Then every member within 2 eps gets an FP64
+                // look and the entries within the bound are counted in FP64.
                 int ncount[2] = {0, 0}; // counts of the walked and the other marginal
                 int steps     = 0;
                 for (int side = 0; side < 2 && !reason; ++side)
@@ -862,138 +888,151 @@ __global__ void __launch_bounds__(kFinishWarps * 32, 1) ksg_finish_kernel(WalkBa
                     const float4   xc   = side == 0 ? xo : xw;
                     const double*  x64  = side == 0 ? xw64 : xo64;
                     const float    eps  = side == 0 ? ew : eo;
+                    const float    eps2 = __fmul_ru(2.0f, eps);
                     const float*   bval = side == 0 ? bs : bd;
                     // band members
-                    float top = -1.0f, sec = -1.0f;
+                    float top  = -1.0f;
                     int   ptop = -1;
                     for (int e = 0; e < nband; ++e)
                     {
                         if (!(bv[e * 32] < lower || ((amem >> e) & 1u)))
                             continue;
-                        const float val  = bval[e * 32];
+                        const float val = bval[e * 32];
                         // row position of the entry in this side's row (-1: other row)
-                        const int   prow = (side == 0) == (e < nW) ? (side == 0 ? mw0 : mo0) + bo[e * 32] : -1;
+                        const int prow = (side == 0) == (e < nW) ? (side == 0 ? mw0 : mo0) + bo[e * 32] : -1;
                         if (val > top)
                         {
-                            sec  = top;
                             top  = val;
                             ptop = prow;
                         }
-                        else if (val > sec)
-                            sec = val;
                     }
-                    // members with v < inlo: the first one below the band start
-                    // in this row holds their maximum (a 4-entry group per round).
-                    // Row values below the band start are < inlo, so when a band
-                    // member already tops inlo by 2 eps they can neither be the
-                    // maximum nor lie within 2 eps of it: no scan.
-                    const bool settled = top >= 0.0f && __fsub_rd(top, __fmul_ru(2.0f, eps)) >= inlo;
-                    int        mm = (side == 0 ? mw0 : mo0) - 1, first = -1;
-                    float      fval = -1.0f, fsec = -1.0f;
-                    while (!settled && mm >= 0 && first < 0)
+                    // members with v < inlo: the first one below the band start in this
+                    // row tells the fine bucket that holds their maximum (a 4-entry
+                    // group per round).  Not needed when a band member is above them.
+                    const int below = side == 0 ? below_w : below_o;
+                    for (int mm = top >= inlo ? -1 : below - 1; mm >= 0;)
                     {
                         const int    g  = mm >> 2;
                         const float4 s4 = row.s4(g);
                         const uint2  j4 = row.j4(g);
-                        bool         ok[4];
+#pragma unroll
+                        for (int q = 3; q >= 0; --q)
+                        {
+                            const float s  = f4get(s4, q);
+                            const bool  in = g * 4 + q <= mm && s < inlo && s > top;
+                            if (dist3f(xc, Xc[in ? u2get16(j4, q) : 0u]) < inlo && in)
+                            {
+                                top  = s;
+                                ptop = g * 4 + q;
+                            }
+                        }
+                        steps += mm - g * 4 + 1;
+                        mm = g * 4 - 1; // the next unexamined position
+                        if (top >= 0.0f && fine_after(s4.x) <= top) // only smaller values from here
+                            break;
+                        if (mm >= 0 && steps > kScanCap)
+                        {
+                            reason = kReasonScan;
+                            break;
+                        }
+                    }
+                    if (reason)
+                        break;
+                    const float tie = __fsub_rd(top, eps2);
+                    const float chi = __fadd_ru(top, eps2);
+                    if (ptop < 0) // listed in the other row: from its fine bucket's start
+                    {
+                        int lo = 0, hi = below;
+                        if (top >= elo)
+                            lo = below, hi = side == 0 ? mw1 : mo1;
+                        const float t = fine_start(top);
+                        while (lo < hi)
+                        {
+                            const int mid = (lo + hi) >> 1;
+                            if (row.s(mid) < t)
+                                lo = mid + 1;
+                            else
+                                hi = mid;
+                        }
+                        ptop = min(lo, Llen - 1);
+                    }
+                    // groups around ptop until the fine buckets lie outside tie .. chi:
+                    // entries up to top, and those within 2 eps of it
+                    int g0 = ptop >> 2, g1 = g0 + 1, le = 0, near = 0;
+                    for (bool up = false;;)
+                    {
+                        const int    g  = up ? g1 : g0;
+                        const float4 s4 = row.s4(g);
 #pragma unroll
                         for (int q = 0; q < 4; ++q)
                         {
-                            const bool in = g * 4 + q <= mm;
-                            ok[q] = in && dist3f(xc, Xc[in ? u2get16(j4, q) : 0u]) < inlo;
+                            const float s = f4get(s4, q); // NaN behind the row: neither
+                            le += s <= top;
+                            near += s >= tie && s <= chi;
                         }
-#pragma unroll
-                        for (int q = 3; q >= 0; --q)
-                            if (ok[q])
-                            {
-                                if (first < 0)
-                                {
-                                    first = g * 4 + q;
-                                    fval  = f4get(s4, q);
-                                }
-                                else
-                                    fsec = fmaxf(fsec, f4get(s4, q));
-                            }
-                        steps += mm - g * 4 + 1;
-                        mm = g * 4 - 1; // the next unexamined position
-                        if (first < 0 && steps > kScanCap)
-                            reason = kReasonScan;
-                    }
-                    if (reason)
-                        break;
-                    if (first >= 0)
-                    {
-                        if (fval > top)
+                        steps += 4;
+                        if (!up)
                         {
-                            sec  = fmaxf(sec, top);
-                            top  = fval;
-                            ptop = first;
+                            if (g0 > 0 && fine_after(s4.x) > tie)
+                            {
+                                --g0;
+                                continue;
+                            }
+                            up = true;
+                            if (!(fine_start(f4get(row.s4(g1 - 1), 3)) <= chi) || g1 * 4 >= Llen)
+                                break;
                         }
                         else
-                            sec = fmaxf(sec, fval);
-                        sec = fmaxf(sec, fsec);
-                    }
-                    const float tie = __fsub_rd(top, __fmul_ru(2.0f, eps));
-                    const float chi = __fadd_ru(top, __fmul_ru(2.0f, eps));
-                    // members below the examined entries that are still within 2 eps
-                    for (; first >= 0 && mm >= 0; --mm)
-                    {
-                        const float sv = row.s(mm);
-                        if (sv < tie)
-                            break;
-                        if (++steps > kScanCap)
+                        {
+                            ++g1;
+                            if (!(fine_start(s4.w) <= chi) || g1 * 4 >= Llen)
+                                break;
+                        }
+                        if (steps > kScanCap)
                         {
                             reason = kReasonScan;
                             break;
                         }
-                        if (dist3f(xc, Xc[row.j(mm)]) < inlo)
-                            sec = fmaxf(sec, sv);
                     }
                     if (reason)
                         break;
-                    bool fast = ptop >= 0 && sec < tie;
-                    if (fast && ptop > 0 && row.s(ptop - 1) >= tie)
-                        fast = false;
-                    if (fast && ptop + 1 < Llen && row.s(ptop + 1) <= chi)
-                        fast = false;
-                    if (fast)
+                    if (near == 1)
                     {
-                        ncount[side] = ptop + 1;
+                        ncount[side] = g0 * 4 + le;
                         continue;
                     }
-                    // FP64 maximum over every member within 2 eps of top
+                    // FP64 maximum over every member within 2 eps of top, then the
+                    // entries below that range and, in FP64, those in it
                     const double q0 = x64[i], q1 = x64[T + i], q2 = x64[2 * T + i];
                     double       best = -1.0;
                     for (int e = 0; e < nband; ++e)
                         if ((bv[e * 32] < lower || ((amem >> e) & 1u)) && bval[e * 32] >= tie)
                             best = fmax(best, dist3r(x64, T, q0, q1, q2, band_frame(e)));
-                    for (int pos = first; pos >= 0; --pos)
-                    {
-                        const float sv = row.s(pos);
-                        if (sv < tie)
-                            break;
-                        if (++steps > kScanCap)
+                    int n = g0 * 4;
+                    for (int pass = 0; pass < 2; ++pass)
+                        for (int g = g0; g < g1; ++g)
                         {
-                            reason = kReasonScan;
-                            break;
+                            const float4 s4  = row.s4(g);
+                            unsigned     amb = 0u;
+#pragma unroll
+                            for (int q = 0; q < 4; ++q)
+                            {
+                                const float s = f4get(s4, q);
+                                n += pass && s < tie;
+                                amb |= (unsigned)(s >= tie && s <= chi && (pass || s < inlo)) << q;
+                            }
+                            for (; amb; amb &= amb - 1)
+                            {
+                                const int j = row.j(g * 4 + __ffs(amb) - 1);
+                                if (!pass && !(dist3f(xc, Xc[j]) < inlo)) // no member
+                                    continue;
+                                const double d = dist3r(x64, T, q0, q1, q2, j);
+                                if (pass)
+                                    n += d <= best;
+                                else
+                                    best = fmax(best, d);
+                            }
                         }
-                        const int j = row.j(pos);
-                        if (dist3f(xc, Xc[j]) < inlo)
-                            best = fmax(best, dist3r(x64, T, q0, q1, q2, j));
-                    }
-                    if (reason)
-                        break;
-                    // count: every entry below the FP64 band, plus the band in FP64
-                    const float   tlo   = __double2float_rd(__dsub_rd(best, (double)eps));
-                    const float   thi   = __double2float_ru(__dadd_ru(best, (double)eps));
-                    const LaneRow rr[4] = {row, row, row, row};
-                    int           lo[4] = {0, 0, 0, 0}, hi[4] = {Llen, Llen, 0, 0};
-                    const float   tt[4] = {tlo, thi, 0.0f, 0.0f};
-                    const bool    st[4] = {true, false, true, true};
-                    row_bounds4(rr, lo, hi, tt, st);
-                    int n = lo[0];
-                    for (int pos = lo[0]; pos < lo[1]; ++pos)
-                        n += dist3r(x64, T, q0, q1, q2, row.j(pos)) <= best;
                     ncount[side] = n;
                 }
                 if (!reason)
@@ -1093,17 +1132,13 @@ cudaError_t launch_ksg_rows(const WalkBatch& b, long long rows, cudaStream_t s)
         return cudaSuccess;
     int          threads = 256, regs = 0;
     const size_t smem    = row_sort_smem(b.maxT - 1, &threads, &regs);
-    void (*kernel)(WalkBatch) = ksg_rows_kernel<256, 0>;
+    void (*kernel)(WalkBatch) = ksg_rows_kernel<1024, 0>;
     if (threads == 256 && regs == 8)
         kernel = ksg_rows_kernel<256, 8>;
     else if (threads == 512 && regs == 8)
         kernel = ksg_rows_kernel<512, 8>;
     else if (threads == 512 && regs == 16)
         kernel = ksg_rows_kernel<512, 16>;
-#if GC_ROWS_128
-    else if (threads == 128 && regs == 16)
-        kernel = ksg_rows_kernel<128, 16>;
-#endif
     // static shared memory comes on top of the dynamic part: always raise
     // the limit to what this launch needs
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(1024, 1) ksg_row_walk_kernel(WalkBatch B)
                     // above it unless the input is not finite
                     const int reason = (r.wrapped || r.lev == 0) ? kReasonBand
                                        : (r.lev >= kWalkBuckets - 1 ? kReasonRange : 0);
-                    p.wres[(size_t)pl * p.Q + iq] = pack_walk(r.lev - 1, r.below, T - 1, reason);
+                    p.wres[(size_t)pl * p.Q + iq] = pack_walk(r.lev - 1, r.below, r.walked, reason);
                 }
                 if (p.walk_elems)
                 {

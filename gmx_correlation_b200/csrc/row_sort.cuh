@@ -2,73 +2,87 @@
 // transfer-entropy fast paths (ksg_fast.cu, te_walk.cu).
 #pragma once
 
+#include <type_traits>
+
 #include "gc_common.cuh"
 
 namespace gc {
 
-// One CTA per sorted row: a query frame's distances to every other frame,
-// sorted ascending with their frames.  Keys are
-// (distance bits << 32 | frame).  A bucket pass over the row's own
-// distribution (range, coarse CDF, histogram, scan, scatter) leaves about one
-// key per bucket, which one thread per bucket insertion-sorts.  R > 0: each
-// thread keeps its R distances (entries tid + r * threads) in registers for
-// the passes; R = 0: distances are recomputed (from L1-resident coordinate
-// rows) in every pass.  THREADS (256 or 512) threads per row; 512
-// only for rows longer than 2048 entries, so every thread owns whole
-// buckets of the scan.  A row with a crowded bucket (more than 64
-// equal-ish distances, e.g. duplicated frames), and rows longer than 8192,
-// are sorted by a bitonic network instead.
+// One CTA per row: a query frame's distances to every other frame, sorted
+// with their frames by a counting sort over fine buckets of 2^kRowFine float
+// ulps (at most a quarter of the walks' buckets).  kRowBins buckets end at the
+// largest possible distance (8 octaves); entries below them are put in full
+// order, or, if they are many, the whole row is, by a bitonic network.
+// R > 0: each thread keeps its R distances (entries tid + r * threads) in
+// registers; R = 0: they are recomputed (from L1-resident coordinate rows)
+// for the second pass.
+//
+// Entries are in bucket order, those of one fine bucket (a few) in any order.
+// That is all the walks need (their own buckets are whole fine ones); the
+// finish and count kernels look at a value's whole fine bucket.
+//
+// Bound by shared-memory atomics and issue slots.  The full sort it replaces
+// (range, coarse distribution, histogram, scan, scatter and one thread's
+// insertion sort per bucket, over eight barriers) took 10.7 ms for the rows of
+// 247 atoms x 2000 frames, 51.8 ms for 151 x 4999 and 289 us for 64 x 500;
+// this one 6.7 ms, 29.9 ms and 209 us.  Fine buckets of 2^15 ulps make it 2%
+// faster there and the finish 3% slower, 2^13 the rows 8% slower; putting the
+// entries of each bucket in order as well gives all of the gain back.
 
-// Bucket counters and cursors carry one padding word per 32, so the
-// contiguous bucket slices a thread scans start in distinct banks.
-__device__ __forceinline__ int rows_skew(int b) { return b + (b >> 5); }
-__host__ __device__ constexpr int rows_skewed(int nbin) { return nbin + (nbin >> 5); }
+constexpr int kRowBins  = 4096;
+constexpr int kRowFine  = 14; // log2 of a fine bucket's width in float ulps
+constexpr int kRowLow   = 32; // entries below the buckets that one thread sorts
 
-// Sorts the row of query frame i over frames 0 .. N (i excluded, N entries
-// in all): dist(j) gives the FP32 distance from the query to frame j.  The
-// sorted distances and frames go to S / P at base + (m / 4) * gstride + m % 4
-// for entry m (the transposed layout of the walk), the last 4-entry group
-// padded with NaN and frame 0.  Every thread of the CTA calls it; it uses
-// the dynamic shared memory (N2 * 8 + rows_skewed(nbin) * 8 bytes, N2 and
-// nbin as in row_sort_smem).  U_row (optional) receives the unsorted
-// distances at U_row[j].
+// Two 16-bit counters per word (a row has at most 16,384 entries).  Place of
+// counter word w: the 16-byte vectors are permuted so that eight threads
+// scanning neighbouring slices of 4, 8 or 16 words by vectors hit eight
+// different bank groups.
+__device__ __forceinline__ int rows_word(int w) { return w ^ ((w >> 3) & 0x1C); }
+
 // Static shared memory of sort_row: the caller's kernel declares one (so a
 // kernel that sorts rows of several kinds holds it once).
 template <int THREADS>
 struct RowSortShared
 {
-    unsigned red_min[THREADS / 32], red_max[THREADS / 32];
-    unsigned coarse[THREADS / 32][64];
-    float    cum[65];
-    int      crowded;
+    unsigned wsum[THREADS / 32];
+    int      full; // order the row by the bitonic network
 };
 
+// Sorts the row of query frame i over frames 0 .. N (i excluded, N entries
+// in all): dist(j) gives the FP32 distance from the query to frame j, at most
+// top.  The distances and frames go to S / P at base + (m / 4) * gstride +
+// m % 4 for entry m (the transposed layout of the walk), the last 4-entry
+// group padded with NaN and frame 0.  Every thread of the CTA calls it; it
+// uses the dynamic shared memory of row_sort_smem.  U_row (optional) receives
+// the unsorted distances at U_row[j].
 template <int THREADS, int R, class DistFn>
-__device__ __forceinline__ void sort_row(RowSortShared<THREADS>& sh, int N, int i, DistFn&& dist,
+__device__ __forceinline__ void sort_row(RowSortShared<THREADS>& sh, int N, int i, float top, DistFn&& dist,
                                          float* __restrict__ S, uint16_t* __restrict__ P, size_t base,
                                          size_t gstride, float* __restrict__ U_row = nullptr)
 {
     extern __shared__ __align__(16) unsigned char rows_smem[];
-    unsigned(&red_min)[THREADS / 32]       = sh.red_min;
-    unsigned(&red_max)[THREADS / 32]       = sh.red_max;
-    unsigned(&coarse)[THREADS / 32][64]    = sh.coarse;
-    float(&cum)[65]                        = sh.cum;
-    int&     crowded                       = sh.crowded;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int Np     = (N + 3) & ~3;                               // whole 4-entry groups
+    unsigned* cursor = reinterpret_cast<unsigned*>(rows_smem);     // [kRowBins / 2]
+    unsigned* vals   = cursor + kRowBins / 2;                        // [Np] distance bits in bucket order
+    uint16_t* frm    = reinterpret_cast<uint16_t*>(vals + Np);     // [Np] their frames
+    auto      frame_of = [i](int m) { return m < i ? m : m + 1; };
+    const int cb       = (int)(__float_as_uint(top) >> kRowFine) - (kRowBins - 1);
+    auto bin_of = [&](float d) -> int { return min(max((int)(__float_as_uint(d) >> kRowFine) - cb, 0), kRowBins - 1); };
 
-    const int         tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    int               N2  = THREADS; // at least one bucket per thread in the scan
-    while (N2 < N)
-        N2 <<= 1;
-    // bucket pass up to 8192 keys; longer rows use the bitonic network alone
-    const int           nbin   = N2 <= 8192 ? (N2 < 4096 ? N2 : 4096) : 0;
-    unsigned long long* keys   = reinterpret_cast<unsigned long long*>(rows_smem); // [N2] sorted output
-    unsigned*           hist   = reinterpret_cast<unsigned*>(keys + N2);           // [skewed nbin]
-    unsigned*           cursor = hist + rows_skewed(nbin);                         // [skewed nbin]
-    auto                frame_of = [i](int m) { return m < i ? m : m + 1; };
-
-    // the row's distances (and later their buckets), entry m = tid + k * threads
-    float dreg[R > 0 ? R : 1];
-    int   breg[R > 0 ? R : 1];
+    if (tid == 0)
+        sh.full = 0;
+    // counter b: adds 1 and returns its value before / reads it
+    auto bump = [cursor](int b) -> unsigned {
+        const int sh = (b & 1) * 16;
+        return (atomicAdd(&cursor[rows_word(b >> 1)], 1u << sh) >> sh) & 0xFFFFu;
+    };
+    auto start_of = [cursor](int b) -> unsigned { return (cursor[rows_word(b >> 1)] >> ((b & 1) * 16)) & 0xFFFFu; };
+    for (int b = tid * 4; b < kRowBins / 2; b += THREADS * 4)
+        *reinterpret_cast<uint4*>(cursor + b) = make_uint4(0u, 0u, 0u, 0u);
+    // the row's distances, and later each key's bucket and its arrival there
+    float    dreg[R > 0 ? R : 1];
+    unsigned breg[R > 0 ? R : 1];
     if constexpr (R > 0)
     {
 #pragma unroll
@@ -95,107 +109,44 @@ __device__ __forceinline__ void sort_row(RowSortShared<THREADS>& sh, int N, int 
                 fn(0, m, dist(frame_of(m)));
         }
     };
-
     // optional unsorted copy of the row, indexed by frame (the query's own
     // frame is left unwritten: no walk reads it)
     if (U_row)
         each([&](int, int m, float d) { U_row[frame_of(m)] = d; });
-    unsigned kmin = 0xFFFFFFFFu, kmax = 0u;
-    each([&](int, int, float d) {
-        const unsigned k = __float_as_uint(d);
-        kmin             = min(kmin, k);
-        kmax             = max(kmax, k);
+    __syncthreads();
+    each([&](int k, int, float d) {
+        const int      b = bin_of(d);
+        const unsigned o = bump(b);
+        if constexpr (R > 0)
+            breg[k] = (unsigned)b | (o << 16);
     });
-    for (int b = tid; b < rows_skewed(nbin); b += THREADS)
-        hist[b] = 0u;
-    for (int e = lane; e < 64; e += 32)
-        coarse[warp][e] = 0u;
-    if (tid == 0)
-        crowded = nbin == 0; // no bucket pass for very long rows
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-    {
-        kmin = min(kmin, __shfl_xor_sync(kFull, kmin, o));
-        kmax = max(kmax, __shfl_xor_sync(kFull, kmax, o));
-    }
-    if (lane == 0)
-    {
-        red_min[warp] = kmin;
-        red_max[warp] = kmax;
-    }
     __syncthreads();
-    kmin = red_min[0];
-    kmax = red_max[0];
-    for (int w = 1; w < THREADS / 32; ++w)
+    // exclusive scan in place: each thread a contiguous slice
+    unsigned low = 0; // thread 0: entries below the buckets
+    constexpr int kSlice = kRowBins / 2 / THREADS; // words
+    constexpr int kVec   = kSlice < 4 ? kSlice : 4;
+    using Vec            = typename std::conditional<kVec == 4, uint4, uint2>::type;
+    static_assert(kVec >= 2 && kSlice % kVec == 0, "slices by vectors");
+    union Words
     {
-        kmin = min(kmin, red_min[w]);
-        kmax = max(kmax, red_max[w]);
-    }
-    // Buckets follow the row's own distribution: a coarse 64-bin histogram
-    // (linear in the value) gives a piecewise-linear CDF, and a key's bucket
-    // is floor(CDF * nbin), so each bucket holds about one key and the
-    // per-bucket insertion sorts stay short and balanced.  Every step is
-    // monotone in the value (FP32 products and sums of non-negative terms,
-    // the fraction clamped to [0, 1]), so buckets keep key order.
-    const float vmin = __uint_as_float(kmin), vmax = __uint_as_float(kmax);
-    const float cinv = vmax > vmin ? 64.0f / (vmax - vmin) : 0.0f;
-    auto coarse_of = [&](float v, float& frac) -> unsigned {
-        const float    t = (v - vmin) * cinv;
-        const unsigned c = min((unsigned)t, 63u);
-        frac             = fminf(t - (float)c, 1.0f);
-        return c;
+        Vec      v;
+        unsigned w[kVec];
     };
-    if (nbin)
-        each([&](int, int, float d) {
-            float f;
-            atomicAdd(&coarse[warp][coarse_of(d, f)], 1u);
-        });
-    __syncthreads();
-    if (warp == 0)
-    {
-        // exclusive prefix over the 64 coarse bins (two per lane), as floats
-        unsigned c0 = 0u, c1 = 0u;
-        for (int w = 0; w < THREADS / 32; ++w)
-        {
-            c0 += coarse[w][2 * lane];
-            c1 += coarse[w][2 * lane + 1];
-        }
-        unsigned incl = c0 + c1;
+    auto slice = [cursor, tid](int v) { return reinterpret_cast<Vec*>(cursor + rows_word(tid * kSlice + v)); };
+    unsigned loc = 0;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1)
+    for (int v = 0; v < kSlice; v += kVec)
+    {
+        Words c;
+        c.v = *slice(v);
+        if (v == 0 && tid == 0)
+            low = c.w[0] & 0xFFFFu;
+#pragma unroll
+        for (int e = 0; e < kVec; ++e)
         {
-            const unsigned y = __shfl_up_sync(kFull, incl, o);
-            if (lane >= o)
-                incl += y;
+            loc += (c.w[e] & 0xFFFFu) + (c.w[e] >> 16);
         }
-        const unsigned excl = incl - c0 - c1;
-        cum[2 * lane]       = (float)excl;
-        cum[2 * lane + 1]   = (float)(excl + c0);
-        if (lane == 31)
-            cum[64] = (float)incl;
     }
-    __syncthreads();
-    const float fscale = (float)nbin / fmaxf((float)N, 1.0f);
-    auto bin_of = [&](float v) -> int {
-        float          f;
-        const unsigned c = coarse_of(v, f);
-        const unsigned b = (unsigned)((cum[c] + f * (cum[c + 1] - cum[c])) * fscale);
-        return rows_skew(b < (unsigned)nbin ? (int)b : nbin - 1);
-    };
-    // histogram
-    if (nbin)
-        each([&](int slot, int, float d) {
-            const int b = bin_of(d);
-            if constexpr (R > 0)
-                breg[slot] = b;
-            atomicAdd(&hist[b], 1u);
-        });
-    __syncthreads();
-    // exclusive scan of hist into cursor (each thread a contiguous slice)
-    const int per = nbin / THREADS; // 0 without a bucket pass
-    unsigned  loc = 0;
-    for (int e = 0; e < per; ++e)
-        loc += hist[rows_skew(tid * per + e)];
     unsigned incl = loc;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1)
@@ -205,64 +156,72 @@ __device__ __forceinline__ void sort_row(RowSortShared<THREADS>& sh, int N, int 
             incl += y;
     }
     if (lane == 31)
-        red_min[warp] = incl;
+        sh.wsum[warp] = incl;
+    if (low > (unsigned)kRowLow)
+        sh.full = 1;
     __syncthreads();
-    unsigned wbase = 0;
+    unsigned run = incl - loc;
     for (int w = 0; w < warp; ++w)
-        wbase += red_min[w];
-    unsigned run = wbase + incl - loc;
-    for (int e = 0; e < per; ++e)
+        run += sh.wsum[w];
+#pragma unroll
+    for (int v = 0; v < kSlice; v += kVec)
     {
-        const int      b = rows_skew(tid * per + e);
-        const unsigned c = hist[b];
-        cursor[b]        = run;
-        if (c > 64)
-            crowded = 1;
-        run += c;
+        Words c;
+        c.v = *slice(v);
+#pragma unroll
+        for (int e = 0; e < kVec; ++e)
+        {
+            const unsigned n = c.w[e], mid = run + (n & 0xFFFFu);
+            c.w[e]           = run | (mid << 16);
+            run              = mid + (n >> 16);
+        }
+        *slice(v) = c.v;
     }
     __syncthreads();
-    // scatter (or place in frame order for the bitonic network)
-    const bool bucketed = !crowded;
-    each([&](int slot, int m, float d) {
-        const int                j   = frame_of(m);
-        const unsigned long long key = ((unsigned long long)__float_as_uint(d) << 32) | (unsigned)j;
-        int                      b   = 0;
-        if (bucketed)
-        {
-            if constexpr (R > 0)
-                b = breg[slot];
-            else
-                b = bin_of(d);
-        }
-        const unsigned pos = bucketed ? atomicAdd(&cursor[b], 1u) : (unsigned)m;
-        keys[pos]          = key;
-    });
-    __syncthreads();
-    if (bucketed)
+    const bool full = sh.full;
+    if (!full)
     {
-        // cursor[b] now holds the end of bucket b; sort each bucket (thread
-        // t takes buckets t, t + threads, ..., so a warp's buckets, and
-        // their keys, lie side by side)
-        for (int b = tid; b < nbin; b += THREADS)
+        each([&](int k, int m, float d) {
+            unsigned at;
+            if constexpr (R > 0)
+                at = start_of((int)(breg[k] & 0xFFFFu)) + (breg[k] >> 16);
+            else
+                at = bump(bin_of(d));
+            vals[at] = __float_as_uint(d);
+            frm[at]  = (uint16_t)frame_of(m);
+        });
+        if (tid < Np - N)
         {
-            const int      bs  = rows_skew(b);
-            const unsigned end = cursor[bs], beg = end - hist[bs];
-            for (unsigned x = beg + 1; x < end; ++x)
-            {
-                const unsigned long long v = keys[x];
-                unsigned                 y = x;
-                while (y > beg && keys[y - 1] > v)
-                {
-                    keys[y] = keys[y - 1];
-                    --y;
-                }
-                keys[y] = v;
-            }
+            vals[N + tid] = 0x7fc00000u;
+            frm[N + tid]  = 0;
         }
+        __syncthreads();
+        if (tid == 0 && low > 1u) // the entries below the buckets, by insertion
+            for (unsigned x = 1; x < low; ++x)
+            {
+                const unsigned v = vals[x];
+                const uint16_t f = frm[x];
+                unsigned       y = x;
+                for (; y > 0 && vals[y - 1] > v; --y)
+                {
+                    vals[y] = vals[y - 1];
+                    frm[y]  = frm[y - 1];
+                }
+                vals[y] = v;
+                frm[y]  = f;
+            }
         __syncthreads();
     }
     else
     {
+        // bitonic network on (distance, frame), over the same shared memory
+        unsigned long long* keys = reinterpret_cast<unsigned long long*>(rows_smem); // [N2]
+        int                 N2   = THREADS;
+        while (N2 < N)
+            N2 <<= 1;
+        each([&](int, int m, float d) {
+            keys[m] = ((unsigned long long)__float_as_uint(d) << 32) | (unsigned)frame_of(m);
+        });
         for (int m = N + tid; m < N2; m += THREADS)
             keys[m] = ~0ull;
         __syncthreads();
@@ -283,45 +242,61 @@ __device__ __forceinline__ void sort_row(RowSortShared<THREADS>& sh, int N, int 
                 __syncthreads();
             }
     }
-    // transposed layout: groups of 4 consecutive entries per query, the
-    // queries of a block side by side (see WalkParams)
-    for (int m = tid; m < N; m += THREADS)
+    // transposed layout: one thread per group of 4 consecutive entries, the
+    // queries of a block side by side (see WalkParams).  The last group runs
+    // out in NaN (never <= any stop value) with frame 0, so the walk reads
+    // whole groups without a bounds test.
+    const unsigned long long* keys = reinterpret_cast<const unsigned long long*>(rows_smem);
+    for (int g = tid; g * 4 < N; g += THREADS)
     {
-        const unsigned long long k   = keys[m];
-        const size_t             idx = base + (size_t)(m >> 2) * gstride + (m & 3);
-        S[idx]                       = __uint_as_float((unsigned)(k >> 32));
-        P[idx]                       = (uint16_t)(k & 0xFFFFu);
-    }
-    // the last 4-entry group runs out in NaN (never <= any stop value) with
-    // frame 0, so the walk reads whole groups without a bounds test
-    if (tid < ((N + 3) & ~3) - N)
-    {
-        const int    m   = N + tid;
-        const size_t idx = base + (size_t)(m >> 2) * gstride + (m & 3);
-        S[idx]           = __int_as_float(0x7fc00000);
-        P[idx]           = 0;
+        uint4 v;
+        uint2 f;
+        if (!full)
+        {
+            v = *reinterpret_cast<const uint4*>(vals + g * 4);
+            f = *reinterpret_cast<const uint2*>(frm + g * 4);
+        }
+        else
+        {
+            unsigned b[4], j[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+            {
+                const bool in = g * 4 + q < N;
+                b[q]          = in ? (unsigned)(keys[g * 4 + q] >> 32) : 0x7fc00000u;
+                j[q]          = in ? (unsigned)keys[g * 4 + q] & 0xFFFFu : 0u;
+            }
+            v = make_uint4(b[0], b[1], b[2], b[3]);
+            f = make_uint2(j[0] | (j[1] << 16), j[2] | (j[3] << 16));
+        }
+        *reinterpret_cast<uint4*>(S + base + (size_t)g * gstride) = v;
+        *reinterpret_cast<uint2*>(P + base + (size_t)g * gstride) = f;
     }
 }
 
-// Shared memory of one sorted row of N entries: keys (N2 * 8 bytes) plus the
-// bucket counters and cursors; *threads and *regs pick the sort_row
-// instantiation (threads per row, distances per thread kept in registers).
-#ifndef GC_ROWS_128
-#define GC_ROWS_128 0 // a build-time setting: 128 threads x 16 distances for rows up to 2048 entries
-#endif
+// The first value of a's fine bucket, and of the next one (a >= 0).
+__device__ __forceinline__ float fine_start(float a) { return __uint_as_float(__float_as_uint(a) >> kRowFine << kRowFine); }
+__device__ __forceinline__ float fine_after(float a)
+{
+    return __uint_as_float(((__float_as_uint(a) >> kRowFine) + 1u) << kRowFine);
+}
 
+// Upper bound of an atom's distances from its FP32 error bound: 2 R, eps >= R 2^-21.
+__device__ __forceinline__ float row_top(float eps_atom) { return eps_atom * 4194304.0f * 1.0001f; }
+
+// Shared memory of one row of N entries; *threads and *regs pick the sort_row
+// instantiation (threads per row, distances per thread kept in registers):
+// 8 per thread up to 2048 entries, then 512 threads with 8 or 16 each; longer
+// rows recompute them.
 inline size_t row_sort_smem(int N, int* threads, int* regs)
 {
-    int N2 = 256;
-    while (N2 < N)
+    *threads = N <= 8 * 256 ? 256 : (N <= 16 * 512 ? 512 : 1024);
+    *regs    = N <= 8 * 512 ? 8 : (N <= 16 * 512 ? 16 : 0);
+    size_t N2 = (size_t)*threads; // the bitonic network's keys
+    while (N2 < (size_t)N)
         N2 <<= 1;
-    const int nbin = N2 <= 8192 ? (N2 < 4096 ? N2 : 4096) : 0;
-    // distances kept in registers, 8 per thread up to 2048 entries, then
-    // 512 threads with 8 or 16 each (measured faster than 256 threads with
-    // 16 or 32 at 4999 entries); longer rows recompute them
-    *threads = N <= 8 * 256 ? (GC_ROWS_128 ? 128 : 256) : (N <= 16 * 512 ? 512 : 256);
-    *regs    = N <= 8 * 256 ? (GC_ROWS_128 ? 16 : 8) : (N <= 8 * 512 ? 8 : (N <= 16 * 512 ? 16 : 0));
-    return (size_t)N2 * 8 + (size_t)rows_skewed(nbin) * 8;
+    const size_t need = (size_t)kRowBins * 2 + (((size_t)N + 3) & ~(size_t)3) * 6;
+    return need > N2 * 8 ? need : N2 * 8;
 }
 
 } // namespace gc

@@ -97,6 +97,7 @@ __device__ __forceinline__ void te_count_query(const TeParams& p, const TeTask& 
         const float  tlo_s = __double2float_rd(__dsub_rd(eps, es));
         const float  tlo_o = __double2float_rd(__dsub_rd(eps, eo));
         const float  thi_o = __double2float_ru(__dadd_ru(eps, eo));
+        const float  thi_s = __double2float_ru(__dadd_ru(eps, es));
         const TeRow  er = te_row(p.SM, p.PM, p, on1 ? tk.a1 : tk.a2, iq);
         const float4* ox = on1 ? x2 : x1;
         const float4  oq = ox[qi];
@@ -128,7 +129,7 @@ __device__ __forceinline__ void te_count_query(const TeParams& p, const TeTask& 
                 const float ov = te3(oq, ox[jv[q]]);
                 if (in && sv[q] < tlo_s && ov < tlo_o)
                     ++n;
-                else if (in && ov <= thi_o)
+                else if (in && sv[q] <= thi_s && ov <= thi_o)
                     amb |= 1u << q;
             }
             for (; amb; amb &= amb - 1) // rare: FP64 on the raw coordinates

@@ -24,6 +24,7 @@
 #include "gc_common.cuh"
 #include "gc_internal.h"
 #include "ksg_fast.h"
+#include "row_sort.cuh"
 #include "row_walk.cuh"
 #include "te_device.cuh"
 #include "te_walk.h"
@@ -268,7 +269,8 @@ __global__ void __launch_bounds__(1024, 1) te_row_count_kernel(TeBatch B)
             continue;
         // every pair on the row of its atom later in the order; codes from the
         // block's smallest k-th distance on (eps is at least that)
-        const int base = (int)(ord[c0].y >> kTeCountShift) - 1;
+        // (rows are in fine-bucket order, so from that distance's fine bucket on)
+        const int base = (int)(ord[c0].y >> kRowFine << (kRowFine - kTeCountShift)) - 1;
         if (threadIdx.x == 0)
             s_next = c0 + 1;
         for (int c = warp; c < 32 && c0 + c < n; c += nwarps)
@@ -300,8 +302,10 @@ __global__ void __launch_bounds__(1024, 1) te_row_count_kernel(TeBatch B)
             const float4* Sg  = reinterpret_cast<const float4*>(row.S);
             const uint2*  Pg  = reinterpret_cast<const uint2*>(row.P);
             const size_t  gs  = row.gstride >> 2;
-            // the row is done when its codes pass every lane's last bucket
-            const int last = (int)__reduce_max_sync(kFull, (unsigned)max(max(k1.hi, k2.hi), 0));
+            // the row is done when its codes pass the fine bucket of every
+            // lane's last one
+            const int top  = (int)__reduce_max_sync(kFull, (unsigned)max(max(k1.hi, k2.hi), 0));
+            const int last = ((top + base) | ((1 << (kRowFine - kTeCountShift)) - 1)) - base;
             const int ngr  = (Llen + 3) >> 2;
             int       n1 = 0, n2 = 0, nl = 0;
             float4    s4 = make_float4(nan, nan, nan, nan);

@@ -8,7 +8,8 @@
 // it takes part in.
 //
 //   te_rows_kernel    per (atom, query): the G row and the M row (3-D
-//                     distances over frames j < N_valid), sorted, with frames.
+//                     distances over frames j < N_valid), in the order of
+//                     narrow buckets, with frames (row_sort.cuh).
 //   te_walk_kernel    one ordered pair per CTA task, one query per lane: walk
 //                     the row (target G or source M) whose k-th value is
 //                     larger, gathering the other distance from the pair's
@@ -17,8 +18,8 @@
 //                     provably passed (the KSG walk's scheme, ksg_fast.cu).
 //   te_finish_kernel  band around the k-th bucket from two row ranges, the
 //                     FP32 k-th value, the FP64 eps from the few values
-//                     within the error bound of it; then n_xfxp and n_xp by
-//                     binary search in the target's G and M rows and n_ypxp
+//                     within the error bound of it; then n_xfxp and n_xp from
+//                     eps's place in the target's G and M rows and n_ypxp
 //                     by enumerating the shorter of the target's and the
 //                     source's M-row prefixes, every decision within the
 //                     error bound of eps re-evaluated in FP64.
@@ -54,11 +55,10 @@ __device__ __forceinline__ void te_pair(const TeParams& p, long k, long& q, int&
 }
 
 // Independent binary searches advanced together: lo[q] becomes the first
-// position in [lo[q], hi[q]) of row r[q] whose value is not < t[q]
-// (strict[q]) / not <= t[q].
+// position in [lo[q], hi[q]] of row r[q] whose value is not < t[q].  Rows are
+// in fine-bucket order, so every t[q] is the first value of a fine bucket.
 template <int NS>
-__device__ __forceinline__ void te_bounds(const TeRow (&r)[NS], int (&lo)[NS], int (&hi)[NS], const float (&t)[NS],
-                                          const bool (&strict)[NS])
+__device__ __forceinline__ void te_bounds(const TeRow (&r)[NS], int (&lo)[NS], int (&hi)[NS], const float (&t)[NS])
 {
     for (;;)
     {
@@ -75,7 +75,7 @@ __device__ __forceinline__ void te_bounds(const TeRow (&r)[NS], int (&lo)[NS], i
         for (int q = 0; q < NS; ++q)
             if (lo[q] < hi[q])
             {
-                if (strict[q] ? v[q] < t[q] : v[q] <= t[q])
+                if (v[q] < t[q])
                     lo[q] = mid[q] + 1;
                 else
                     hi[q] = mid[q];
@@ -95,7 +95,7 @@ constexpr int kTeAmbCap = 8;
 // natoms * Q the M rows, each over the frames j < N_valid, j != qi.
 // ---------------------------------------------------------------------------
 template <int THREADS, int R>
-__global__ void __launch_bounds__(THREADS) te_rows_kernel(TeBatch B)
+__global__ void __launch_bounds__(THREADS, THREADS == 256 ? 6 : (THREADS == 512 ? 2 : 1)) te_rows_kernel(TeBatch B)
 {
     const long long r   = blockIdx.x;
     const int       dsc = te_desc_of(B.rprefix, B.n, r);
@@ -111,16 +111,17 @@ __global__ void __launch_bounds__(THREADS) te_rows_kernel(TeBatch B)
     const float4*   xr  = p.X32 + (size_t)a * p.T;
     const float4    qp  = xr[qi];
     const size_t    base = ((size_t)a * (p.Lpad >> 2) * p.Qp + iq) * 4, gs = (size_t)p.Qp * 4;
+    const float     top = row_top(p.eps_atom[a]);
     __shared__ RowSortShared<THREADS> sh;
     if (g)
     {
         const float4 qf = xr[qi + lag];
         sort_row<THREADS, R>(
-            sh, p.Nv - 1, qi, [&](int j) { return fmaxf(te3(qf, xr[j + lag]), te3(qp, xr[j])); }, p.SG, p.PG, base,
+            sh, p.Nv - 1, qi, top, [&](int j) { return fmaxf(te3(qf, xr[j + lag]), te3(qp, xr[j])); }, p.SG, p.PG, base,
             gs);
     }
     else
-        sort_row<THREADS, R>(sh, p.Nv - 1, qi, [&](int j) { return te3(qp, xr[j]); }, p.SM, p.PM, base, gs);
+        sort_row<THREADS, R>(sh, p.Nv - 1, qi, top, [&](int j) { return te3(qp, xr[j]); }, p.SM, p.PM, base, gs);
 }
 
 // ---------------------------------------------------------------------------
@@ -492,14 +493,13 @@ __global__ void __launch_bounds__(kTeFinishWarps * 32, 1) te_finish_kernel(TeBat
                 const float ehi    = __uint_as_float(Lb + ((unsigned)(bstar + 1) << shift));
                 const float inlo   = __fsub_rd(elo, e2);
                 const float bandhi = __fadd_ru(ehi, e2);
-                if (m_end < Llen && rw.s(m_end) <= bandhi)
-                    reason = kTeReasonPrefix;
-                const TeRow rr[4] = {rw, rw, ro, ro};
-                int         lo[4] = {0, 0, 0, 0}, hi[4] = {m_end, m_end, Llen, Llen};
-                const float tt[4] = {inlo, bandhi, inlo, bandhi};
-                const bool  st[4] = {true, false, true, false};
-                te_bounds<4>(rr, lo, hi, tt, st);
-                const int mw0 = lo[0], mw1 = lo[1], mo0 = lo[2], mo1 = lo[3];
+                // the rows are in the order of their fine buckets: from the one of
+                // inlo to the one of bandhi
+                const TeRow rr[2] = {rw, ro};
+                int         lo[2] = {0, 0}, hi[2] = {Llen, Llen};
+                const float from = fine_start(fmaxf(inlo, 0.0f)), tt[2] = {from, from};
+                te_bounds<2>(rr, lo, hi, tt);
+                const int mw0 = lo[0], mo0 = lo[1];
                 int       nband = 0, nlo = 0;
                 auto add = [&](float v, int j) {
                     if (nband < kTeBandCap)
@@ -510,42 +510,48 @@ __global__ void __launch_bounds__(kTeFinishWarps * 32, 1) te_finish_kernel(TeBat
                     ++nband;
                     nlo += v < elo;
                 };
-                for (int g0 = mw0 >> 2; g0 * 4 < mw1; ++g0) // walked value in the band, other <= bandhi
+                int mw1 = min(mw0, Llen - 1) >> 2; // walked value in the band, other <= bandhi
+                for (bool more = true; more;)
                 {
-                    const float4 s4 = rw.s4(g0);
-                    const uint2  j4 = rw.j4(g0);
+                    const float4 s4 = rw.s4(mw1);
+                    const uint2  j4 = rw.j4(mw1);
 #pragma unroll
                     for (int q = 0; q < 4; ++q)
                     {
-                        const int mm = g0 * 4 + q;
-                        if (mm >= mw0 && mm < mw1)
+                        const float sv = f4at(s4, q); // NaN behind the row: not in the band
+                        if (sv >= inlo && sv <= bandhi)
                         {
                             const int   j  = (int)u2at16(j4, q);
-                            const float sv = f4at(s4, q);
                             const float ov = wg ? yval(j) : gval(j);
                             if (ov <= bandhi)
                                 add(fmaxf(sv, ov), j);
                         }
                     }
+                    ++mw1;
+                    more = mw1 * 4 < Llen && fine_start(s4.w) <= bandhi;
                 }
-                for (int g0 = mo0 >> 2; g0 * 4 < mo1; ++g0) // other value in the band, walked < inlo
+                int mo1 = min(mo0, Llen - 1) >> 2; // other value in the band, walked < inlo
+                for (bool more = true; more;)
                 {
-                    const float4 d4 = ro.s4(g0);
-                    const uint2  j4 = ro.j4(g0);
+                    const float4 d4 = ro.s4(mo1);
+                    const uint2  j4 = ro.j4(mo1);
 #pragma unroll
                     for (int q = 0; q < 4; ++q)
                     {
-                        const int mm = g0 * 4 + q;
-                        if (mm >= mo0 && mm < mo1)
+                        const float dv = f4at(d4, q);
+                        if (dv >= inlo && dv <= bandhi)
                         {
                             const int   j  = (int)u2at16(j4, q);
-                            const float dv = f4at(d4, q);
                             const float wv = wg ? gval(j) : yval(j);
                             if (wv < inlo)
                                 add(dv, j);
                         }
                     }
+                    ++mo1;
+                    more = mo1 * 4 < Llen && fine_start(d4.w) <= bandhi;
                 }
+                mw1 = min(mw1 * 4, Llen);
+                mo1 = min(mo1 * 4, Llen);
                 int       n_in = prefix - nlo; // #{v < inlo}
                 const int r    = K - n_in;     // rank of the k-th value in the band
                 if (!reason && (nband > kTeBandCap || r < 1 || r > nband))
@@ -610,27 +616,56 @@ __global__ void __launch_bounds__(kTeFinishWarps * 32, 1) te_finish_kernel(TeBat
                 {
                     const float tlo1 = __double2float_rd(__dsub_rd(eps, (double)e1));
                     const float thi1 = __double2float_ru(__dadd_ru(eps, (double)e1));
-                    const float tlo2 = __double2float_rd(__dsub_rd(eps, (double)e2a));
                     const float thi2 = __double2float_ru(__dadd_ru(eps, (double)e2a));
-                    const TeRow cr[5] = {G1, G1, M1, M1, M2};
-                    int         clo[5] = {0, 0, 0, 0, 0}, chi[5] = {Llen, Llen, Llen, Llen, Llen};
-                    const float ct[5] = {tlo1, thi1, tlo1, thi1, thi2};
-                    const bool  cs[5] = {true, false, true, false, false};
-                    te_bounds<5>(cr, clo, chi, ct, cs);
-                    // n_xfxp: G row of the target; n_xp: its M row
-                    int n_xfxp = clo[0];
-                    for (int pos = clo[0]; pos < clo[1]; ++pos)
+                    const TeRow cr[3] = {G1, M1, M2};
+                    // eps's fine buckets in G1 and M2 lie in the band's entries
+                    int clo[3] = {wg ? mw0 : mo0, 0, wg ? mo0 : mw0}, chi[3] = {wg ? mw1 : mo1, Llen, wg ? mo1 : mw1};
+                    const float ct[3] = {fine_start(fmaxf(tlo1, 0.0f)), fine_start(fmaxf(tlo1, 0.0f)), fine_after(thi2)};
+                    te_bounds<3>(cr, clo, chi, ct);
+                    // Entries of G1 (n_xfxp) and M1 (n_xp) below eps: those before
+                    // the fine bucket of tlo1, and of the groups up to the fine
+                    // bucket of thi1 the ones below tlo1 and, in FP64, those up to
+                    // thi1.  Both rows' groups are loaded together; the FP64
+                    // looks come after them, so the lanes take theirs at once.
+                    int  gg = min(clo[0], Llen - 1) >> 2, gm = min(clo[1], Llen - 1) >> 2;
+                    int  n_xfxp = gg * 4, n_xp = gm * 4;
+                    bool on_g = true, on_m = true;
+                    auto look = [&](const TeRow& row, int& g, bool& on, int& n, unsigned& amb, int at) {
+                        const float4 s4 = row.s4(g);
+#pragma unroll
+                        for (int q = 0; q < 4; ++q)
+                        {
+                            const float s = f4at(s4, q); // NaN behind the row: neither
+                            n += s < tlo1;
+                            amb |= (unsigned)(s >= tlo1 && s <= thi1) << (at + q);
+                        }
+                        ++g;
+                        on = g * 4 < Llen && fine_start(s4.w) <= thi1;
+                    };
+                    do
                     {
-                        const int j = G1.j(pos);
-                        n_xfxp += fmax(q64.fut(j), q64.past(j)) < eps;
-                    }
-                    int n_xp = clo[2];
-                    for (int pos = clo[2]; pos < clo[3]; ++pos)
-                        n_xp += q64.past(M1.j(pos)) < eps;
+                        const int g0 = gg * 4, m0 = gm * 4;
+                        unsigned  ag = 0u, am = 0u;
+                        for (int at = 0; at < 32 && (on_g || on_m); at += 4)
+                        {
+                            if (on_g)
+                                look(G1, gg, on_g, n_xfxp, ag, at);
+                            if (on_m)
+                                look(M1, gm, on_m, n_xp, am, at);
+                        }
+                        for (; ag; ag &= ag - 1)
+                        {
+                            const int j = G1.j(g0 + __ffs(ag) - 1);
+                            n_xfxp += fmax(q64.fut(j), q64.past(j)) < eps;
+                        }
+                        for (; am; am &= am - 1)
+                            n_xp += q64.past(M1.j(m0 + __ffs(am) - 1)) < eps;
+                    } while (on_g || on_m);
+                    const int end1 = min(gm * 4, Llen); // M1's entries up to thi1 lie before
                     // n_ypxp is counted by te_count_kernel over the shorter of
                     // the two M-row prefixes that can hold a value below eps:
                     // it gets eps (in wres) and the prefix (in cnt.y).
-                    const int  end1 = clo[3], end2 = clo[4];
+                    const int  end2 = clo[2];
                     const bool on1  = end1 <= end2;
                     const int  ne   = on1 ? end1 : end2;
                     p.wres[(size_t)pl * p.Q + iq] = (unsigned long long)__double_as_longlong(eps);
@@ -1010,17 +1045,13 @@ cudaError_t launch_te_rows(const TeBatch& b, long long rows, cudaStream_t s)
         return cudaSuccess;
     int          threads = 256, regs = 0;
     const size_t smem    = row_sort_smem(b.maxNv - 1, &threads, &regs);
-    void (*kernel)(TeBatch) = te_rows_kernel<256, 0>;
+    void (*kernel)(TeBatch) = te_rows_kernel<1024, 0>;
     if (threads == 256 && regs == 8)
         kernel = te_rows_kernel<256, 8>;
     else if (threads == 512 && regs == 8)
         kernel = te_rows_kernel<512, 8>;
     else if (threads == 512 && regs == 16)
         kernel = te_rows_kernel<512, 16>;
-#if GC_ROWS_128
-    else if (threads == 128 && regs == 16)
-        kernel = te_rows_kernel<128, 16>;
-#endif
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess)
         return e;

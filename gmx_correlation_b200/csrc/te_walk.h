@@ -9,7 +9,7 @@
 // alone and Y on the source alone, so each (atom, query) has two sorted
 // rows shared by every pair it takes part in: its G row (the 6-D embedding
 // distances) and its M row (the 3-D distances Da(qi, j), j < N_valid).  The
-// counts are n_xfxp = #{G < eps}, n_xp = #{D1 < eps} (binary searches in
+// counts are n_xfxp = #{G < eps}, n_xp = #{D1 < eps} (eps's place in
 // the target's G and M rows) and n_ypxp = #{max(D1, Y) < eps}.
 #pragma once
 

@@ -67,3 +67,41 @@ def test_long_rows_equal_exact(gc, n, T, k, kind):
     np.testing.assert_array_equal(ax, bx)
     np.testing.assert_array_equal(ay, by)
     np.testing.assert_array_equal(a, b)
+
+
+def _sort_traj(kind, n, T, seed):
+    rng = np.random.default_rng(seed)
+    x = _traj("smooth", n, T, seed)
+    if kind == "few_close":  # a dozen frames nearly equal: distances below the fine buckets, few
+        x[:, 1:13] = x[:, :1] + 1e-5 * rng.standard_normal((n, 12, 3)).astype(np.float32)
+    elif kind == "many_close":  # all frames nearly equal but for three far ones
+        x = x[:, :1] + 1e-4 * (x - x[:, :1])
+        x[:, [1, T // 2, T - 1]] += 50.0
+    elif kind == "constant":  # one atom that never moves
+        x[0] = x[0, :1]
+    return x
+
+
+@pytest.mark.parametrize("n,T,k,kind", [
+    (3, 13, 12, "few_close"), (4, 256, 5, "few_close"), (25, 257, 9, "many_close"), (3, 300, 20, "constant"),
+    (3, 2049, 30, "smooth"), (3, 2050, 30, "few_close"), (24, 2051, 12, "many_close"), (3, 4097, 8, "few_close"),
+    (3, 4098, 40, "smooth"), (2, 8193, 100, "few_close"), (2, 8194, 20, "smooth"), (3, 9002, 15, "many_close"),
+    (2, 16385, 6, "smooth"),
+])
+def test_rows_equal_exact(gc, n, T, k, kind):
+    x = _sort_traj(kind, n, T, seed=n + T)
+    a, ax, ay = gc.kraskov_corrmatrix(x, k, detail=True)
+    b, bx, by = gc.kraskov_corrmatrix(x, k, path=gc.PATH_EXACT_FP64, detail=True)
+    np.testing.assert_array_equal(ax, bx)
+    np.testing.assert_array_equal(ay, by)
+    np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("n,T,k,lag,kind", [
+    (3, 14, 5, 1, "few_close"), (4, 259, 9, 2, "many_close"), (3, 300, 20, 3, "constant"), (25, 301, 7, 1, "few_close"),
+    (24, 2052, 40, 1, "many_close"), (3, 2051, 25, 1, "few_close"), (3, 4100, 30, 2, "smooth"),
+    (2, 8200, 50, 5, "few_close"), (2, 9001, 12, 1, "many_close"),
+])
+def test_te_fine_buckets_equal_exact(gc, n, T, k, lag, kind):
+    x = _sort_traj(kind, n, T, seed=n + T)
+    np.testing.assert_array_equal(gc.te_matrix(x, k, lag), gc.te_matrix(x, k, lag, path=gc.PATH_EXACT_FP64))
