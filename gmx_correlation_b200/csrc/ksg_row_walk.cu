@@ -24,6 +24,7 @@
 namespace gc {
 
 constexpr int kOrderThreads = 256;
+constexpr int kRwAhead      = 8; // frames of a tile column a lane loads together
 
 // One CTA per (descriptor, query of its block): rank of every atom by its
 // k-th marginal distance (ties by atom), and the code of that distance.
@@ -99,13 +100,21 @@ __global__ void __launch_bounds__(1024, 1) ksg_row_walk_kernel(WalkBatch B)
             }
             if (threadIdx.x == 0)
                 s_next = pa0;
-            for (int c = warp; c < 32 && b0 + c < n; c += nwarps)
-            {
+            rw_fill(min(32, n - b0), T, kRwAhead, warp, nwarps, [&](int c, int j0) {
                 const float4* xr = p.X32 + (size_t)ord[b0 + c].x * T;
                 const float4  q  = xr[i];
-                for (int j = lane; j < T; j += 32)
-                    tile[rw_row((unsigned)j) ^ (unsigned)c] = rw_code(dist3f(q, xr[j]), shift, base);
-            }
+                float4        v[kRwAhead];
+#pragma unroll
+                for (int e = 0; e < kRwAhead; ++e)
+                    v[e] = xr[min(j0 + e * 32 + lane, T - 1)];
+#pragma unroll
+                for (int e = 0; e < kRwAhead; ++e)
+                {
+                    const int j = j0 + e * 32 + lane;
+                    if (j < T)
+                        tile[rw_row((unsigned)j) ^ (unsigned)c] = rw_code(dist3f(q, v[e]), shift, base);
+                }
+            });
             __syncthreads();
             for (;;)
             {

@@ -108,6 +108,7 @@ __device__ __forceinline__ void te_tile(const TeParams& p, const uint2* ord, int
 // The count's 16-bit codes: 2^13 float ulps wide (a tenth of a percent: one
 // or two frames of a pair share eps's bucket), relative to the base.
 constexpr int kTeCountShift = 13;
+constexpr int kTeAhead      = 8; // frames of a tile column a lane loads together
 __device__ __forceinline__ int te_code16(float d, int base)
 {
     return min(max((int)(__float_as_uint(d) >> kTeCountShift) - base, 0), 65535);
@@ -273,14 +274,22 @@ __global__ void __launch_bounds__(1024, 1) te_row_count_kernel(TeBatch B)
         const int base = (int)(ord[c0].y >> kRowFine << (kRowFine - kTeCountShift)) - 1;
         if (threadIdx.x == 0)
             s_next = c0 + 1;
-        for (int c = warp; c < 32 && c0 + c < n; c += nwarps)
-        {
+        rw_fill(min(32, n - c0), Nv, kTeAhead, warp, nwarps, [&](int c, int j0) {
             const float4* x = p.X32 + (size_t)ord[c0 + c].x * T;
             const float4  q = x[qi];
-            for (int j = lane; j < Nv; j += 32)
-                *reinterpret_cast<uint16_t*>(tile + (te_row16((unsigned)j) ^ (unsigned)(2 * c))) =
-                    (uint16_t)te_code16(te3(q, x[j]), base);
-        }
+            float         d[kTeAhead];
+#pragma unroll
+            for (int e = 0; e < kTeAhead; ++e)
+                d[e] = te3(q, x[min(j0 + e * 32 + lane, Nv - 1)]);
+#pragma unroll
+            for (int e = 0; e < kTeAhead; ++e)
+            {
+                const int j = j0 + e * 32 + lane;
+                if (j < Nv)
+                    *reinterpret_cast<uint16_t*>(tile + (te_row16((unsigned)j) ^ (unsigned)(2 * c))) =
+                        (uint16_t)te_code16(d[e], base);
+            }
+        });
         __syncthreads();
         const unsigned lane2 = (unsigned)lane * 2u;
         for (;;)
