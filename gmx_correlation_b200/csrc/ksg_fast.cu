@@ -83,7 +83,7 @@ __global__ void ksg_x32_kernel(const double* __restrict__ X64, int natoms, int T
 // marginal distances (self excluded) in bucket order with their frames
 // (sort_row).
 template <int THREADS, int R>
-__global__ void __launch_bounds__(THREADS, THREADS == 256 ? 6 : (THREADS == 512 ? 2 : 1)) ksg_rows_kernel(WalkBatch B)
+__global__ void __launch_bounds__(THREADS, row_ctas(THREADS, R)) ksg_rows_kernel(WalkBatch B)
 {
     // row blockIdx.x of the launch -> descriptor, atom, query of its block
     const long long   r   = blockIdx.x;
@@ -1133,14 +1133,14 @@ cudaError_t launch_ksg_rows(const WalkBatch& b, long long rows, cudaStream_t s)
     int          threads = 256, regs = 0;
     const size_t smem    = row_sort_smem(b.maxT - 1, &threads, &regs);
     void (*kernel)(WalkBatch) = ksg_rows_kernel<1024, 0>;
-    if (threads == 256 && regs == 8)
-        kernel = ksg_rows_kernel<256, 8>;
-    else if (threads == 512 && regs == 8)
-        kernel = ksg_rows_kernel<512, 8>;
-    else if (threads == 512 && regs == 16)
+    if (threads == 64)
+        kernel = ksg_rows_kernel<64, 8>;
+    else if (threads == 128)
+        kernel = regs == 8 ? ksg_rows_kernel<128, 8> : ksg_rows_kernel<128, 16>;
+    else if (threads == 256)
+        kernel = ksg_rows_kernel<256, 16>;
+    else if (threads == 512)
         kernel = ksg_rows_kernel<512, 16>;
-    // static shared memory comes on top of the dynamic part: always raise
-    // the limit to what this launch needs
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess)
         return e;

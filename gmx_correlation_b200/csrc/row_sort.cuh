@@ -25,17 +25,23 @@ namespace gc {
 // (range, coarse distribution, histogram, scan, scatter and one thread's
 // insertion sort per bucket, over eight barriers) took 10.7 ms for the rows of
 // 247 atoms x 2000 frames, 51.8 ms for 151 x 4999 and 289 us for 64 x 500;
-// this one 6.7 ms, 29.9 ms and 209 us.  Fine buckets of 2^15 ulps make it 2%
-// faster there and the finish 3% slower, 2^13 the rows 8% slower; putting the
-// entries of each bucket in order as well gives all of the gain back.
+// this one 6.55 ms, 28.2 ms and 134 us.  Fine buckets of 2^15 ulps make it 2%
+// faster and the finish 3% slower, 2^13 the rows 8% slower; putting the
+// entries of each bucket in order as well costs as much as the full sort.
 
 constexpr int kRowBins  = 4096;
 constexpr int kRowFine  = 14; // log2 of a fine bucket's width in float ulps
 constexpr int kRowLow   = 32; // entries below the buckets that one thread sorts
 
+// CTAs an SM should hold (the register limit of the row kernels).
+constexpr int row_ctas(int threads, int regs)
+{
+    return threads == 1024 ? 1 : (regs == 8 || threads == 512 ? 1536 : 1280) / threads;
+}
+
 // Two 16-bit counters per word (a row has at most 16,384 entries).  Place of
 // counter word w: the 16-byte vectors are permuted so that eight threads
-// scanning neighbouring slices of 4, 8 or 16 words by vectors hit eight
+// scanning neighbouring slices of up to 32 words by vectors hit eight
 // different bank groups.
 __device__ __forceinline__ int rows_word(int w) { return w ^ ((w >> 3) & 0x1C); }
 
@@ -80,9 +86,9 @@ __device__ __forceinline__ void sort_row(RowSortShared<THREADS>& sh, int N, int 
     auto start_of = [cursor](int b) -> unsigned { return (cursor[rows_word(b >> 1)] >> ((b & 1) * 16)) & 0xFFFFu; };
     for (int b = tid * 4; b < kRowBins / 2; b += THREADS * 4)
         *reinterpret_cast<uint4*>(cursor + b) = make_uint4(0u, 0u, 0u, 0u);
-    // the row's distances, and later each key's bucket and its arrival there
+    // the row's distances, and later each key's arrival in its bucket
     float    dreg[R > 0 ? R : 1];
-    unsigned breg[R > 0 ? R : 1];
+    unsigned areg[R > 0 ? (R + 1) / 2 : 1]; // two 16-bit numbers each
     if constexpr (R > 0)
     {
 #pragma unroll
@@ -115,10 +121,14 @@ __device__ __forceinline__ void sort_row(RowSortShared<THREADS>& sh, int N, int 
         each([&](int, int m, float d) { U_row[frame_of(m)] = d; });
     __syncthreads();
     each([&](int k, int, float d) {
-        const int      b = bin_of(d);
-        const unsigned o = bump(b);
+        const unsigned o = bump(bin_of(d));
         if constexpr (R > 0)
-            breg[k] = (unsigned)b | (o << 16);
+        {
+            if (k & 1)
+                areg[k >> 1] |= o << 16;
+            else
+                areg[k >> 1] = o;
+        }
     });
     __syncthreads();
     // exclusive scan in place: each thread a contiguous slice
@@ -184,7 +194,7 @@ __device__ __forceinline__ void sort_row(RowSortShared<THREADS>& sh, int N, int 
         each([&](int k, int m, float d) {
             unsigned at;
             if constexpr (R > 0)
-                at = start_of((int)(breg[k] & 0xFFFFu)) + (breg[k] >> 16);
+                at = start_of(bin_of(d)) + ((areg[k >> 1] >> ((k & 1) * 16)) & 0xFFFFu);
             else
                 at = bump(bin_of(d));
             vals[at] = __float_as_uint(d);
@@ -285,13 +295,16 @@ __device__ __forceinline__ float fine_after(float a)
 __device__ __forceinline__ float row_top(float eps_atom) { return eps_atom * 4194304.0f * 1.0001f; }
 
 // Shared memory of one row of N entries; *threads and *regs pick the sort_row
-// instantiation (threads per row, distances per thread kept in registers):
-// 8 per thread up to 2048 entries, then 512 threads with 8 or 16 each; longer
-// rows recompute them.
+// instantiation (threads per row, distances per thread kept in registers).
+// The passes are short, so what counts is how little a barrier holds up:
+// few threads a row, many rows an SM.  64 x 500: 209 us by 256 threads, 169
+// by 256 with 4 distances, 142 by 128, 134 by 64; 247 x 2000: 6.78 ms by 256,
+// 6.55 by 128; 150 x 3000: 11.2 ms by 512, 9.7 by 256; 151 x 4999: 29.8 ms by
+// 512 (two rows an SM), 28.2 (three), 30.3 by 256 with 32 distances.
 inline size_t row_sort_smem(int N, int* threads, int* regs)
 {
-    *threads = N <= 8 * 256 ? 256 : (N <= 16 * 512 ? 512 : 1024);
-    *regs    = N <= 8 * 512 ? 8 : (N <= 16 * 512 ? 16 : 0);
+    *threads = N <= 8 * 64 ? 64 : (N <= 16 * 128 ? 128 : (N <= 16 * 256 ? 256 : (N <= 16 * 512 ? 512 : 1024)));
+    *regs    = N <= 8 * 128 ? 8 : (N <= 16 * 512 ? 16 : 0);
     size_t N2 = (size_t)*threads; // the bitonic network's keys
     while (N2 < (size_t)N)
         N2 <<= 1;

@@ -95,7 +95,7 @@ constexpr int kTeAmbCap = 8;
 // natoms * Q the M rows, each over the frames j < N_valid, j != qi.
 // ---------------------------------------------------------------------------
 template <int THREADS, int R>
-__global__ void __launch_bounds__(THREADS, THREADS == 256 ? 6 : (THREADS == 512 ? 2 : 1)) te_rows_kernel(TeBatch B)
+__global__ void __launch_bounds__(THREADS, row_ctas(THREADS, R)) te_rows_kernel(TeBatch B)
 {
     const long long r   = blockIdx.x;
     const int       dsc = te_desc_of(B.rprefix, B.n, r);
@@ -1046,11 +1046,13 @@ cudaError_t launch_te_rows(const TeBatch& b, long long rows, cudaStream_t s)
     int          threads = 256, regs = 0;
     const size_t smem    = row_sort_smem(b.maxNv - 1, &threads, &regs);
     void (*kernel)(TeBatch) = te_rows_kernel<1024, 0>;
-    if (threads == 256 && regs == 8)
-        kernel = te_rows_kernel<256, 8>;
-    else if (threads == 512 && regs == 8)
-        kernel = te_rows_kernel<512, 8>;
-    else if (threads == 512 && regs == 16)
+    if (threads == 64)
+        kernel = te_rows_kernel<64, 8>;
+    else if (threads == 128)
+        kernel = regs == 8 ? te_rows_kernel<128, 8> : te_rows_kernel<128, 16>;
+    else if (threads == 256)
+        kernel = te_rows_kernel<256, 16>;
+    else if (threads == 512)
         kernel = te_rows_kernel<512, 16>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess)

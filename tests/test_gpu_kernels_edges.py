@@ -84,6 +84,7 @@ def _sort_traj(kind, n, T, seed):
 
 @pytest.mark.parametrize("n,T,k,kind", [
     (3, 13, 12, "few_close"), (4, 256, 5, "few_close"), (25, 257, 9, "many_close"), (3, 300, 20, "constant"),
+    (3, 513, 20, "smooth"), (24, 514, 11, "few_close"), (3, 1025, 40, "smooth"), (3, 1026, 25, "few_close"),
     (3, 2049, 30, "smooth"), (3, 2050, 30, "few_close"), (24, 2051, 12, "many_close"), (3, 4097, 8, "few_close"),
     (3, 4098, 40, "smooth"), (2, 8193, 100, "few_close"), (2, 8194, 20, "smooth"), (3, 9002, 15, "many_close"),
     (2, 16385, 6, "smooth"),
@@ -99,6 +100,7 @@ def test_rows_equal_exact(gc, n, T, k, kind):
 
 @pytest.mark.parametrize("n,T,k,lag,kind", [
     (3, 14, 5, 1, "few_close"), (4, 259, 9, 2, "many_close"), (3, 300, 20, 3, "constant"), (25, 301, 7, 1, "few_close"),
+    (3, 514, 20, 1, "smooth"), (24, 516, 11, 2, "few_close"), (3, 1026, 30, 1, "smooth"), (3, 1030, 30, 4, "smooth"),
     (24, 2052, 40, 1, "many_close"), (3, 2051, 25, 1, "few_close"), (3, 4100, 30, 2, "smooth"),
     (2, 8200, 50, 5, "few_close"), (2, 9001, 12, 1, "many_close"),
 ])
