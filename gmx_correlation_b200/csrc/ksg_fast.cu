@@ -619,13 +619,12 @@ __global__ void __launch_bounds__(kFinishWarps * 32, 1) ksg_finish_kernel(WalkBa
     const int      warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     unsigned char* base = smem_raw + (size_t)warp * kBandSlotBytes * kBandCap * 32;
     // per-lane columns: band entry e of lane l at [e * 32 + l]: joint value v,
-    // walked-marginal value s, other-marginal value d and the row position as
-    // an offset from the start of its range (the walked-row range holds the
-    // first entries, the other-row range the rest)
+    // the smaller marginal value m and the row position as an offset from the
+    // start of its range (the walked-row range holds the first entries, the
+    // other-row range the rest), bit 15 set where v is the walked marginal
     float*    bv = reinterpret_cast<float*>(base) + lane;
-    float*    bs = bv + kBandCap * 32;
-    float*    bd = bs + kBandCap * 32;
-    uint16_t* bo = reinterpret_cast<uint16_t*>(bd + kBandCap * 32 - lane) + lane;
+    float*    bm = bv + kBandCap * 32;
+    uint16_t* bo = reinterpret_cast<uint16_t*>(bm + kBandCap * 32 - lane) + lane;
 
     const long long total = B.fprefix[B.n];
     for (;;)
@@ -707,13 +706,13 @@ __global__ void __launch_bounds__(kFinishWarps * 32, 1) ksg_finish_kernel(WalkBa
                     }
                     int nlo = 0;
                     nband   = 0;
-                    auto add = [&](float v, float sv, float dv, int off) {
+                    auto add = [&](float sv, float dv, int off) {
+                        const float v = fmaxf(sv, dv);
                         if (nband < kBandCap)
                         {
                             bv[nband * 32] = v;
-                            bs[nband * 32] = sv;
-                            bd[nband * 32] = dv;
-                            bo[nband * 32] = (uint16_t)off;
+                            bm[nband * 32] = fminf(sv, dv);
+                            bo[nband * 32] = (uint16_t)(off | (sv >= dv ? 0x8000 : 0));
                         }
                         ++nband;
                         nlo += v < elo;
@@ -741,7 +740,7 @@ __global__ void __launch_bounds__(kFinishWarps * 32, 1) ksg_finish_kernel(WalkBa
                                 const int   j  = (int)u2get16(j4, q);
                                 const float dv = dist3f(xo, X32o[in ? j : 0]);
                                 if (in && dv <= bandhi)
-                                    add(fmaxf(sv, dv), sv, dv, g * 4 + q - mw0);
+                                    add(sv, dv, g * 4 + q - mw0);
                             }
                             ++g;
                             s4 = ns;
@@ -769,7 +768,7 @@ __global__ void __launch_bounds__(kFinishWarps * 32, 1) ksg_finish_kernel(WalkBa
                                 const int   j  = (int)u2get16(j4, q);
                                 const float sv = dist3f(xw, X32w[in ? j : 0]);
                                 if (in && sv < inlo)
-                                    add(dv, sv, dv, g * 4 + q - mo0);
+                                    add(sv, dv, g * 4 + q - mo0);
                             }
                             ++g;
                             d4 = nd;
@@ -811,7 +810,8 @@ __global__ void __launch_bounds__(kFinishWarps * 32, 1) ksg_finish_kernel(WalkBa
                 }
                 // frame of band entry e (for the FP64 paths)
                 auto band_frame = [&](int e) -> int {
-                    return e < nW ? rw.j(mw0 + bo[e * 32]) : ro.j(mo0 + bo[e * 32]);
+                    const int off = bo[e * 32] & 0x7FFF;
+                    return e < nW ? rw.j(mw0 + off) : ro.j(mo0 + off);
                 };
 
                 // ---- certain members and the ambiguous set ------------------------
@@ -889,7 +889,10 @@ __global__ void __launch_bounds__(kFinishWarps * 32, 1) ksg_finish_kernel(WalkBa
                     const double*  x64  = side == 0 ? xw64 : xo64;
                     const float    eps  = side == 0 ? ew : eo;
                     const float    eps2 = __fmul_ru(2.0f, eps);
-                    const float*   bval = side == 0 ? bs : bd;
+                    // an entry's value of this side
+                    auto bval = [&](int e) -> float {
+                        return ((bo[e * 32] & 0x8000) != 0) == (side == 0) ? bv[e * 32] : bm[e * 32];
+                    };
                     // band members
                     float top  = -1.0f;
                     int   ptop = -1;
@@ -897,9 +900,9 @@ __global__ void __launch_bounds__(kFinishWarps * 32, 1) ksg_finish_kernel(WalkBa
                     {
                         if (!(bv[e * 32] < lower || ((amem >> e) & 1u)))
                             continue;
-                        const float val = bval[e * 32];
+                        const float val = bval(e);
                         // row position of the entry in this side's row (-1: other row)
-                        const int prow = (side == 0) == (e < nW) ? (side == 0 ? mw0 : mo0) + bo[e * 32] : -1;
+                        const int prow = (side == 0) == (e < nW) ? (side == 0 ? mw0 : mo0) + (bo[e * 32] & 0x7FFF) : -1;
                         if (val > top)
                         {
                             top  = val;
@@ -1006,7 +1009,7 @@ __global__ void __launch_bounds__(kFinishWarps * 32, 1) ksg_finish_kernel(WalkBa
                     const double q0 = x64[i], q1 = x64[T + i], q2 = x64[2 * T + i];
                     double       best = -1.0;
                     for (int e = 0; e < nband; ++e)
-                        if ((bv[e * 32] < lower || ((amem >> e) & 1u)) && bval[e * 32] >= tie)
+                        if ((bv[e * 32] < lower || ((amem >> e) & 1u)) && bval(e) >= tie)
                             best = fmax(best, dist3r(x64, T, q0, q1, q2, band_frame(e)));
                     int n = g0 * 4;
                     for (int pass = 0; pass < 2; ++pass)

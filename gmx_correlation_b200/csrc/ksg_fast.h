@@ -8,9 +8,14 @@ namespace gc {
 
 constexpr int kWalkWarps   = 32;       // most warps per walk CTA
 #ifndef GC_FINISH_WARPS
-#define GC_FINISH_WARPS 20 // a build-time setting for timing other finish CTA shapes
+#define GC_FINISH_WARPS 25 // a build-time setting for timing other finish CTA shapes
 #endif
-constexpr int kFinishWarps = GC_FINISH_WARPS; // warps per finish CTA
+// Warps per finish CTA.  The finish gathers coordinates through L1, which has
+// what the band entries leave of an SM's 256 KB.  20 warps with 14-byte
+// entries leave about 60 KB: 30.6 ms at 247 x 2000 k=100 and 44.1 at 151 x
+// 4999 (24 such warps leave 28 KB: 43.8 and 68.7 ms); with 10-byte entries 20
+// warps take 29.4 and 41.2 ms, 24 28.1 and 39.4, 25 (72 registers) 27.4 and 38.7.
+constexpr int kFinishWarps = GC_FINISH_WARPS;
 constexpr int kWalkBuckets = 128;      // per-lane histogram buckets
 #ifndef GC_BAND_CAP
 #define GC_BAND_CAP 20 // a build-time setting for timing other capacities
@@ -23,7 +28,7 @@ constexpr int kRwMaxAtoms   = 4096; // row walk: atoms the per-query ordering ta
 // Row walk: bytes of the code tile of T frames.
 __host__ __device__ inline size_t rw_tile_bytes(int T) { return ((size_t)T * 32 + 127) & ~(size_t)127; }
 constexpr int kBandCap     = GC_BAND_CAP; // band entries kept per lane
-constexpr int kBandSlotBytes = 14;     // v, s, d (f32), row position in its range (u16)
+constexpr int kBandSlotBytes = 10;     // joint and smaller marginal value (f32), row position in its range (u16)
 constexpr uint32_t kHandOver = 0xFFFFFFFFu; // cnt value of a query handed to the exact kernel
 
 // Sorted marginal rows of one query block, transposed so that the 32
