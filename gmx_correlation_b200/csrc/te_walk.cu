@@ -476,8 +476,6 @@ __global__ void __launch_bounds__(kTeFinishWarps * 32, 1) te_finish_kernel(TeBat
             const TeRow   M2 = te_row(p.SM, p.PM, p, a2, iq);
             const float   gk = G1.s(K - 1), yk = M2.s(K - 1);
             const bool    wg = gk >= yk;
-            const TeRow&  rw = wg ? G1 : M2;
-            const TeRow&  ro = wg ? M2 : G1;
             const unsigned Lb = __float_as_uint(wg ? gk : yk) >> shift << shift;
             const float4* x1 = p.X32 + (size_t)a1 * T;
             const float4* x2 = p.X32 + (size_t)a2 * T;
@@ -495,11 +493,11 @@ __global__ void __launch_bounds__(kTeFinishWarps * 32, 1) te_finish_kernel(TeBat
                 const float bandhi = __fadd_ru(ehi, e2);
                 // the rows are in the order of their fine buckets: from the one of
                 // inlo to the one of bandhi
-                const TeRow rr[2] = {rw, ro};
+                const TeRow rr[2] = {G1, M2};
                 int         lo[2] = {0, 0}, hi[2] = {Llen, Llen};
                 const float from = fine_start(fmaxf(inlo, 0.0f)), tt[2] = {from, from};
                 te_bounds<2>(rr, lo, hi, tt);
-                const int mw0 = lo[0], mo0 = lo[1];
+                const int g0 = lo[0], y0 = lo[1];
                 int       nband = 0, nlo = 0;
                 auto add = [&](float v, int j) {
                     if (nband < kTeBandCap)
@@ -510,48 +508,51 @@ __global__ void __launch_bounds__(kTeFinishWarps * 32, 1) te_finish_kernel(TeBat
                     ++nband;
                     nlo += v < elo;
                 };
-                int mw1 = min(mw0, Llen - 1) >> 2; // walked value in the band, other <= bandhi
+                // The walked row's values in the band with the other value up to
+                // bandhi, and the other row's with the walked value below inlo.  Row
+                // by row and not walked row first, so that all lanes gather alike.
+                int g1 = min(g0, Llen - 1) >> 2;
                 for (bool more = true; more;)
                 {
-                    const float4 s4 = rw.s4(mw1);
-                    const uint2  j4 = rw.j4(mw1);
+                    const float4 s4 = G1.s4(g1);
+                    const uint2  j4 = G1.j4(g1);
 #pragma unroll
                     for (int q = 0; q < 4; ++q)
                     {
-                        const float sv = f4at(s4, q); // NaN behind the row: not in the band
-                        if (sv >= inlo && sv <= bandhi)
+                        const float gv = f4at(s4, q); // NaN behind the row: not in the band
+                        if (gv >= inlo && gv <= bandhi)
                         {
                             const int   j  = (int)u2at16(j4, q);
-                            const float ov = wg ? yval(j) : gval(j);
-                            if (ov <= bandhi)
-                                add(fmaxf(sv, ov), j);
+                            const float yv = yval(j);
+                            if (wg ? yv <= bandhi : yv < inlo)
+                                add(fmaxf(gv, yv), j);
                         }
                     }
-                    ++mw1;
-                    more = mw1 * 4 < Llen && fine_start(s4.w) <= bandhi;
+                    ++g1;
+                    more = g1 * 4 < Llen && fine_start(s4.w) <= bandhi;
                 }
-                int mo1 = min(mo0, Llen - 1) >> 2; // other value in the band, walked < inlo
+                int y1 = min(y0, Llen - 1) >> 2;
                 for (bool more = true; more;)
                 {
-                    const float4 d4 = ro.s4(mo1);
-                    const uint2  j4 = ro.j4(mo1);
+                    const float4 s4 = M2.s4(y1);
+                    const uint2  j4 = M2.j4(y1);
 #pragma unroll
                     for (int q = 0; q < 4; ++q)
                     {
-                        const float dv = f4at(d4, q);
-                        if (dv >= inlo && dv <= bandhi)
+                        const float yv = f4at(s4, q);
+                        if (yv >= inlo && yv <= bandhi)
                         {
                             const int   j  = (int)u2at16(j4, q);
-                            const float wv = wg ? gval(j) : yval(j);
-                            if (wv < inlo)
-                                add(dv, j);
+                            const float gv = gval(j);
+                            if (wg ? gv < inlo : gv <= bandhi)
+                                add(fmaxf(gv, yv), j);
                         }
                     }
-                    ++mo1;
-                    more = mo1 * 4 < Llen && fine_start(d4.w) <= bandhi;
+                    ++y1;
+                    more = y1 * 4 < Llen && fine_start(s4.w) <= bandhi;
                 }
-                mw1 = min(mw1 * 4, Llen);
-                mo1 = min(mo1 * 4, Llen);
+                g1 = min(g1 * 4, Llen);
+                y1 = min(y1 * 4, Llen);
                 int       n_in = prefix - nlo; // #{v < inlo}
                 const int r    = K - n_in;     // rank of the k-th value in the band
                 if (!reason && (nband > kTeBandCap || r < 1 || r > nband))
@@ -619,7 +620,7 @@ __global__ void __launch_bounds__(kTeFinishWarps * 32, 1) te_finish_kernel(TeBat
                     const float thi2 = __double2float_ru(__dadd_ru(eps, (double)e2a));
                     const TeRow cr[3] = {G1, M1, M2};
                     // eps's fine buckets in G1 and M2 lie in the band's entries
-                    int clo[3] = {wg ? mw0 : mo0, 0, wg ? mo0 : mw0}, chi[3] = {wg ? mw1 : mo1, Llen, wg ? mo1 : mw1};
+                    int clo[3] = {g0, 0, y0}, chi[3] = {g1, Llen, y1};
                     const float ct[3] = {fine_start(fmaxf(tlo1, 0.0f)), fine_start(fmaxf(tlo1, 0.0f)), fine_after(thi2)};
                     te_bounds<3>(cr, clo, chi, ct);
                     // Entries of G1 (n_xfxp) and M1 (n_xp) below eps: those before
@@ -644,7 +645,7 @@ __global__ void __launch_bounds__(kTeFinishWarps * 32, 1) te_finish_kernel(TeBat
                     };
                     do
                     {
-                        const int g0 = gg * 4, m0 = gm * 4;
+                        const int gb = gg * 4, mb = gm * 4;
                         unsigned  ag = 0u, am = 0u;
                         for (int at = 0; at < 32 && (on_g || on_m); at += 4)
                         {
@@ -655,11 +656,11 @@ __global__ void __launch_bounds__(kTeFinishWarps * 32, 1) te_finish_kernel(TeBat
                         }
                         for (; ag; ag &= ag - 1)
                         {
-                            const int j = G1.j(g0 + __ffs(ag) - 1);
+                            const int j = G1.j(gb + __ffs(ag) - 1);
                             n_xfxp += fmax(q64.fut(j), q64.past(j)) < eps;
                         }
                         for (; am; am &= am - 1)
-                            n_xp += q64.past(M1.j(m0 + __ffs(am) - 1)) < eps;
+                            n_xp += q64.past(M1.j(mb + __ffs(am) - 1)) < eps;
                     } while (on_g || on_m);
                     const int end1 = min(gm * 4, Llen); // M1's entries up to thi1 lie before
                     // n_ypxp is counted by te_count_kernel over the shorter of
