@@ -10,7 +10,7 @@ namespace gc {
 
 // One CTA per row: a query frame's distances to every other frame, sorted
 // with their frames by a counting sort over fine buckets of 2^kRowFine float
-// ulps (at most a quarter of the walks' buckets).  kRowBins buckets end at the
+// ulps (an eighth of the walks' narrowest buckets).  kRowBins buckets end at the
 // largest possible distance (8 octaves); entries below them are put in full
 // order, or, if they are many, the whole row is, by a bitonic network.
 // R > 0: each thread keeps its R distances (entries tid + r * threads) in

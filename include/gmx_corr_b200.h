@@ -124,7 +124,8 @@ gc_status gc_ksg_matrix_prepared(const double* X, const double* psi, int natoms,
 /* gc_ksg_matrix keeps the device workspace of its last call on each device
  * (a few GB at 247 atoms x 2000 frames) and reuses it when the next call has
  * the same shape (atoms, frames, k, path, pair range); explicit pair lists are
- * not kept.  gc_release_cache frees every kept workspace. */
+ * not kept.  gc_te_matrix keeps its last plan in the same way.  gc_release_cache
+ * frees every kept workspace and the device blocks kept for later calls. */
 void gc_release_cache(void);
 
 /* KSG MI matrices of ntraj trajectories in one batched run: trajectory i
@@ -381,8 +382,8 @@ gc_status gc_ksg_screened(const gc_traj_view* traj, int k, gc_screen_model* mode
  * No counterpart in the reference.  For callers that cannot allocate device
  * memory (a plugin whose host application owns all device memory through its
  * own pool, or a latency-critical caller that cannot take cudaMalloc /
- * cudaFree): computes the pair MI of every atom pair with the exact FP64 KSG
- * kernels, taking all scratch from one fixed array of about 9.8 MB that the
+ * cudaFree): computes the pair MI of every atom pair with the brute-force
+ * KSG kernels (FP32 search, exact FP64 repair), taking all scratch from one fixed array of about 9.8 MB that the
  * library holds on every device that loads it until the process exits.
  * Limits: natoms <= 64, nframes <= 1024; larger calls fail with
  * GC_ERR_INVALID.  d_xyz: device [natoms][nframes][3] mean-centred
