@@ -31,21 +31,22 @@ struct LaneRow
 {
     const float*    S;
     const uint16_t* P;
-    size_t          gstride; // elements between consecutive 4-entry groups
+    size_t          gstride; // elements from a run to the next
+    int             run;     // log2 of a run's 4-entry groups
 
-    __device__ __forceinline__ float  s(int m) const { return S[(size_t)(m >> 2) * gstride + (m & 3)]; }
-    __device__ __forceinline__ int    j(int m) const { return P[(size_t)(m >> 2) * gstride + (m & 3)]; }
+    __device__ __forceinline__ float  s(int m) const { return S[row_entry(m, gstride, run)]; }
+    __device__ __forceinline__ int    j(int m) const { return P[row_entry(m, gstride, run)]; }
     __device__ __forceinline__ float4 s4(int g) const
     {
-        return *reinterpret_cast<const float4*>(S + (size_t)g * gstride);
+        return *reinterpret_cast<const float4*>(S + row_entry(g * 4, gstride, run));
     }
-    __device__ __forceinline__ uint2 j4(int g) const { return *reinterpret_cast<const uint2*>(P + (size_t)g * gstride); }
+    __device__ __forceinline__ uint2 j4(int g) const { return *reinterpret_cast<const uint2*>(P + row_entry(g * 4, gstride, run)); }
 };
 
 __device__ __forceinline__ LaneRow lane_row(const WalkParams& p, int atom, int iq)
 {
-    const size_t base = ((size_t)atom * (p.Lpad >> 2) * p.Qp + iq) * 4;
-    return LaneRow{p.S + base, p.P + base, (size_t)p.Qp * 4};
+    const size_t base = ((size_t)atom * (p.Lpad >> 2) * p.Qp + ((size_t)iq << p.run)) * 4;
+    return LaneRow{p.S + base, p.P + base, ((size_t)p.Qp * 4) << p.run, p.run};
 }
 
 __device__ __forceinline__ double dist3r(const double* __restrict__ r, int T, double q0, double q1, double q2, int j)

@@ -99,7 +99,8 @@ __global__ void __launch_bounds__(THREADS, row_ctas(THREADS, R)) ksg_rows_kernel
     __shared__ RowSortShared<THREADS> sh;
     sort_row<THREADS, R>(
         sh, T - 1, i, row_top(w.eps_atom[a]), [&](int j) { return dist3f(q, xr[j]); }, w.S, w.P,
-        ((size_t)a * (Lpad >> 2) * Qp + iq) * 4, (size_t)Qp * 4, w.U ? w.U + ((size_t)a * Qp + iq) * w.Tpad : nullptr);
+        ((size_t)a * (Lpad >> 2) * Qp + ((size_t)iq << w.run)) * 4, ((size_t)Qp * 4) << w.run, w.run,
+        w.U ? w.U + ((size_t)a * Qp + iq) * w.Tpad : nullptr);
 }
 
 namespace {
@@ -280,7 +281,7 @@ __device__ __forceinline__ void walk_query_group(const WalkParams& p, long pl, i
     // of each group and a group short of 4 ends the walk.
     const float4* Sg = reinterpret_cast<const float4*>(u.rw.S); // 4-entry groups of this lane's row
     const uint2*  Pg = reinterpret_cast<const uint2*>(u.rw.P);
-    const size_t  gs = (size_t)p.Qp;                            // group stride
+    const size_t  gs = (size_t)p.Qp << p.run;                  // groups from a run to the next
     int           m_end = 0, cnt_lo = 0, R = 0, thr = 0, grp = 0;
     unsigned      wrap = 0u; // bit 8 set once a counter below the top passed 255
     float         stop = inf;
@@ -302,8 +303,8 @@ __device__ __forceinline__ void walk_query_group(const WalkParams& p, long pl, i
         }
         // prefetch the next group (the last group again at the end)
         const int      nxt   = grp < last ? grp + 1 : grp;
-        const float4   ns4   = Sg[(size_t)nxt * gs];
-        const uint2    nj4   = Pg[(size_t)nxt * gs];
+        const float4   ns4   = Sg[row_group(nxt, gs, p.run)];
+        const uint2    nj4   = Pg[row_group(nxt, gs, p.run)];
         const float    sv[4] = {s4.x, s4.y, s4.z, s4.w};
         const unsigned jv[4] = {j4.x & 0xFFFFu, j4.x >> 16, j4.y & 0xFFFFu, j4.y >> 16};
         bool           tkn[4];

@@ -31,10 +31,32 @@ constexpr int kBandCap     = GC_BAND_CAP; // band entries kept per lane
 constexpr int kBandSlotBytes = 10;     // joint and smaller marginal value (f32), row position in its range (u16)
 constexpr uint32_t kHandOver = 0xFFFFFFFFu; // cnt value of a query handed to the exact kernel
 
+// Rows are stored in runs of 2^run 4-entry groups, the runs of a block's queries
+// side by side.  Place of entry m / of group g in a row; stride: elements /
+// groups from one of its runs to the next.
+__host__ __device__ inline size_t row_entry(int m, size_t stride, int run)
+{
+    return (size_t)(m >> (2 + run)) * stride + (m & ((4 << run) - 1));
+}
+__host__ __device__ inline size_t row_group(int g, size_t stride, int run)
+{
+    return (size_t)(g >> run) * stride + (g & ((1 << run) - 1));
+}
+// The run of a launch's rows.  A walk with one query per lane reads the same
+// group of 32 queries at once: single groups.  The row sort writes a row and the
+// row walk reads it from one CTA or warp, where single groups are a cache line
+// each: 247 x 2000: 55.2 ms with single groups, 51.7 / 50.3 / 49.9 with runs of
+// 2 / 4 / 8; 151 x 4999: 111.7, 101.1 / 96.8 / 95.2; TE 247 x 2000: 150.4, 144.3
+// / 140.6 / 140.2.  Short rows end in the finish, whose lanes read neighbouring
+// queries: 64 x 500: 700 us, 664 / 651 / 661; TE 40 x 700: finish 316, 340 / 343 /
+// 363 us.  A pair list at 247 x 2000: lane walk 2.3 ms, 2.6 / 3.2 / 4.1.
+inline int row_run(bool row_walk, int maxLen) { return !row_walk ? 0 : (maxLen > 1024 ? 3 : 2); }
+
 // Sorted marginal rows of one query block, transposed so that the 32
-// queries of a warp read consecutive addresses: entry m of the row of
-// (atom a, query i0 + iq) is element ((a * Lq + m / 4) * Qp + iq) * 4 + m % 4
-// of S (distances) and of P (frames), Lq = Lpad / 4.
+// queries of a warp read neighbouring addresses: entry m of the row of
+// (atom a, query i0 + iq) is element (a * Lq * Qp + (iq << run)) * 4 +
+// row_entry(m, (Qp * 4) << run, run) of S (distances) and of P (frames),
+// Lq = Lpad / 4 (a multiple of 8).
 struct WalkParams
 {
     const float4*   X32;      // [natoms][T] centred FP32 coordinates
@@ -43,6 +65,7 @@ struct WalkParams
     float*          S;
     uint16_t*       P;
     int             natoms, Lpad, Qp, i0, Q, T, K, box, rank_shift;
+    int             run; // row_run of the launch
     long            pair_begin, pair_count;
     const int2*     pair_ab;    // optional [pair_count] (a1, a2) of an explicit pair list
     const int*      pair_order; // optional task order: task k computes local pair pair_order[k]

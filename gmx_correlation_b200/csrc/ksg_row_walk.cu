@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(1024, 1) ksg_row_walk_kernel(WalkBatch B)
                 const bool      live = pb < pa;
                 const LaneRow   row  = lane_row(p, a, iq);
                 const RwBracket r    = rw_walk(tile, reinterpret_cast<const float4*>(row.S),
-                                               reinterpret_cast<const uint2*>(row.P), (size_t)p.Qp, T - 1, p.K, shift, w0,
+                                               reinterpret_cast<const uint2*>(row.P), row.gstride >> 2, row.run, T - 1, p.K, shift, w0,
                                                w0 - 1 - base, live, hist, stage, lane);
                 if (live)
                 {

@@ -5,6 +5,7 @@
 #include <type_traits>
 
 #include "gc_common.cuh"
+#include "ksg_fast.h"
 
 namespace gc {
 
@@ -56,15 +57,16 @@ struct RowSortShared
 
 // Sorts the row of query frame i over frames 0 .. N (i excluded, N entries
 // in all): dist(j) gives the FP32 distance from the query to frame j, at most
-// top.  The distances and frames go to S / P at base + (m / 4) * gstride +
-// m % 4 for entry m (the transposed layout of the walk), the last 4-entry
+// top.  The distances and frames go to S / P at base + row_entry(m, gstride,
+// run_log) for entry m (the transposed layout of the walk), the last 4-entry
 // group padded with NaN and frame 0.  Every thread of the CTA calls it; it
 // uses the dynamic shared memory of row_sort_smem.  U_row (optional) receives
 // the unsorted distances at U_row[j].
 template <int THREADS, int R, class DistFn>
 __device__ __forceinline__ void sort_row(RowSortShared<THREADS>& sh, int N, int i, float top, DistFn&& dist,
                                          float* __restrict__ S, uint16_t* __restrict__ P, size_t base,
-                                         size_t gstride, float* __restrict__ U_row = nullptr)
+                                         size_t gstride, int run_log,
+                                         float* __restrict__ U_row = nullptr)
 {
     extern __shared__ __align__(16) unsigned char rows_smem[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -279,8 +281,8 @@ __device__ __forceinline__ void sort_row(RowSortShared<THREADS>& sh, int N, int 
             v = make_uint4(b[0], b[1], b[2], b[3]);
             f = make_uint2(j[0] | (j[1] << 16), j[2] | (j[3] << 16));
         }
-        *reinterpret_cast<uint4*>(S + base + (size_t)g * gstride) = v;
-        *reinterpret_cast<uint2*>(P + base + (size_t)g * gstride) = f;
+        *reinterpret_cast<uint4*>(S + base + row_entry(g * 4, gstride, run_log)) = v;
+        *reinterpret_cast<uint2*>(P + base + row_entry(g * 4, gstride, run_log)) = f;
     }
 }
 

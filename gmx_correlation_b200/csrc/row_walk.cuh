@@ -66,7 +66,7 @@ struct RwBracket
     bool wrapped; // a counter overflowed: the bracket is not usable
 };
 
-// The warp walks the sorted row (4-entry groups Sg / Pg with stride gs, Llen
+// The warp walks the sorted row (4-entry groups Sg / Pg in runs, see row_group, Llen
 // entries, NaN behind the last) until every live lane's k-th joint value is
 // bracketed.  w0: the code of the row's own k-th value, a lower bound of
 // every lane's k-th joint value; woff = w0 - 1 - base of the tile (0 .. 128,
@@ -80,7 +80,7 @@ struct RwBracket
 // Bound by issue slots and the histogram's read-modify-write (two
 // conflict-free wavefronts): about 13 instructions per entry and lane.
 __device__ __forceinline__ RwBracket rw_walk(const unsigned char* tile, const float4* __restrict__ Sg,
-                                             const uint2* __restrict__ Pg, size_t gs, int Llen, int K, int shift,
+                                             const uint2* __restrict__ Pg, size_t gs, int rrun, int Llen, int K, int shift,
                                              int w0, int woff, bool live, unsigned char* hist, unsigned char* stage,
                                              int lane)
 {
@@ -103,8 +103,8 @@ __device__ __forceinline__ RwBracket rw_walk(const unsigned char* tile, const fl
     uint2          j4  = make_uint2(0u, 0u);
     if (lane < ngr)
     {
-        s4 = Sg[(size_t)lane * gs];
-        j4 = Pg[(size_t)lane * gs];
+        s4 = Sg[row_group(lane, gs, rrun)];
+        j4 = Pg[row_group(lane, gs, rrun)];
     }
     RwBracket r{kTop, 0, Llen, false};
     bool      done = !live;
@@ -137,8 +137,8 @@ __device__ __forceinline__ RwBracket rw_walk(const unsigned char* tile, const fl
         s4          = make_float4(nan, nan, nan, nan);
         if (g < ngr)
         {
-            s4 = Sg[(size_t)g * gs];
-            j4 = Pg[(size_t)g * gs];
+            s4 = Sg[row_group(g, gs, rrun)];
+            j4 = Pg[row_group(g, gs, rrun)];
         }
         const int nsub = min(kRwChunk / 16, (Llen - m0 + 15) >> 4);
         for (int sub = 0; sub < nsub; ++sub)

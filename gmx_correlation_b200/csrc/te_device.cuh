@@ -2,6 +2,7 @@
 #pragma once
 
 #include "gc_common.cuh"
+#include "ksg_fast.h"
 #include "te_walk.h"
 
 namespace gc {
@@ -31,21 +32,22 @@ struct TeRow
 {
     const float*    S;
     const uint16_t* P;
-    size_t          gstride; // elements between consecutive 4-entry groups
+    size_t          gstride; // elements from a run to the next
+    int             run;     // log2 of a run's 4-entry groups
 
-    __device__ __forceinline__ float s(int m) const { return S[(size_t)(m >> 2) * gstride + (m & 3)]; }
-    __device__ __forceinline__ int   j(int m) const { return P[(size_t)(m >> 2) * gstride + (m & 3)]; }
+    __device__ __forceinline__ float s(int m) const { return S[row_entry(m, gstride, run)]; }
+    __device__ __forceinline__ int   j(int m) const { return P[row_entry(m, gstride, run)]; }
     __device__ __forceinline__ float4 s4(int g) const
     {
-        return *reinterpret_cast<const float4*>(S + (size_t)g * gstride);
+        return *reinterpret_cast<const float4*>(S + row_entry(g * 4, gstride, run));
     }
-    __device__ __forceinline__ uint2 j4(int g) const { return *reinterpret_cast<const uint2*>(P + (size_t)g * gstride); }
+    __device__ __forceinline__ uint2 j4(int g) const { return *reinterpret_cast<const uint2*>(P + row_entry(g * 4, gstride, run)); }
 };
 
 __device__ __forceinline__ TeRow te_row(const float* S, const uint16_t* P, const TeParams& p, int atom, int iq)
 {
-    const size_t base = ((size_t)atom * (p.Lpad >> 2) * p.Qp + iq) * 4;
-    return TeRow{S + base, P + base, (size_t)p.Qp * 4};
+    const size_t base = ((size_t)atom * (p.Lpad >> 2) * p.Qp + ((size_t)iq << p.run)) * 4;
+    return TeRow{S + base, P + base, ((size_t)p.Qp * 4) << p.run, p.run};
 }
 
 __device__ __forceinline__ float f4at(const float4& v, int q)
@@ -103,7 +105,7 @@ __device__ __forceinline__ void te_count_query(const TeParams& p, const TeTask& 
         const float4  oq = ox[qi];
         const float4* Sg = reinterpret_cast<const float4*>(er.S);
         const uint2*  Pg = reinterpret_cast<const uint2*>(er.P);
-        const size_t  gs = (size_t)p.Qp;
+        const size_t  gs = (size_t)p.Qp << p.run;
         const int     ng = (ne + 3) >> 2;
         int           n  = 0;
         float4        s4 = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -117,8 +119,8 @@ __device__ __forceinline__ void te_count_query(const TeParams& p, const TeTask& 
         {
             // the next group is loaded while this one is counted
             const int    nx  = g0 + 1 < ng ? g0 + 1 : g0;
-            const float4 ns4 = Sg[(size_t)nx * gs];
-            const uint2  nj4 = Pg[(size_t)nx * gs];
+            const float4 ns4 = Sg[row_group(nx, gs, p.run)];
+            const uint2  nj4 = Pg[row_group(nx, gs, p.run)];
             const float  sv[4] = {s4.x, s4.y, s4.z, s4.w};
             const unsigned jv[4] = {j4.x & 0xFFFFu, j4.x >> 16, j4.y & 0xFFFFu, j4.y >> 16};
             unsigned     amb = 0u;

@@ -177,7 +177,7 @@ __global__ void __launch_bounds__(1024, 1) te_row_walk_kernel(TeBatch B)
                     continue;
                 const TeRow row = wg ? te_row(p.SG, p.PG, p, (int)oa.x, iq) : te_row(p.SM, p.PM, p, (int)oa.x, iq);
                 const RwBracket r = rw_walk(tile, reinterpret_cast<const float4*>(row.S),
-                                            reinterpret_cast<const uint2*>(row.P), row.gstride >> 2, p.Nv - 1, p.K, shift,
+                                            reinterpret_cast<const uint2*>(row.P), row.gstride >> 2, row.run, p.Nv - 1, p.K, shift,
                                             w0, w0 - 1 - base, live, hist, stage, lane);
                 if (live)
                 {
@@ -321,8 +321,8 @@ __global__ void __launch_bounds__(1024, 1) te_row_count_kernel(TeBatch B)
             uint2     j4 = make_uint2(0u, 0u);
             if (lane < ngr)
             {
-                s4 = Sg[(size_t)lane * gs];
-                j4 = Pg[(size_t)lane * gs];
+                s4 = Sg[row_group(lane, gs, row.run)];
+                j4 = Pg[row_group(lane, gs, row.run)];
             }
             bool more = true; // warp-uniform
             for (int m0 = 0; more && m0 < Llen; m0 += kRwChunk)
@@ -336,8 +336,8 @@ __global__ void __launch_bounds__(1024, 1) te_row_count_kernel(TeBatch B)
                 s4          = make_float4(nan, nan, nan, nan);
                 if (g < ngr)
                 {
-                    s4 = Sg[(size_t)g * gs];
-                    j4 = Pg[(size_t)g * gs];
+                    s4 = Sg[row_group(g, gs, row.run)];
+                    j4 = Pg[row_group(g, gs, row.run)];
                 }
                 const int nsub = min(kRwChunk / 8, (Llen - m0 + 7) >> 3);
                 for (int sub = 0; more && sub < nsub; ++sub)

@@ -110,7 +110,8 @@ __global__ void __launch_bounds__(THREADS, row_ctas(THREADS, R)) te_rows_kernel(
     const int       lag = p.lag;
     const float4*   xr  = p.X32 + (size_t)a * p.T;
     const float4    qp  = xr[qi];
-    const size_t    base = ((size_t)a * (p.Lpad >> 2) * p.Qp + iq) * 4, gs = (size_t)p.Qp * 4;
+    const size_t    base = ((size_t)a * (p.Lpad >> 2) * p.Qp + ((size_t)iq << p.run)) * 4;
+    const size_t    gs   = ((size_t)p.Qp * 4) << p.run;
     const float     top = row_top(p.eps_atom[a]);
     __shared__ RowSortShared<THREADS> sh;
     if (g)
@@ -118,10 +119,11 @@ __global__ void __launch_bounds__(THREADS, row_ctas(THREADS, R)) te_rows_kernel(
         const float4 qf = xr[qi + lag];
         sort_row<THREADS, R>(
             sh, p.Nv - 1, qi, top, [&](int j) { return fmaxf(te3(qf, xr[j + lag]), te3(qp, xr[j])); }, p.SG, p.PG, base,
-            gs);
+            gs, p.run);
     }
     else
-        sort_row<THREADS, R>(sh, p.Nv - 1, qi, top, [&](int j) { return te3(qp, xr[j]); }, p.SM, p.PM, base, gs);
+        sort_row<THREADS, R>(sh, p.Nv - 1, qi, top, [&](int j) { return te3(qp, xr[j]); }, p.SM, p.PM, base, gs,
+                             p.run);
 }
 
 // ---------------------------------------------------------------------------
@@ -230,7 +232,7 @@ __device__ __forceinline__ void te_walk_group(const TeParams& p, const TeTask& t
     };
     const float4* Sg = reinterpret_cast<const float4*>(rw.S);
     const uint2*  Pg = reinterpret_cast<const uint2*>(rw.P);
-    const size_t  gs = (size_t)p.Qp;
+    const size_t  gs = (size_t)p.Qp << p.run;
     int           m_end = 0, cnt_lo = 0, Rs = 0, thr = 0, grp = 0;
     unsigned      wrap = 0u;
     float         stop = inf;
@@ -251,8 +253,8 @@ __device__ __forceinline__ void te_walk_group(const TeParams& p, const TeTask& t
             break;
         }
         const int      nxt   = grp < last ? grp + 1 : grp;
-        const float4   ns4   = Sg[(size_t)nxt * gs];
-        const uint2    nj4   = Pg[(size_t)nxt * gs];
+        const float4   ns4   = Sg[row_group(nxt, gs, p.run)];
+        const uint2    nj4   = Pg[row_group(nxt, gs, p.run)];
         const float    sv[4] = {s4.x, s4.y, s4.z, s4.w};
         const unsigned jv[4] = {j4.x & 0xFFFFu, j4.x >> 16, j4.y & 0xFFFFu, j4.y >> 16};
         bool           tkn[4];

@@ -27,8 +27,8 @@ constexpr int kTeBandCap = 24; // band entries kept per lane in the finish kerne
 constexpr int kTeFinishWarps = GC_TE_FINISH_WARPS;
 
 // One query block of one trajectory.  Entry m of the G row of (atom a,
-// query i0 + iq) is element ((a * Lq + m / 4) * Qp + iq) * 4 + m % 4 of
-// SG / PG (distance / frame), Lq = Lpad / 4; the M rows likewise in SM / PM.
+// query i0 + iq) is in SG / PG (distance / frame) where a KSG row of that atom
+// and query is (WalkParams); the M rows likewise in SM / PM.
 struct TeParams
 {
     const float4*   X32;      // [natoms][T] centred FP32 raw coordinates
@@ -39,6 +39,7 @@ struct TeParams
     float*          SM;
     uint16_t*       PM;
     int             natoms, T, lag, Nv, K, Lpad, Qp, i0, Q;
+    int             run; // row_run of the launch (ksg_fast.h)
     long            pair_count; // ordered pairs q = a1 * (natoms - 1) + (a2 < a1 ? a2 : a2 - 1)
     const int*      pair_order; // walk / finish task k computes ordered pair pair_order[k]
     int             shift;      // walk histogram bucket = 2^shift float ulps above the lower bound
