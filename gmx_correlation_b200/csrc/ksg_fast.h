@@ -50,7 +50,16 @@ __host__ __device__ inline size_t row_group(int g, size_t stride, int run)
 // / 140.6 / 140.2.  Short rows end in the finish, whose lanes read neighbouring
 // queries: 64 x 500: 700 us, 664 / 651 / 661; TE 40 x 700: finish 316, 340 / 343 /
 // 363 us.  A pair list at 247 x 2000: lane walk 2.3 ms, 2.6 / 3.2 / 4.1.
-inline int row_run(bool row_walk, int maxLen) { return !row_walk ? 0 : (maxLen > 1024 ? 3 : 2); }
+// With up to 24 pairs an atom (pair lists, few atoms) the rows outweigh the lane
+// walk: runs of 2.  16 atoms x 2000: 1.14 -> 1.03 ms, 8 x 5000: 2.38 -> 1.94, 23 x
+// 500 218 -> 204 us, TE 22 x 2000 4.35 -> 4.06 ms; 1,519 pairs of 247 x 2000 save
+// 1.7 ms of rows and finish for .3 ms of walk, so about 40 pairs an atom break even.
+inline int row_run(bool row_walk, int maxLen, long long pairs, int natoms)
+{
+    if (!row_walk)
+        return pairs <= 24LL * natoms ? 1 : 0;
+    return maxLen > 1024 ? 3 : 2;
+}
 
 // Sorted marginal rows of one query block, transposed so that the 32
 // queries of a warp read neighbouring addresses: entry m of the row of

@@ -204,7 +204,7 @@ gc_status KsgLaunch::build(const std::vector<std::vector<WalkParams>>& wave_desc
         for (const WalkParams& d : wv)
         {
             all.push_back(d);
-            all.back().run = row_run(row_walk, d.T - 1);
+            all.back().run = row_run(row_walk, d.T - 1, d.pair_count, d.natoms);
             qp.push_back(qp.back() + d.Q);
             up.push_back(up.back() + (long long)d.Q * ((d.natoms + 31) / 32));
             maxT                 = std::max(maxT, d.T);

@@ -213,7 +213,7 @@ gc_status TeLaunch::build(const std::vector<std::vector<TeParams>>& wave_descs, 
         for (const TeParams& d : wv)
         {
             all.push_back(d);
-            all.back().run      = gc::row_run(row_walk, d.Nv - 1);
+            all.back().run      = gc::row_run(row_walk, d.Nv - 1, d.pair_count, d.natoms);
             const long long grp = (d.Q + 31) / 32;
             rp.push_back(rp.back() + 2LL * d.natoms * d.Q);
             wp.push_back(wp.back() + (grp + chunk - 1) / chunk * d.pair_count);
