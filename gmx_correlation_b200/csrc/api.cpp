@@ -370,7 +370,7 @@ namespace {
 // One run of a plan: the normalisation of d_xyz into the plan's rows (or,
 // with d_xyz == nullptr, a finiteness check of rows the caller already
 // placed there), then the neighbour statistics and the MI reduction.
-gc_status plan_run(gc_ksg_plan* p, const double* d_xyz, double* d_pair_mi, cudaStream_t s)
+gc_status plan_enqueue(gc_ksg_plan* p, const double* d_xyz, double* d_pair_mi, cudaStream_t s)
 {
     p->launches = 0;
     GC_TRY_CUDA(cudaMemsetAsync(p->status.p, 0, sizeof(int), s));
@@ -412,6 +412,16 @@ gc_status plan_run(gc_ksg_plan* p, const double* d_xyz, double* d_pair_mi, cudaS
     GC_TRY_CUDA(cudaGetLastError());
     GC_TRY_CUDA(cudaEventRecord(p->ev_done, s));
     return GC_OK;
+}
+
+// A run that fails in the middle has not recorded ev_done, which the plan's
+// end waits for: what it did enqueue is waited for here.
+gc_status plan_run(gc_ksg_plan* p, const double* d_xyz, double* d_pair_mi, cudaStream_t s)
+{
+    const gc_status st = plan_enqueue(p, d_xyz, d_pair_mi, s);
+    if (st != GC_OK)
+        drain(s);
+    return st;
 }
 
 } // namespace
@@ -514,7 +524,10 @@ void gc_ksg_plan_destroy(gc_ksg_plan* p)
             cudaEventDestroy(p->ev_done);
         }
         if (p->stream)
+        {
+            cudaStreamSynchronize(p->stream); // an upload that no run followed
             cudaStreamDestroy(p->stream);
+        }
         if (p->ev0)
             cudaEventDestroy(p->ev0);
         if (p->ev1)

@@ -358,6 +358,7 @@ gc_status gc_te_batch(const gc_traj_view* trajs, const int* ks, int ntraj, int l
     }
     TeBatchPlan* bp = g_te[cur];
     cudaStream_t s  = bp->stream;
+    StreamDrain  drained{s};
     for (int i = 0; i < ntraj; ++i)
         GC_TRY(upload_traj(&trajs[i], bp->items[(size_t)i]->xyz.p, s));
     if (!bp->exec)
@@ -441,6 +442,7 @@ gc_status gc_gcmi_batch(const gc_traj_view* trajs, int ntraj, const gc_opts* opt
     }
     GcmiBatchPlan* bp = g_gcmi[cur];
     cudaStream_t   s  = bp->stream;
+    StreamDrain    drained{s};
     for (int i = 0; i < ntraj; ++i)
         GC_TRY(upload_traj(&trajs[i], bp->items[(size_t)i]->xyz.p, s));
     if (!bp->exec)

@@ -206,19 +206,38 @@ inline gc_status check_view(const gc_traj_view* v)
     return GC_OK;
 }
 
-// Uploads the view's coordinates into a contiguous device block.
+// Waits for what is ordered on s, so that device blocks and caller's arrays in
+// use there are free: on the way out of a call that failed in the middle.  A
+// stream under capture has nothing in flight and is left alone.
+inline void drain(cudaStream_t s)
+{
+    cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &c) == cudaSuccess && c == cudaStreamCaptureStatusNone)
+        cudaStreamSynchronize(s);
+    cudaGetLastError(); // the caller reports the first error
+}
+
+// Drains a stream at the end of a scope: declared after the pooled buffers
+// that work on it uses, so they return to the pool idle on every path.
+struct StreamDrain
+{
+    cudaStream_t s;
+    ~StreamDrain() { drain(s); }
+};
+
+// Uploads the view's coordinates into a contiguous device block.  After an
+// error no copy is in flight.
 inline gc_status upload_traj(const gc_traj_view* v, double* d_xyz, cudaStream_t s)
 {
     const size_t row = (size_t)v->nframes * 3;
+    cudaError_t  e   = cudaSuccess;
     if (v->xyz)
-    {
-        GC_TRY_CUDA(cudaMemcpyAsync(d_xyz, v->xyz, sizeof(double) * row * v->natoms, cudaMemcpyHostToDevice, s));
-    }
-    else
-    {
-        for (int a = 0; a < v->natoms; ++a)
-            GC_TRY_CUDA(cudaMemcpyAsync(d_xyz + row * a, v->rows[a], sizeof(double) * row, cudaMemcpyHostToDevice, s));
-    }
+        e = cudaMemcpyAsync(d_xyz, v->xyz, sizeof(double) * row * v->natoms, cudaMemcpyHostToDevice, s);
+    for (int a = 0; !v->xyz && e == cudaSuccess && a < v->natoms; ++a)
+        e = cudaMemcpyAsync(d_xyz + row * a, v->rows[a], sizeof(double) * row, cudaMemcpyHostToDevice, s);
+    if (e != cudaSuccess)
+        drain(s);
+    GC_TRY_CUDA(e);
     return GC_OK;
 }
 

@@ -90,6 +90,8 @@ struct BatchPlan
     std::vector<int>                        key; // natoms, T, k per trajectory
     ~BatchPlan()
     {
+        if (stream) // the members' blocks return to the pool idle
+            cudaStreamSynchronize(stream);
         if (exec)
             cudaGraphExecDestroy(exec);
         if (stream)
@@ -385,6 +387,7 @@ gc_status gc_ksg_batch(const gc_traj_view* trajs, const int* ks, int ntraj, cons
     }
     BatchPlan* bp = g_batch[cur];
     cudaStream_t s = bp->stream;
+    StreamDrain  drained{s};
     for (int i = 0; i < ntraj; ++i)
         GC_TRY(upload_traj(&trajs[i], bp->t[(size_t)i]->xyz.p, s));
     if (!bp->tuned)

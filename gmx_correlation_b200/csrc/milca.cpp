@@ -140,11 +140,7 @@ gc_status run(Call& c)
     const size_t       nq = (size_t)c.N * Kr;
     PoolBuf<double>    X, psi, phi, eps, mic, mir;
     PoolBuf<int>       cnt, maxd, order, status;
-    struct Drain
-    {
-        cudaStream_t s;
-        ~Drain() { cudaStreamSynchronize(s); }
-    } drain{st};
+    StreamDrain        drained{st};
     GC_TRY(X.alloc((size_t)D * c.N));
     for (int d = 0; d < D; ++d)
         GC_TRY_CUDA(cudaMemcpyAsync(X.p + (size_t)d * c.N, c.rows[(size_t)d], sizeof(double) * c.N,

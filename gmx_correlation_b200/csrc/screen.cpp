@@ -464,11 +464,7 @@ gc_status gc_screen_features(const gc_traj_view* traj, int k, const gc_opts* opt
     PoolBuf<double> d_xyz;
     PoolBuf<float>  d_out, d_pca;
     PoolBuf<int2>   d_ab;
-    struct Drain // the stream has drained before the buffers return to the pool
-    {
-        cudaStream_t s;
-        ~Drain() { cudaStreamSynchronize(s); }
-    } drain{ss.s};
+    StreamDrain     drained{ss.s};
     GC_TRY(d_xyz.alloc((size_t)traj->natoms * traj->nframes * 3));
     GC_TRY(d_out.alloc((size_t)std::max<long>(count, 1) * width));
     GC_TRY(upload_traj(traj, d_xyz.p, ss.s));
@@ -671,11 +667,7 @@ gc_status gc_ksg_screened(const gc_traj_view* traj, int k, gc_screen_model* m, c
 
     PoolBuf<double> d_xyz, d_mi;
     PoolBuf<float>  d_F, d_Y, d_mean, d_sd;
-    struct Drain // the stream has drained before the buffers return to the pool
-    {
-        cudaStream_t s;
-        ~Drain() { cudaStreamSynchronize(s); }
-    } drain{s};
+    StreamDrain     drained{s};
     GC_TRY(d_xyz.alloc((size_t)n * T * 3));
     GC_TRY(d_F.alloc((size_t)P * gc::kScreenIn));
     GC_TRY(d_Y.alloc((size_t)P * m->members));

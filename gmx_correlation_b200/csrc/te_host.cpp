@@ -321,6 +321,40 @@ struct gc_te_plan
     double              walk_mean = 0.0;
 };
 
+namespace {
+
+gc_status te_plan_enqueue(gc_te_plan* p, const double* d_xyz, double* d_te, cudaStream_t s)
+{
+    const int n = p->natoms;
+    GC_TRY_CUDA(cudaMemsetAsync(p->status.p, 0, sizeof(int), s));
+    GC_TRY_CUDA(cudaMemsetAsync(d_te, 0, sizeof(double) * (size_t)n * n, s));
+    GC_TRY(p->tt.prepare(d_xyz, p->status.p, s));
+    p->launches = 2;
+    GC_TRY_CUDA(cudaEventRecord(p->ev0, s));
+    if (p->walk)
+    {
+        GC_TRY(p->tl.enqueue(p->sms, s));
+        GC_TRY_CUDA(cudaEventRecord(p->ev1, s));
+        GC_TRY_CUDA(gc::launch_te_reduce(p->tt.cnt.p, n, p->Nv, p->K, p->tt.psi.p, d_te, p->sms, s));
+        p->launches += p->tl.launches + 1;
+    }
+    else
+    {
+        if (p->path == GC_PATH_EXACT_FP64)
+            gc::launch_te_exact(p->tt.XT.p, n, p->T, p->K, p->lag, p->tt.cnt.p, s, p->wide);
+        else
+            gc::launch_te_fast(p->tt.XT.p, p->tt.X32.p, p->tt.eps.p, n, p->T, p->K, p->lag, p->tt.cnt.p, s);
+        GC_TRY_CUDA(cudaEventRecord(p->ev1, s));
+        gc::launch_te_finalize(p->tt.cnt.p, n, p->T, p->K, p->lag, p->tt.psi.p, d_te, s, p->wide);
+        p->launches += 2;
+    }
+    GC_TRY_CUDA(cudaGetLastError());
+    GC_TRY_CUDA(cudaEventRecord(p->ev_done, s));
+    return GC_OK;
+}
+
+} // namespace
+
 extern "C" {
 
 gc_status gc_te_plan_create(int natoms, int nframes, int k, int lag, const gc_opts* opts, gc_te_plan** out)
@@ -384,33 +418,11 @@ gc_status gc_te_plan_run(gc_te_plan* p, const double* d_xyz, double* d_te, void*
         return fail(GC_ERR_INVALID, "null plan or device buffer");
     DeviceScope dev(p->device);
     GC_TRY(dev.st);
-    cudaStream_t s = stream ? (cudaStream_t)stream : p->stream;
-    const int    n = p->natoms;
-    GC_TRY_CUDA(cudaMemsetAsync(p->status.p, 0, sizeof(int), s));
-    GC_TRY_CUDA(cudaMemsetAsync(d_te, 0, sizeof(double) * (size_t)n * n, s));
-    GC_TRY(p->tt.prepare(d_xyz, p->status.p, s));
-    p->launches = 2;
-    GC_TRY_CUDA(cudaEventRecord(p->ev0, s));
-    if (p->walk)
-    {
-        GC_TRY(p->tl.enqueue(p->sms, s));
-        GC_TRY_CUDA(cudaEventRecord(p->ev1, s));
-        GC_TRY_CUDA(gc::launch_te_reduce(p->tt.cnt.p, n, p->Nv, p->K, p->tt.psi.p, d_te, p->sms, s));
-        p->launches += p->tl.launches + 1;
-    }
-    else
-    {
-        if (p->path == GC_PATH_EXACT_FP64)
-            gc::launch_te_exact(p->tt.XT.p, n, p->T, p->K, p->lag, p->tt.cnt.p, s, p->wide);
-        else
-            gc::launch_te_fast(p->tt.XT.p, p->tt.X32.p, p->tt.eps.p, n, p->T, p->K, p->lag, p->tt.cnt.p, s);
-        GC_TRY_CUDA(cudaEventRecord(p->ev1, s));
-        gc::launch_te_finalize(p->tt.cnt.p, n, p->T, p->K, p->lag, p->tt.psi.p, d_te, s, p->wide);
-        p->launches += 2;
-    }
-    GC_TRY_CUDA(cudaGetLastError());
-    GC_TRY_CUDA(cudaEventRecord(p->ev_done, s));
-    return GC_OK;
+    cudaStream_t    s  = stream ? (cudaStream_t)stream : p->stream;
+    const gc_status st = te_plan_enqueue(p, d_xyz, d_te, s);
+    if (st != GC_OK) // ev_done, which the plan's end waits for, is not recorded
+        drain(s);
+    return st;
 }
 
 } // extern "C"
@@ -586,7 +598,10 @@ void gc_te_plan_destroy(gc_te_plan* p)
     if (p->ev1)
         cudaEventDestroy(p->ev1);
     if (p->stream)
+    {
+        cudaStreamSynchronize(p->stream); // an upload that no run followed
         cudaStreamDestroy(p->stream);
+    }
     delete p;
 }
 

@@ -1,0 +1,106 @@
+"""The host code on a CUDA runtime without a GPU (fake_cudart.cpp): what a
+call leaves behind when a runtime call in the middle of it fails, what it does
+when device memory is short, and what it leaves set for other threads."""
+import ctypes
+import subprocess
+
+import numpy as np
+import pytest
+
+from tests.conftest import ROOT
+
+TESTS = ROOT / "tests"
+
+
+@pytest.fixture(scope="module")
+def fake(tmp_path_factory):
+    """The package bound to the library's objects linked with the fake runtime."""
+    import gmx_correlation_b200 as gc
+    from gmx_correlation_b200 import build
+    build.build()
+    so = tmp_path_factory.mktemp("fake") / "libgmxcorr_fake.so"
+    subprocess.run([build.CXX, "-std=c++17", "-O1", "-fPIC", "-shared", "-Wl,-Bsymbolic",
+                    f"-I{build.CUDA_HOME / 'include'}", "-o", str(so), str(TESTS / "fake_cudart.cpp"),
+                    *sorted(str(o) for o in build.BUILD.glob("*.o")), "-lpthread"], check=True)
+    mp = pytest.MonkeyPatch()
+    mp.setenv("GMXCORR_B200_LIB", str(so))
+    mp.setattr(gc, "_lib", None)
+    L = gc.lib()
+    for f in ("fake_calls",):
+        getattr(L, f).restype = ctypes.c_long
+    for f in ("fake_live", "fake_peak"):
+        getattr(L, f).restype = ctypes.c_size_t
+    L.fake_reset.argtypes = [ctypes.c_long]
+    L.fake_limit.argtypes = [ctypes.c_size_t]
+    yield gc
+    mp.undo()
+
+
+def _x(n, T, seed=0):
+    return np.random.default_rng(seed).standard_normal((n, T, 3))
+
+
+def _plan(gc, make):
+    """A plan's run on device buffers of its own stream, then its end without a sync."""
+    p = make()
+    buf = np.zeros(200000)
+    try:
+        p.run(buf.ctypes.data, buf.ctypes.data, None)
+    finally:
+        p.close()
+
+
+CALLS = {
+    "ksg": lambda gc: gc.kraskov_corrmatrix(_x(5, 60), 4),
+    "ksg rows": lambda gc: gc.kraskov_corrmatrix(_x(30, 60), 4),
+    "ksg shard": lambda gc: gc.kraskov_corrmatrix(_x(5, 60), 4, pairs=(1, 7)),
+    "ksg long": lambda gc: gc.kraskov_corrmatrix(_x(2, 16400), 4),
+    "ksg exact": lambda gc: gc.kraskov_corrmatrix(_x(5, 60), 4, path=gc.PATH_EXACT_FP64),
+    "ksg plan": lambda gc: _plan(gc, lambda: gc.KsgPlan(6, 70, 4)),
+    "te plan": lambda gc: _plan(gc, lambda: gc.TePlan(6, 70, 4, 1)),
+    "pair": lambda gc: gc.kraskov_wrap(np.ones((6, 90)), np.ones(91), 1, 0, 4),
+    "prepare": lambda gc: gc.kraskov_prepare(_x(3, 50)),
+    "gauss": lambda gc: gc.gauss_corrmatrix(_x(4, 50)),
+    "gcmi": lambda gc: gc.gcmi_corrmatrix(_x(4, 50)),
+    "te": lambda gc: gc.te_matrix(_x(5, 70), 4, 1),
+    "te rows": lambda gc: gc.te_matrix(_x(30, 70), 4, 1),
+    "ksg batch": lambda gc: gc.ksg_batch([_x(5, 60), _x(3, 50)], 4),
+    "te batch": lambda gc: gc.te_batch([_x(5, 60), _x(3, 50)], 4, 1),
+    "gcmi batch": lambda gc: gc.gcmi_batch([_x(5, 60), _x(3, 50)]),
+    "features": lambda gc: gc.screen_features(_x(4, 60), 4),
+}
+
+
+@pytest.mark.parametrize("kept", [False, True])
+@pytest.mark.parametrize("name", CALLS)
+def test_failed_call_leaves_no_work_pending(fake, name, kept):
+    """Whatever runtime call fails, the streams have drained when the call
+    returns: its device blocks may be handed to the next call at once, and
+    copies from the caller's arrays have ended.  kept: with the plan or graph
+    of an earlier call of the shape."""
+    L, call = fake.lib(), CALLS[name]
+
+    def ready():
+        fake.batch_release()
+        fake.release_cache()
+        if kept:
+            call(fake)
+
+    ready()
+    L.fake_reset(0)
+    call(fake)
+    total = L.fake_calls()
+    assert total > 3 and L.fake_bad() == 0
+    for at in range(1, total + 1):
+        ready()
+        L.fake_reset(at)
+        try:
+            call(fake)
+        except fake.GCError:
+            pass
+        where = f"{name}: runtime call {at} of {total} failed"
+        assert L.fake_pending() == 0, f"{where}: work pending"
+        assert L.fake_bad() == 0, f"{where}: a stream destroyed with work pending"
+        call(fake)
+    fake.batch_release()
+    fake.release_cache()
