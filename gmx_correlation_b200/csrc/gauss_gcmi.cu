@@ -453,8 +453,8 @@ void launch_copula(const double* xyz, int natoms, int T, double* zt, double* Z, 
     while (P < T)
         P <<= 1;
     const size_t smem = (size_t)P * (sizeof(double) + sizeof(int));
-    if (smem > 48 * 1024)
-        cudaFuncSetAttribute(copula_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > 48 * 1024 && allow_dynamic_smem(copula_kernel) != cudaSuccess)
+        return; // the caller finds the error
     const int threads = P / 2 < 512 ? P / 2 : 512;
     copula_kernel<<<natoms * 3, threads, smem, s>>>(xyz, T, P, zt, Z, status);
 }

@@ -10,6 +10,20 @@ namespace gc {
 
 constexpr unsigned kFull = 0xffffffffu;
 
+// Dynamic shared memory a CTA may ask for: the 227 KB opt-in maximum on
+// sm_100 less room for the kernels' static variables.
+constexpr size_t kMaxDynamicSmem = 226 * 1024;
+
+// Lets launches of the kernel use up to kMaxDynamicSmem.  The limit belongs to
+// the function on its device, for all threads of the process: set to one
+// call's own size it could fall, between another thread's call and its launch,
+// below what that launch needs.
+template <class Kernel>
+inline cudaError_t allow_dynamic_smem(Kernel* kernel)
+{
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxDynamicSmem);
+}
+
 // Grid geometry of the joint KSG search for one pair: cells on component 0
 // of atom a1 and component 0 of atom a2 (make_box2ind(x, 6, N, 0, dimx, ...),
 // lib/kraskov.cpp:1294), cell index (int)(x*inveps) & (bs-1) (:69-71), query

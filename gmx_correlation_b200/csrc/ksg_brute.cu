@@ -605,7 +605,8 @@ void launch_ksg_brute(const double* X, int natoms, int T, int K, long pair_begin
     const int  box   = ksg_box_count(T, K), shift = rank_top_shift(box, T);
     const size_t smem = (size_t)3 * chunk * sizeof(float2) + (size_t)warps * bf_warp_bytes(Q);
     auto         go   = [&](auto kernel) {
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (allow_dynamic_smem(kernel) != cudaSuccess)
+            return; // the caller finds the error
         kernel<<<(unsigned)(pair_count * nqb), warps * 32, smem, s>>>(X, mid, eps, T, K, pair_begin, pair_count, pair_ab,
                                                                      nqb, chunk, box, shift, cnt, cnt_y);
     };

@@ -1145,23 +1145,19 @@ cudaError_t launch_ksg_rows(const WalkBatch& b, long long rows, cudaStream_t s)
         kernel = ksg_rows_kernel<256, 16>;
     else if (threads == 512)
         kernel = ksg_rows_kernel<512, 16>;
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_dynamic_smem(kernel);
     if (e != cudaSuccess)
         return e;
     kernel<<<(unsigned)rows, threads, smem, s>>>(b);
     return cudaGetLastError();
 }
 
-// Shared memory budget of one CTA (the 227 KB opt-in maximum on sm_100, less
-// room for the static variables).
-constexpr size_t kSmemBudget = 226 * 1024;
-
 int walk_max_staged_warps(int maxT)
 {
     const size_t rows = (size_t)2 * maxT * 16;
-    if (rows >= kSmemBudget)
+    if (rows >= kMaxDynamicSmem)
         return 0;
-    int w = (int)((kSmemBudget - rows) / ((size_t)kWalkBuckets * 32));
+    int w = (int)((kMaxDynamicSmem - rows) / ((size_t)kWalkBuckets * 32));
     w     = w > kWalkWarps ? kWalkWarps : w;
     return w >= 8 ? w : 0;
 }
@@ -1169,9 +1165,9 @@ int walk_max_staged_warps(int maxT)
 int walk_max_db_warps(int maxT)
 {
     const size_t rows = (size_t)48 * maxT;
-    if (rows >= kSmemBudget)
+    if (rows >= kMaxDynamicSmem)
         return 0;
-    const int w = (int)((kSmemBudget - rows) / ((size_t)kWalkBuckets * 32));
+    const int w = (int)((kMaxDynamicSmem - rows) / ((size_t)kWalkBuckets * 32));
     return w > kWalkWarps ? kWalkWarps : w;
 }
 
@@ -1190,7 +1186,7 @@ cudaError_t launch_ksg_walk(const WalkBatch& b, int warps, bool staged, int sms,
     {
         void (*kernel)(WalkBatch) = lo ? ksg_walk_db_kernel<true> : ksg_walk_db_kernel<false>;
         const size_t smem = (size_t)48 * b.maxT + (size_t)warps * kWalkBuckets * 32;
-        cudaError_t  e    = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t  e    = allow_dynamic_smem(kernel);
         if (e != cudaSuccess)
             return e;
         kernel<<<sms, warps * 32, smem, s>>>(b);
@@ -1202,7 +1198,7 @@ cudaError_t launch_ksg_walk(const WalkBatch& b, int warps, bool staged, int sms,
                  : (staged ? (lo ? ksg_walk_kernel<true, true, false> : ksg_walk_kernel<true, false, false>)
                            : (lo ? ksg_walk_kernel<false, true, false> : ksg_walk_kernel<false, false, false>));
     const size_t smem = (staged ? (size_t)2 * b.maxT * 16 : 0) + (size_t)warps * kWalkBuckets * 32;
-    cudaError_t  e    = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t  e    = allow_dynamic_smem(kernel);
     if (e != cudaSuccess)
         return e;
     int per_sm = 0;
@@ -1217,7 +1213,7 @@ cudaError_t launch_ksg_walk(const WalkBatch& b, int warps, bool staged, int sms,
 cudaError_t launch_ksg_finish(const WalkBatch& b, int sms, cudaStream_t s)
 {
     const size_t smem = (size_t)kFinishWarps * kBandSlotBytes * kBandCap * 32;
-    cudaError_t  e    = cudaFuncSetAttribute(ksg_finish_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t  e    = allow_dynamic_smem(ksg_finish_kernel);
     if (e != cudaSuccess)
         return e;
     int per_sm = 0;

@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(1024, 1) ksg_row_walk_kernel(WalkBatch B)
 
 int row_walk_warps(int maxT, int* ctas)
 {
-    const size_t tile = rw_tile_bytes(maxT), warp = kRwHistBytes + kRwStageBytes, all = (size_t)226 * 1024;
+    const size_t tile = rw_tile_bytes(maxT), warp = kRwHistBytes + kRwStageBytes, all = kMaxDynamicSmem;
     *ctas             = 1;
     if (tile + 8 * warp > all)
         return 0;
@@ -184,7 +184,7 @@ cudaError_t launch_ksg_row_walk(const WalkBatch& b, long long queries, int maxn,
     int          ctas  = 1;
     const int    warps = row_walk_warps(b.maxT, &ctas);
     const size_t smem  = rw_tile_bytes(b.maxT) + (size_t)warps * (kRwHistBytes + kRwStageBytes);
-    e = cudaFuncSetAttribute(ksg_row_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    e = allow_dynamic_smem(ksg_row_walk_kernel);
     if (e != cudaSuccess)
         return e;
     ksg_row_walk_kernel<<<sms * ctas, warps * 32, smem, s>>>(b);

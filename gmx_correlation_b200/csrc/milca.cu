@@ -377,8 +377,7 @@ cudaError_t launch_milca(const MilcaParams& p, const MilcaSum& s, cudaStream_t s
     const size_t smem = milca_smem_per_warp(p.krange, Kp) * kMilcaWarps;
     if (smem > 48 * 1024)
     {
-        const cudaError_t e = cudaFuncSetAttribute(milca_query_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   (int)smem);
+        const cudaError_t e = allow_dynamic_smem(milca_query_kernel);
         if (e != cudaSuccess)
             return e;
     }

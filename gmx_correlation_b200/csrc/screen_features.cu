@@ -424,7 +424,7 @@ cudaError_t launch_screen_features(const double* xyz, int natoms, int T, int K, 
     while (P < T)
         P <<= 1;
     const size_t smem = (size_t)P * 8;
-    cudaError_t  e    = cudaFuncSetAttribute(screen_atom_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t  e    = allow_dynamic_smem(screen_atom_kernel);
     if (e != cudaSuccess)
         return e;
     screen_atom_kernel<<<natoms, 256, smem, s>>>(xyz, T, P, stats, bins);

@@ -421,7 +421,7 @@ namespace {
 // Warps per CTA and CTAs per SM beside a tile (0: it does not leave room for `least`).
 int te_row_warps(size_t tile, size_t warp_bytes, int least, int* ctas)
 {
-    const size_t all = (size_t)226 * 1024, half = all / 2 - 1024;
+    const size_t all = kMaxDynamicSmem, half = all / 2 - 1024;
     *ctas            = 1;
     if (tile + least * warp_bytes > all)
         return 0;
@@ -461,7 +461,7 @@ cudaError_t launch_te_row_walk(const TeBatch& b, long long queries, int maxn, in
     const size_t tile  = rw_tile_bytes(b.maxNv);
     const int    warps = te_row_warps(tile, kRwHistBytes + kRwStageBytes, 8, &ctas);
     const size_t smem  = tile + (size_t)warps * (kRwHistBytes + kRwStageBytes);
-    e = cudaFuncSetAttribute(te_row_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    e = allow_dynamic_smem(te_row_walk_kernel);
     if (e != cudaSuccess)
         return e;
     te_row_walk_kernel<<<sms * ctas, warps * 32, smem, s>>>(b);
@@ -476,7 +476,7 @@ cudaError_t launch_te_row_count(const TeBatch& b, long long queries, int sms, cu
     const size_t tile  = 2 * rw_tile_bytes(b.maxNv);
     const int    warps = te_row_warps(tile, kTeCountWarpBytes, 16, &ctas);
     const size_t smem  = tile + (size_t)warps * kTeCountWarpBytes;
-    cudaError_t  e = cudaFuncSetAttribute(te_row_count_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t  e = allow_dynamic_smem(te_row_count_kernel);
     if (e != cudaSuccess)
         return e;
     te_row_count_kernel<<<sms * ctas, warps * 32, smem, s>>>(b);

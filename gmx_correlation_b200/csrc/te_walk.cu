@@ -1057,7 +1057,7 @@ cudaError_t launch_te_rows(const TeBatch& b, long long rows, cudaStream_t s)
         kernel = te_rows_kernel<256, 16>;
     else if (threads == 512)
         kernel = te_rows_kernel<512, 16>;
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_dynamic_smem(kernel);
     if (e != cudaSuccess)
         return e;
     kernel<<<(unsigned)rows, threads, smem, s>>>(b);
@@ -1070,12 +1070,12 @@ cudaError_t launch_te_walk(const TeBatch& b, int warps, bool staged, int sms, cu
     // two staged pair tasks per CTA (12-byte rows) where they fit beside the
     // warps' histograms, else one (16-byte rows)
     const size_t hist = (size_t)warps * kWalkBuckets * 32;
-    const bool   dbuf = staged && (size_t)48 * b.maxT + hist <= (size_t)226 * 1024;
+    const bool   dbuf = staged && (size_t)48 * b.maxT + hist <= kMaxDynamicSmem;
     void (*kernel)(TeBatch) = dbuf     ? (lo ? te_walk_db_kernel<true> : te_walk_db_kernel<false>)
                               : staged ? (lo ? te_walk_kernel<true, true> : te_walk_kernel<true, false>)
                                        : (lo ? te_walk_kernel<false, true> : te_walk_kernel<false, false>);
     const size_t smem = (dbuf ? (size_t)48 * b.maxT : (staged ? (size_t)2 * b.maxT * 16 : 0)) + hist;
-    cudaError_t  e    = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t  e    = allow_dynamic_smem(kernel);
     if (e != cudaSuccess)
         return e;
     int per_sm = 0;
@@ -1090,7 +1090,7 @@ cudaError_t launch_te_walk(const TeBatch& b, int warps, bool staged, int sms, cu
 cudaError_t launch_te_finish(const TeBatch& b, int sms, cudaStream_t s)
 {
     const size_t smem = (size_t)kTeFinishWarps * 6 * kTeBandCap * 32;
-    cudaError_t  e    = cudaFuncSetAttribute(te_finish_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t  e    = allow_dynamic_smem(te_finish_kernel);
     if (e != cudaSuccess)
         return e;
     int per_sm = 0;
@@ -1110,7 +1110,7 @@ cudaError_t launch_te_count(const TeBatch& b, int warps, bool staged, int sms, c
     const bool   dbuf    = staged && db <= (size_t)224 * 1024;
     void (*kernel)(TeBatch) = dbuf ? te_count_db_kernel : (staged ? te_count_kernel<true> : te_count_kernel<false>);
     const size_t smem = dbuf ? db : (staged ? (size_t)2 * b.maxT * 16 : 0);
-    cudaError_t  e    = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t  e    = allow_dynamic_smem(kernel);
     if (e != cudaSuccess)
         return e;
     int per_sm = 0;

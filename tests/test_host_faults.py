@@ -104,3 +104,27 @@ def test_failed_call_leaves_no_work_pending(fake, name, kept):
         call(fake)
     fake.batch_release()
     fake.release_cache()
+
+
+def test_shared_memory_limits_do_not_depend_on_the_call(fake):
+    """A kernel's dynamic shared memory limit belongs to the function on its
+    device: a value of one call's own could lower it between another thread's
+    setting it and its launch."""
+    fake.release_cache()
+    for n, T, k in ((30, 200, 5), (30, 2500, 5), (5, 900, 300), (4, 7000, 6), (3, 12000, 6), (2, 16500, 9)):
+        x = _x(n, T)
+        fake.kraskov_corrmatrix(x, k)
+        fake.te_matrix(x, k, 1)
+        fake.gcmi_corrmatrix(x)
+        fake.kraskov_wrap(np.ones((6, T)), np.ones(T + 1), 1, 0, k)
+        if T <= 16384:
+            fake.screen_features(x, k)
+    for T in (300, 2500, 900):
+        fake.ksg_batch([_x(30, T), _x(5, T // 2)], 5)
+        fake.te_batch([_x(30, T), _x(5, T // 2)], 5, 1)
+    fake.batch_release()
+    fake.release_cache()
+    names = ctypes.create_string_buffer(4096)
+    varying = fake.lib().fake_varying_limits(names, 4096)
+    assert fake.lib().fake_limited() > 10
+    assert varying == 0, names.value.decode()
