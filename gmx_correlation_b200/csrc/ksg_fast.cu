@@ -79,28 +79,51 @@ __global__ void ksg_x32_kernel(const double* __restrict__ X64, int natoms, int T
         eps_atom[a] = __double2float_ru(R * (1.0 + 0x1p-40) * 0x1p-21) + 1e-30f;
 }
 
+namespace {
+
+// Row r of a launch's row sort: descriptor, atom and query of its block.
+struct RowOf
+{
+    const WalkParams* w;
+    int               a, iq;
+};
+
+__device__ __forceinline__ RowOf row_of(const WalkBatch& B, long long r)
+{
+    const int         dsc = batch_desc(B.rprefix, B.n, r);
+    const WalkParams* w   = B.d + dsc;
+    const int         row = (int)(r - B.rprefix[dsc]), a = row / w->Q;
+    return RowOf{w, a, row - a * w->Q};
+}
+
+// Distances of the row's query to its atom's frames.
+struct RowDist
+{
+    const float4*                    x;
+    float4                           q;
+    __device__ __forceinline__ explicit RowDist(const RowOf& o)
+        : x(o.w->X32 + (size_t)o.a * o.w->T), q(x[o.w->i0 + o.iq])
+    {
+    }
+    __device__ __forceinline__ float operator()(int j) const { return dist3f(q, x[j]); }
+};
+
+} // namespace
+
 // One CTA per (atom, query) of the launch's query blocks: the row's T-1
 // marginal distances (self excluded) in bucket order with their frames
 // (sort_row).
 template <int THREADS, int R>
 __global__ void __launch_bounds__(THREADS, row_ctas(THREADS, R)) ksg_rows_kernel(WalkBatch B)
 {
-    // row blockIdx.x of the launch -> descriptor, atom, query of its block
-    const long long   r   = blockIdx.x;
-    const int         dsc = batch_desc(B.rprefix, B.n, r);
-    const WalkParams& w   = B.d[dsc];
-    const int         T = w.T, Q = w.Q, Qp = w.Qp, Lpad = w.Lpad;
-    const int         row = (int)(r - B.rprefix[dsc]);
-    const int         a   = row / Q;
-    const int         iq  = row - a * Q;
-    const int         i   = w.i0 + iq;
-    const float4*     xr  = w.X32 + (size_t)a * T;
-    const float4      q   = xr[i];
+    const RowOf       o = row_of(B, blockIdx.x);
+    const WalkParams& w = *o.w;
     __shared__ RowSortShared<THREADS> sh;
     sort_row<THREADS, R>(
-        sh, T - 1, i, row_top(w.eps_atom[a]), [&](int j) { return dist3f(q, xr[j]); }, w.S, w.P,
-        ((size_t)a * (Lpad >> 2) * Qp + ((size_t)iq << w.run)) * 4, ((size_t)Qp * 4) << w.run, w.run,
-        w.U ? w.U + ((size_t)a * Qp + iq) * w.Tpad : nullptr);
+        sh, w.T - 1, w.i0 + o.iq, row_top(w.eps_atom[o.a]), RowDist(o),
+        [&B]() { return RowDist(row_of(B, rows_block())); }, w.S, w.P,
+        ((size_t)o.a * (w.Lpad >> 2) * w.Qp + ((size_t)o.iq << w.run)) * 4, ((size_t)w.Qp * 4) << w.run, w.run,
+        w.U ? w.U + ((size_t)o.a * w.Qp + o.iq) * w.Tpad : nullptr);
 }
 
 namespace {

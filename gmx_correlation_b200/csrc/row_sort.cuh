@@ -13,7 +13,13 @@ namespace gc {
 // with their frames by a counting sort over fine buckets of 2^kRowFine float
 // ulps (an eighth of the walks' narrowest buckets).  kRowBins buckets end at the
 // largest possible distance (8 octaves); entries below them are put in full
-// order, or, if they are many, the whole row is, by a bitonic network.
+// order, or, if they are many, sorted again in the same way by the buckets that
+// end at the largest of them.  That happens where an atom's largest distance is
+// over 256 times a usual one: a broken frame, a stretch of frames in another
+// periodic image.  FP32 coordinates leave no room for a fourth level but
+// distances of zero.  One frame 200 nm off, by a bitonic network over the whole
+// row and by levels: 80 x 4999, k = 100: 236 -> 59.6 ms for the matrix, TE
+// 30 x 5000 167 -> 35.6 ms, 64 x 900 4.37 -> 2.40 ms.
 // R > 0: each thread keeps its R distances (entries tid + r * threads) in
 // registers; R = 0: they are recomputed (from L1-resident coordinate rows)
 // for the second pass.
@@ -52,45 +58,130 @@ template <int THREADS>
 struct RowSortShared
 {
     unsigned wsum[THREADS / 32];
-    int      full; // order the row by the bitonic network
+    unsigned low;                // entries below the buckets
+    unsigned wmax[THREADS / 32]; // largest of them by warp
 };
+
+// Bucket of a distance, where cb is the code of bucket 0.
+__device__ __forceinline__ int rows_bin(float d, int cb)
+{
+    return min(max((int)(__float_as_uint(d) >> kRowFine) - cb, 0), kRowBins - 1);
+}
+
+// Counter b of the cursors: adds 1 and returns its value before.
+__device__ __forceinline__ unsigned rows_bump(unsigned* cursor, int b)
+{
+    const int sh = (b & 1) * 16;
+    return (atomicAdd(&cursor[rows_word(b >> 1)], 1u << sh) >> sh) & 0xFFFFu;
+}
+
+template <int THREADS>
+__device__ __forceinline__ void rows_clear(unsigned* cursor, int tid)
+{
+    for (int b = tid * 4; b < kRowBins / 2; b += THREADS * 4)
+        *reinterpret_cast<uint4*>(cursor + b) = make_uint4(0u, 0u, 0u, 0u);
+}
+
+// Exclusive scan of the counters in place (each thread a contiguous slice),
+// with a barrier before and after.  Returns the first counter.
+template <int THREADS>
+__device__ __forceinline__ unsigned rows_scan(RowSortShared<THREADS>& sh, unsigned* cursor, int tid)
+{
+    const int     lane = tid & 31, warp = tid >> 5;
+    constexpr int kSlice = kRowBins / 2 / THREADS; // words
+    constexpr int kVec   = kSlice < 4 ? kSlice : 4;
+    using Vec            = typename std::conditional<kVec == 4, uint4, uint2>::type;
+    static_assert(kVec >= 2 && kSlice % kVec == 0, "slices by vectors");
+    union Words
+    {
+        Vec      v;
+        unsigned w[kVec];
+    };
+    auto slice = [cursor, tid](int v) { return reinterpret_cast<Vec*>(cursor + rows_word(tid * kSlice + v)); };
+    __syncthreads();
+    unsigned loc = 0;
+#pragma unroll
+    for (int v = 0; v < kSlice; v += kVec)
+    {
+        Words c;
+        c.v = *slice(v);
+        if (v == 0 && tid == 0)
+            sh.low = c.w[0] & 0xFFFFu;
+#pragma unroll
+        for (int e = 0; e < kVec; ++e)
+        {
+            loc += (c.w[e] & 0xFFFFu) + (c.w[e] >> 16);
+        }
+    }
+    unsigned incl = loc;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1)
+    {
+        const unsigned y = __shfl_up_sync(kFull, incl, o);
+        if (lane >= o)
+            incl += y;
+    }
+    if (lane == 31)
+        sh.wsum[warp] = incl;
+    __syncthreads();
+    const unsigned low = sh.low;
+    unsigned       run = incl - loc;
+    for (int w = 0; w < warp; ++w)
+        run += sh.wsum[w];
+#pragma unroll
+    for (int v = 0; v < kSlice; v += kVec)
+    {
+        Words c;
+        c.v = *slice(v);
+#pragma unroll
+        for (int e = 0; e < kVec; ++e)
+        {
+            const unsigned n = c.w[e], mid = run + (n & 0xFFFFu);
+            c.w[e]           = run | (mid << 16);
+            run              = mid + (n >> 16);
+        }
+        *slice(v) = c.v;
+    }
+    __syncthreads();
+    return low;
+}
+
+// blockIdx.x as a value of its own: what is computed from it is not what was
+// computed before, kept in registers.
+__device__ __forceinline__ long long rows_block()
+{
+    long long r = blockIdx.x;
+    asm volatile("" : "+l"(r));
+    return r;
+}
 
 // Sorts the row of query frame i over frames 0 .. N (i excluded, N entries
 // in all): dist(j) gives the FP32 distance from the query to frame j, at most
 // top.  The distances and frames go to S / P at base + row_entry(m, gstride,
 // run_log) for entry m (the transposed layout of the walk), the last 4-entry
 // group padded with NaN and frame 0.  Every thread of the CTA calls it; it
-// uses the dynamic shared memory of row_sort_smem.  U_row (optional) receives
-// the unsorted distances at U_row[j].
-template <int THREADS, int R, class DistFn>
+// uses the dynamic shared memory of row_sort_smem.  again() gives dist anew,
+// for the further levels, so that the usual rows' registers do not carry it.
+// U_row (optional) receives the unsorted distances at U_row[j].
+template <int THREADS, int R, class DistFn, class AgainFn>
 __device__ __forceinline__ void sort_row(RowSortShared<THREADS>& sh, int N, int i, float top, DistFn&& dist,
-                                         float* __restrict__ S, uint16_t* __restrict__ P, size_t base,
+                                         AgainFn&& again, float* __restrict__ S, uint16_t* __restrict__ P, size_t base,
                                          size_t gstride, int run_log,
                                          float* __restrict__ U_row = nullptr)
 {
     extern __shared__ __align__(16) unsigned char rows_smem[];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x;
     const int Np     = (N + 3) & ~3;                               // whole 4-entry groups
     unsigned* cursor = reinterpret_cast<unsigned*>(rows_smem);     // [kRowBins / 2]
     unsigned* vals   = cursor + kRowBins / 2;                        // [Np] distance bits in bucket order
     uint16_t* frm    = reinterpret_cast<uint16_t*>(vals + Np);     // [Np] their frames
     auto      frame_of = [i](int m) { return m < i ? m : m + 1; };
-    const int cb       = (int)(__float_as_uint(top) >> kRowFine) - (kRowBins - 1);
-    auto bin_of = [&](float d) -> int { return min(max((int)(__float_as_uint(d) >> kRowFine) - cb, 0), kRowBins - 1); };
-
-    if (tid == 0)
-        sh.full = 0;
-    // counter b: adds 1 and returns its value before / reads it
-    auto bump = [cursor](int b) -> unsigned {
-        const int sh = (b & 1) * 16;
-        return (atomicAdd(&cursor[rows_word(b >> 1)], 1u << sh) >> sh) & 0xFFFFu;
-    };
-    auto start_of = [cursor](int b) -> unsigned { return (cursor[rows_word(b >> 1)] >> ((b & 1) * 16)) & 0xFFFFu; };
-    for (int b = tid * 4; b < kRowBins / 2; b += THREADS * 4)
-        *reinterpret_cast<uint4*>(cursor + b) = make_uint4(0u, 0u, 0u, 0u);
+    const int cb       = (int)(__float_as_uint(top) >> kRowFine) - (kRowBins - 1); // code of bucket 0
+    auto      start_of = [cursor](int b) -> unsigned { return (cursor[rows_word(b >> 1)] >> ((b & 1) * 16)) & 0xFFFFu; };
+    rows_clear<THREADS>(cursor, tid);
     // the row's distances, and later each key's arrival in its bucket
     float    dreg[R > 0 ? R : 1];
-    unsigned areg[R > 0 ? (R + 1) / 2 : 1]; // two 16-bit numbers each
+    unsigned areg[R > 0 ? (R + 1) / 2 : 1] = {}; // two 16-bit numbers each
     if constexpr (R > 0)
     {
 #pragma unroll
@@ -123,7 +214,7 @@ __device__ __forceinline__ void sort_row(RowSortShared<THREADS>& sh, int N, int 
         each([&](int, int m, float d) { U_row[frame_of(m)] = d; });
     __syncthreads();
     each([&](int k, int, float d) {
-        const unsigned o = bump(bin_of(d));
+        const unsigned o = rows_bump(cursor, rows_bin(d, cb));
         if constexpr (R > 0)
         {
             if (k & 1)
@@ -132,157 +223,87 @@ __device__ __forceinline__ void sort_row(RowSortShared<THREADS>& sh, int N, int 
                 areg[k >> 1] = o;
         }
     });
-    __syncthreads();
-    // exclusive scan in place: each thread a contiguous slice
-    unsigned low = 0; // thread 0: entries below the buckets
-    constexpr int kSlice = kRowBins / 2 / THREADS; // words
-    constexpr int kVec   = kSlice < 4 ? kSlice : 4;
-    using Vec            = typename std::conditional<kVec == 4, uint4, uint2>::type;
-    static_assert(kVec >= 2 && kSlice % kVec == 0, "slices by vectors");
-    union Words
+    unsigned low = rows_scan<THREADS>(sh, cursor, tid);
+    each([&](int k, int m, float d) {
+        unsigned at;
+        if constexpr (R > 0)
+            at = start_of(rows_bin(d, cb)) + ((areg[k >> 1] >> ((k & 1) * 16)) & 0xFFFFu);
+        else
+            at = rows_bump(cursor, rows_bin(d, cb));
+        vals[at] = __float_as_uint(d);
+        frm[at]  = (uint16_t)frame_of(m);
+    });
+    if (tid < Np - N)
     {
-        Vec      v;
-        unsigned w[kVec];
-    };
-    auto slice = [cursor, tid](int v) { return reinterpret_cast<Vec*>(cursor + rows_word(tid * kSlice + v)); };
-    unsigned loc = 0;
-#pragma unroll
-    for (int v = 0; v < kSlice; v += kVec)
-    {
-        Words c;
-        c.v = *slice(v);
-        if (v == 0 && tid == 0)
-            low = c.w[0] & 0xFFFFu;
-#pragma unroll
-        for (int e = 0; e < kVec; ++e)
-        {
-            loc += (c.w[e] & 0xFFFFu) + (c.w[e] >> 16);
-        }
-    }
-    unsigned incl = loc;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1)
-    {
-        const unsigned y = __shfl_up_sync(kFull, incl, o);
-        if (lane >= o)
-            incl += y;
-    }
-    if (lane == 31)
-        sh.wsum[warp] = incl;
-    if (low > (unsigned)kRowLow)
-        sh.full = 1;
-    __syncthreads();
-    unsigned run = incl - loc;
-    for (int w = 0; w < warp; ++w)
-        run += sh.wsum[w];
-#pragma unroll
-    for (int v = 0; v < kSlice; v += kVec)
-    {
-        Words c;
-        c.v = *slice(v);
-#pragma unroll
-        for (int e = 0; e < kVec; ++e)
-        {
-            const unsigned n = c.w[e], mid = run + (n & 0xFFFFu);
-            c.w[e]           = run | (mid << 16);
-            run              = mid + (n >> 16);
-        }
-        *slice(v) = c.v;
+        vals[N + tid] = 0x7fc00000u;
+        frm[N + tid]  = 0;
     }
     __syncthreads();
-    const bool full = sh.full;
-    if (!full)
+    // Further levels: the entries in bucket 0 or below it, which lie in the
+    // row's first places, go there again by the buckets that end at the largest
+    // of them (their distances recomputed: the first level's registers are free).
+#pragma unroll 1
+    while (low > (unsigned)kRowLow)
     {
-        each([&](int k, int m, float d) {
-            unsigned at;
-            if constexpr (R > 0)
-                at = start_of(bin_of(d)) + ((areg[k >> 1] >> ((k & 1) * 16)) & 0xFFFFu);
-            else
-                at = bump(bin_of(d));
-            vals[at] = __float_as_uint(d);
-            frm[at]  = (uint16_t)frame_of(m);
-        });
-        if (tid < Np - N)
-        {
-            vals[N + tid] = 0x7fc00000u;
-            frm[N + tid]  = 0;
-        }
+        int t = tid;
+        asm volatile("" : "+r"(t)); // its addresses are not the first level's, kept in registers
+        unsigned most = 0;
+#pragma unroll 1
+        for (unsigned e = t; e < low; e += THREADS)
+            most = max(most, vals[e]);
+        most = __reduce_max_sync(kFull, most);
+        if ((t & 31) == 0)
+            sh.wmax[t >> 5] = most;
+        rows_clear<THREADS>(cursor, t);
         __syncthreads();
-        if (tid == 0 && low > 1u) // the entries below the buckets, by insertion
-            for (unsigned x = 1; x < low; ++x)
+#pragma unroll 1
+        for (int w = 0; w < THREADS / 32; ++w)
+            most = max(most, sh.wmax[w]);
+        const int  at0  = (int)(most >> kRowFine) - (kRowBins - 1);
+        const auto same = again();
+        auto       here = [&](auto&& fn) {
+#pragma unroll 1
+            for (int m = t; m < N; m += THREADS)
             {
-                const unsigned v = vals[x];
-                const uint16_t f = frm[x];
-                unsigned       y = x;
-                for (; y > 0 && vals[y - 1] > v; --y)
-                {
-                    vals[y] = vals[y - 1];
-                    frm[y]  = frm[y - 1];
-                }
-                vals[y] = v;
-                frm[y]  = f;
+                const int   j = frame_of(m);
+                const float d = same(j);
+                if (__float_as_uint(d) <= most)
+                    fn(j, d);
             }
-        __syncthreads();
-    }
-    else
-    {
-        // bitonic network on (distance, frame), over the same shared memory
-        unsigned long long* keys = reinterpret_cast<unsigned long long*>(rows_smem); // [N2]
-        int                 N2   = THREADS;
-        while (N2 < N)
-            N2 <<= 1;
-        each([&](int, int m, float d) {
-            keys[m] = ((unsigned long long)__float_as_uint(d) << 32) | (unsigned)frame_of(m);
+        };
+        here([&](int, float d) { rows_bump(cursor, rows_bin(d, at0)); });
+        low = rows_scan<THREADS>(sh, cursor, t);
+        here([&](int j, float d) {
+            const unsigned at = rows_bump(cursor, rows_bin(d, at0));
+            vals[at]          = __float_as_uint(d);
+            frm[at]           = (uint16_t)j;
         });
-        for (int m = N + tid; m < N2; m += THREADS)
-            keys[m] = ~0ull;
         __syncthreads();
-        for (int k = 2; k <= N2; k <<= 1)
-            for (int j = k >> 1; j > 0; j >>= 1)
-            {
-                for (int t = tid; t < (N2 >> 1); t += THREADS)
-                {
-                    const int                idx = ((t / j) * (j << 1)) + (t % j);
-                    const int                prt = idx + j;
-                    const unsigned long long x = keys[idx], y = keys[prt];
-                    if ((x > y) == ((idx & k) == 0))
-                    {
-                        keys[idx] = y;
-                        keys[prt] = x;
-                    }
-                }
-                __syncthreads();
-            }
     }
+    if (tid == 0) // the entries below the buckets, by insertion
+        for (unsigned x = 1; x < low; ++x)
+        {
+            const unsigned v = vals[x];
+            const uint16_t f = frm[x];
+            unsigned       y = x;
+            for (; y > 0 && vals[y - 1] > v; --y)
+            {
+                vals[y] = vals[y - 1];
+                frm[y]  = frm[y - 1];
+            }
+            vals[y] = v;
+            frm[y]  = f;
+        }
+    __syncthreads();
     // transposed layout: one thread per group of 4 consecutive entries, the
     // queries of a block side by side (see WalkParams).  The last group runs
     // out in NaN (never <= any stop value) with frame 0, so the walk reads
     // whole groups without a bounds test.
-    const unsigned long long* keys = reinterpret_cast<const unsigned long long*>(rows_smem);
     for (int g = tid; g * 4 < N; g += THREADS)
     {
-        uint4 v;
-        uint2 f;
-        if (!full)
-        {
-            v = *reinterpret_cast<const uint4*>(vals + g * 4);
-            f = *reinterpret_cast<const uint2*>(frm + g * 4);
-        }
-        else
-        {
-            unsigned b[4], j[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q)
-            {
-                const bool in = g * 4 + q < N;
-                b[q]          = in ? (unsigned)(keys[g * 4 + q] >> 32) : 0x7fc00000u;
-                j[q]          = in ? (unsigned)keys[g * 4 + q] & 0xFFFFu : 0u;
-            }
-            v = make_uint4(b[0], b[1], b[2], b[3]);
-            f = make_uint2(j[0] | (j[1] << 16), j[2] | (j[3] << 16));
-        }
-        *reinterpret_cast<uint4*>(S + base + row_entry(g * 4, gstride, run_log)) = v;
-        *reinterpret_cast<uint2*>(P + base + row_entry(g * 4, gstride, run_log)) = f;
+        const size_t at                  = base + row_entry(g * 4, gstride, run_log);
+        *reinterpret_cast<uint4*>(S + at) = *reinterpret_cast<const uint4*>(vals + g * 4);
+        *reinterpret_cast<uint2*>(P + at) = *reinterpret_cast<const uint2*>(frm + g * 4);
     }
 }
 
@@ -307,11 +328,7 @@ inline size_t row_sort_smem(int N, int* threads, int* regs)
 {
     *threads = N <= 8 * 64 ? 64 : (N <= 16 * 128 ? 128 : (N <= 16 * 256 ? 256 : (N <= 16 * 512 ? 512 : 1024)));
     *regs    = N <= 8 * 128 ? 8 : (N <= 16 * 512 ? 16 : 0);
-    size_t N2 = (size_t)*threads; // the bitonic network's keys
-    while (N2 < (size_t)N)
-        N2 <<= 1;
-    const size_t need = (size_t)kRowBins * 2 + (((size_t)N + 3) & ~(size_t)3) * 6;
-    return need > N2 * 8 ? need : N2 * 8;
+    return (size_t)kRowBins * 2 + (((size_t)N + 3) & ~(size_t)3) * 6;
 }
 
 } // namespace gc

@@ -94,36 +94,65 @@ constexpr int kTeAmbCap = 8;
 // Sorted rows: blocks [0, natoms * Q) of a descriptor are G rows, the next
 // natoms * Q the M rows, each over the frames j < N_valid, j != qi.
 // ---------------------------------------------------------------------------
+namespace {
+
+// Row r of a launch's row sort.
+struct TeRowOf
+{
+    const TeParams* p;
+    int             a, iq;
+    bool            g;
+};
+
+__device__ __forceinline__ TeRowOf te_row_of(const TeBatch& B, long long r)
+{
+    const int       dsc = te_desc_of(B.rprefix, B.n, r);
+    const TeParams* p   = B.d + dsc;
+    const int       row = (int)(r - B.rprefix[dsc]), per = p->natoms * p->Q;
+    const bool      g   = row < per;
+    const int       rem = g ? row : row - per, a = rem / p->Q;
+    return TeRowOf{p, a, rem - a * p->Q, g};
+}
+
+// Distances of the row's query over its atom's frames: future and past (G), or
+// the past alone.
+template <bool G>
+struct TeRowDist
+{
+    const float4*                    x;
+    float4                           qp, qf;
+    int                              lag;
+    __device__ __forceinline__ explicit TeRowDist(const TeRowOf& o)
+        : x(o.p->X32 + (size_t)o.a * o.p->T), qp(x[o.p->i0 + o.iq]), qf(qp), lag(o.p->lag)
+    {
+        if (G)
+            qf = x[o.p->i0 + o.iq + lag];
+    }
+    __device__ __forceinline__ float operator()(int j) const
+    {
+        return G ? fmaxf(te3(qf, x[j + lag]), te3(qp, x[j])) : te3(qp, x[j]);
+    }
+};
+
+} // namespace
+
 template <int THREADS, int R>
 __global__ void __launch_bounds__(THREADS, row_ctas(THREADS, R)) te_rows_kernel(TeBatch B)
 {
-    const long long r   = blockIdx.x;
-    const int       dsc = te_desc_of(B.rprefix, B.n, r);
-    const TeParams& p   = B.d[dsc];
-    const int       row = (int)(r - B.rprefix[dsc]);
-    const int       per = p.natoms * p.Q;
-    const bool      g   = row < per;
-    const int       rem = g ? row : row - per;
-    const int       a   = rem / p.Q;
-    const int       iq  = rem - a * p.Q;
-    const int       qi  = p.i0 + iq;
-    const int       lag = p.lag;
-    const float4*   xr  = p.X32 + (size_t)a * p.T;
-    const float4    qp  = xr[qi];
-    const size_t    base = ((size_t)a * (p.Lpad >> 2) * p.Qp + ((size_t)iq << p.run)) * 4;
+    const TeRowOf   o   = te_row_of(B, blockIdx.x);
+    const TeParams& p   = *o.p;
+    const size_t    base = ((size_t)o.a * (p.Lpad >> 2) * p.Qp + ((size_t)o.iq << p.run)) * 4;
     const size_t    gs   = ((size_t)p.Qp * 4) << p.run;
-    const float     top = row_top(p.eps_atom[a]);
+    const float     top  = row_top(p.eps_atom[o.a]);
     __shared__ RowSortShared<THREADS> sh;
-    if (g)
-    {
-        const float4 qf = xr[qi + lag];
+    if (o.g)
         sort_row<THREADS, R>(
-            sh, p.Nv - 1, qi, top, [&](int j) { return fmaxf(te3(qf, xr[j + lag]), te3(qp, xr[j])); }, p.SG, p.PG, base,
-            gs, p.run);
-    }
+            sh, p.Nv - 1, p.i0 + o.iq, top, TeRowDist<true>(o),
+            [&B]() { return TeRowDist<true>(te_row_of(B, rows_block())); }, p.SG, p.PG, base, gs, p.run);
     else
-        sort_row<THREADS, R>(sh, p.Nv - 1, qi, top, [&](int j) { return te3(qp, xr[j]); }, p.SM, p.PM, base, gs,
-                             p.run);
+        sort_row<THREADS, R>(
+            sh, p.Nv - 1, p.i0 + o.iq, top, TeRowDist<false>(o),
+            [&B]() { return TeRowDist<false>(te_row_of(B, rows_block())); }, p.SM, p.PM, base, gs, p.run);
 }
 
 // ---------------------------------------------------------------------------
