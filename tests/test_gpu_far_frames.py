@@ -69,3 +69,27 @@ def test_a_far_frame_costs_little_more(gc, n, T, k, lag):
     the same trajectory without it leaves room for more than two whole sorts
     (a full sort of such rows took 5 to 9 times)."""
     assert _ms(gc, _traj("frame", n, T, 3), k, lag) < 3.0 * _ms(gc, _traj("smooth", n, T, 3), k, lag)
+
+
+def _handoffs(gc, x, k, pair_list=None):
+    torch = pytest.importorskip("torch")
+    n, T = x.shape[0], x.shape[1]
+    p = gc.KsgPlan(n, T, k, pair_list=pair_list)
+    d_x = torch.from_numpy(np.ascontiguousarray(x)).cuda()
+    d_out = torch.zeros(n * (n - 1) // 2, dtype=torch.float64, device="cuda")
+    p.run(d_x.data_ptr(), d_out.data_ptr())
+    p.sync()
+    h = p.handoffs
+    p.close()
+    return h
+
+
+@pytest.mark.parametrize("n,T,k", [(60, 2000, 100), (30, 3000, 10)])
+def test_rows_for_many_pairs_hand_over_no_more(gc, n, T, k):
+    """The walk of a row for 32 pairs at once settles the queries that the walk
+    with one query per lane (pair lists) settles: both count into the same
+    buckets up to a query's bracket.  They differ in how far behind it an
+    overflow still counts (up to 16 entries here, one bucket there)."""
+    x = _traj("stretch", n, T, seed=7)
+    one = _handoffs(gc, x, k, pair_list=np.arange(n * (n - 1) // 2))
+    assert _handoffs(gc, x, k) <= 1.05 * one + 50
