@@ -75,7 +75,8 @@ __host__ __device__ constexpr size_t bf_warp_bytes(int q)
 
 } // namespace
 
-// Midrange of every component and the atom's FP32 error bound (as ksg_x32_kernel).
+// Midrange of every component and the atom's FP32 error bound (as ksg_x32_kernel;
+// infinite where FP32 does not hold the centred coordinates).
 __global__ void __launch_bounds__(256) ksg_range_kernel(const double* __restrict__ X, int T, double* __restrict__ mid,
                                                         float* __restrict__ eps_atom)
 {
@@ -110,9 +111,12 @@ __global__ void __launch_bounds__(256) ksg_range_kernel(const double* __restrict
                 lo = fmin(lo, s_lo[w]);
                 hi = fmax(hi, s_hi[w]);
             }
-            const double c = 0.5 * (lo + hi);
+            const double c = 0.5 * (lo + hi), R = fmax(hi - c, c - lo);
             mid[a * 3 + d] = c;
-            s_R            = fmax(s_R, fmax(hi - c, c - lo));
+            // rows may hold anything (gc_ksg_pair): beyond FP32, or with no
+            // midrange, no bound holds, and with an infinite one every query of
+            // the atom's pairs is left to the FP64 routine
+            s_R = R < 1e38 ? fmax(s_R, R) : __longlong_as_double(0x7ff0000000000000LL);
         }
     }
     if (threadIdx.x == 0)
