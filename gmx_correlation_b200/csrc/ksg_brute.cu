@@ -11,8 +11,10 @@
 //
 //   1. histogram of the joint distances (256 buckets of 2^18 float ulps, the
 //      top one holding the largest possible distance): the bucket of the k-th
-//      value.  A bucket with more than kBfRefine values is split by a second
-//      histogram.
+//      value.  Where that lies 8 octaves and more below the top (an atom with a
+//      frame or a stretch of frames far off), the buckets move down and the
+//      frames are counted again.  A bucket with more than kBfRefine values is
+//      split by a further histogram.
 //   2. the values below the bucket are counted and their marginal maxima
 //      taken; the bucket's values, and 2 eps around it, are listed.  The
 //      k-th value by rank, the values within 2 eps of it ordered in FP64 with
@@ -20,8 +22,12 @@
 //   3. marginal distances below each maximum are counted, those within 2 eps
 //      listed and settled in FP64.
 //
-// A query the scheme cannot settle (too many values near a bound, a k-th
-// distance below 1/256 of the range) takes the exact FP64 routine.
+// Where more marginal distances lie within 2 eps than are listed (coordinates
+// stored with few digits: many equal distances), the frames are looked at twice
+// more for them.  With k frames at distance zero (repeated frames) the counts are
+// those of the marginal distances of zero.  A query the scheme cannot settle (too
+// many joint values near a bound, a k-th distance near zero, coordinates FP32 does
+// not hold) takes the exact FP64 routine.
 //
 // The exact FP64 kernel evaluates every distance in about seven FP64 passes
 // (radix selection); measured against it on one B200: 28 pairs of 20,001
@@ -51,9 +57,12 @@ struct BfQuery
     float    inlo, bandhi;   // the band: the bucket and 2 eps around it
     float    lower, upper;   // k-th value -+ 2 eps
     float    top[2];         // marginal maxima over the members
+    int      code;           // float code of the lowest bucket
+    int      open;           // the k-th value lies below it: counted again
     int      below;          // frames below the bucket, the query's own included
     int      nlist, nnear[2];
-    int      state;          // 0: running, 1: left to the FP64 routine, 2: no query
+    int      n[2];           // marginal distances below 2 eps of the maxima, the query's own included
+    int      state;          // 0: running, 1: left to the FP64 routine, 2: no query, 3: k-th distance near zero
 };
 
 // Both sums of two packed FP32 additions (round to nearest, as the single ones).
@@ -199,7 +208,10 @@ __global__ void __launch_bounds__(512) ksg_brute_kernel(const double* __restrict
             q3[q][d]       = make_float2(-u.x, -u.y);
         }
         if (lane == 0)
+        {
             qs[q].state = i0 + q < T ? 0 : 2;
+            qs[q].code  = cbase;
+        }
     }
     const bool whole = chunk >= T;
     // fn(j, q, dx, dy) for every frame and query; every thread of the CTA calls it
@@ -285,26 +297,56 @@ __global__ void __launch_bounds__(512) ksg_brute_kernel(const double* __restrict
         atomicAdd(&hist[q * kBfBins + min(max(b, 0), kBfBins - 1)], 1u);
     });
     __syncwarp();
-    bool split = false; // a bucket of this warp has to be split
-#pragma unroll 1
-    for (int q = 0; q < Q; ++q)
-    {
+    bool split = false, lower = false; // a bucket of this warp has to be split, a query counted again below
+    auto bucket = [&](int q) {
         int bin, below, in;
         find(hist + q * kBfBins, K + 1, bin, below, in); // the query itself is the first, in bucket 0
+        const int  code = qs[q].code;
+        const bool down = qs[q].state == 0 && bin == 0 && code > kBfBins &&
+                          __uint_as_float((unsigned)code << kBfShift) > 32.0f * e2; // buckets wider than 2 eps
+        __syncwarp();
         if (lane == 0)
         {
             BfQuery& u = qs[q];
             u.below    = below;
-            u.lo       = (unsigned)(max(bin, 0) + cbase) << kBfShift;
+            u.lo       = (unsigned)(max(bin, 0) + code) << kBfShift;
             u.hi       = u.lo + (1u << kBfShift);
             u.nlist    = in;
-            if (u.state == 0 && (bin < 1 || cbase < 1))
-                u.state = 1;
+            u.open     = down;
+            if (down)
+                u.code = code - (kBfBins - 1); // the lowest bucket becomes the top one
+            else if (u.state == 0 && (bin < 1 || code < 1))
+                u.state = bin == 0 ? 3 : 1;
         }
-        split |= in > kBfRefine;
-    }
+        lower |= down;
+        split |= !down && in > kBfRefine;
+    };
+#pragma unroll 1
+    for (int q = 0; q < Q; ++q)
+        bucket(q);
     __syncwarp();
-    if (__syncthreads_or(split))
+    const bool more = __syncthreads_or(split || lower);
+    while (more && __syncthreads_or(lower))
+    {
+        clear();
+        int base[Q];
+#pragma unroll
+        for (int q = 0; q < Q; ++q)
+            base[q] = qs[q].code;
+        frames([&](int, int q, float dx, float dy) {
+            const int b = (int)(__float_as_uint(fmaxf(dx, dy)) >> kBfShift) - base[q];
+            if (b < kBfBins)
+                atomicAdd(&hist[q * kBfBins + max(b, 0)], 1u);
+        });
+        __syncwarp();
+        lower = false;
+#pragma unroll 1
+        for (int q = 0; q < Q; ++q)
+            if (qs[q].open)
+                bucket(q);
+        __syncwarp();
+    }
+    if (more && __syncthreads_or(split))
     {
         clear();
         unsigned lo[Q], hi[Q];
@@ -538,6 +580,25 @@ __global__ void __launch_bounds__(512) ksg_brute_kernel(const double* __restrict
         }
     });
     __syncwarp();
+    auto store = [&](int i, int n0, int n1) {
+        const size_t at = (size_t)pl * T + i;
+        if (cnt_y) // wide counts: n_x and n_y in separate planes
+        {
+            cnt[at]   = (uint32_t)n0;
+            cnt_y[at] = (uint32_t)n1;
+        }
+        else
+            cnt[at] = (uint32_t)n0 | ((uint32_t)n1 << 16);
+    };
+    // whether frame j is one of the k nearest of query q, from its joint distance
+    auto member = [&](int q, int j, float v) -> bool {
+        bool is = v < qs[q].lower;
+        if (!is && v <= qs[q].upper) // one of the ordered values: listed as a member
+            for (int e = 0; e < qs[q].nlist && !is; ++e)
+                is = list_j(q, e) == ((unsigned)j | kMember);
+        return is;
+    };
+    unsigned late = 0u; // queries the lists do not settle
 #pragma unroll
     for (int q = 0; q < Q; ++q)
     {
@@ -546,6 +607,11 @@ __global__ void __launch_bounds__(512) ksg_brute_kernel(const double* __restrict
         n[0]    = (int)__reduce_add_sync(kFull, (unsigned)nx[q]);
         n[1]    = (int)__reduce_add_sync(kFull, (unsigned)ny[q]);
         bool ok = qs[q].state == 0 && qs[q].nnear[0] <= kBfNear && qs[q].nnear[1] <= kBfNear;
+        if (lane == 0)
+        {
+            qs[q].n[0] = n[0];
+            qs[q].n[1] = n[1];
+        }
 #pragma unroll
         for (int side = 0; side < 2; ++side)
         {
@@ -560,11 +626,7 @@ __global__ void __launch_bounds__(512) ksg_brute_kernel(const double* __restrict
                     d = dist3r(x, T, x[i], x[T + i], x[2 * T + i], j);
                     float dx, dy;
                     dist32(i, j, dx, dy);
-                    const float v = fmaxf(dx, dy);
-                    is            = v < qs[q].lower;
-                    if (!is && v <= qs[q].upper) // one of the ordered values: listed as a member
-                        for (int e = 0; e < qs[q].nlist && !is; ++e)
-                            is = list_j(q, e) == ((unsigned)j | kMember);
+                    is = member(q, j, fmaxf(dx, dy));
                 }
             }
             const double best = warp_max(is ? d : -1.0);
@@ -573,20 +635,73 @@ __global__ void __launch_bounds__(512) ksg_brute_kernel(const double* __restrict
             // the query's own frame was counted when it lies below the bound
             n[side] += add - ((side == 0 ? lo_x[q] : lo_y[q]) > 0.0f ? 1 : 0);
         }
-        const int state = qs[q].state;
-        if (state != 2 && !ok)
-            exact_query_nxy(X, T, K, a1, a2, i, box, rank_shift, hist, lane, n[0], n[1]);
-        if (state != 2 && lane == 0)
+        if (ok && lane == 0)
+            store(i, n[0], n[1]);
+        late |= (unsigned)(!ok && qs[q].state != 2) << q;
+        __syncwarp();
+    }
+#pragma unroll 1
+    for (; late; late &= late - 1)
+    {
+        const int q = __ffs(late) - 1, i = min(i0 + q, T - 1);
+        int       n[2] = {qs[q].n[0], qs[q].n[1]};
+        bool      ok   = false;
+        if (qs[q].state == 0)
         {
-            const size_t at = (size_t)pl * T + i;
-            if (cnt_y) // wide counts: n_x and n_y in separate planes
+            // more marginal distances near a maximum than are listed, or no
+            // member among them: the maximum, then the count
+            ok = true;
+#pragma unroll 1
+            for (int side = 0; side < 2; ++side)
             {
-                cnt[at]   = (uint32_t)n[0];
-                cnt_y[at] = (uint32_t)n[1];
+                const double* x   = side == 0 ? xa : xb;
+                const float   top = qs[q].top[side], e = side == 0 ? e2a : e2b;
+                const float   lo = __fsub_rd(top, e), hi = __fadd_ru(top, e);
+                double        best = -1.0;
+                int           add  = 0;
+#pragma unroll 1
+                for (int pass = 0; pass < 2; ++pass)
+                {
+                    double m = -1.0;
+                    for (int j = lane; j < T; j += 32)
+                    {
+                        float dx, dy;
+                        dist32(i, j, dx, dy);
+                        const float v = side == 0 ? dx : dy;
+                        if (j == i || !(v >= lo && v <= hi) || (pass == 0 && !member(q, j, fmaxf(dx, dy))))
+                            continue;
+                        const double d = dist3r(x, T, x[i], x[T + i], x[2 * T + i], j);
+                        m              = fmax(m, d);
+                        add += pass != 0 && d <= best;
+                    }
+                    if (pass == 0)
+                        best = warp_max(m);
+                }
+                ok      = ok && best >= 0.0;
+                n[side] += (int)__reduce_add_sync(kFull, (unsigned)add) - (lo > 0.0f ? 1 : 0);
             }
-            else
-                cnt[at] = (uint32_t)n[0] | ((uint32_t)n[1] << 16);
         }
+        else if (qs[q].state == 3)
+        {
+            // distances of zero: with k of the joint ones both maxima are zero
+            int z = 0, zx = 0, zy = 0;
+            for (int j = lane; j < T; j += 32)
+                if (j != i)
+                {
+                    const bool x0 = dist3r(xa, T, xa[i], xa[T + i], xa[2 * T + i], j) == 0.0;
+                    const bool y0 = dist3r(xb, T, xb[i], xb[T + i], xb[2 * T + i], j) == 0.0;
+                    zx += x0;
+                    zy += y0;
+                    z += x0 && y0;
+                }
+            n[0] = (int)__reduce_add_sync(kFull, (unsigned)zx);
+            n[1] = (int)__reduce_add_sync(kFull, (unsigned)zy);
+            ok   = (int)__reduce_add_sync(kFull, (unsigned)z) >= K;
+        }
+        if (!ok)
+            exact_query_nxy(X, T, K, a1, a2, i, box, rank_shift, hist, lane, n[0], n[1]);
+        if (lane == 0)
+            store(i, n[0], n[1]);
         __syncwarp();
     }
 }
