@@ -103,9 +103,14 @@ __global__ void __launch_bounds__(512) copula_kernel(const double* __restrict__ 
         val[t] = v;
         idx[t] = t < T ? t : -1;
     }
-    if (bad)
-        atomicOr(status, kStatNonFinite);
-    __syncthreads();
+    // a value that is not finite is not ranked: the padding (frame -1) would come
+    // before it in the order, and its score has no place
+    if (__syncthreads_or(bad))
+    {
+        if (threadIdx.x == 0)
+            atomicOr(status, kStatNonFinite);
+        return;
+    }
     for (int k = 2; k <= P; k <<= 1)
         for (int j = k >> 1; j > 0; j >>= 1)
         {
