@@ -73,6 +73,26 @@ struct DeviceScope
     }
 };
 
+// cudaMalloc; when memory is short, once more after idle plans and the pool
+// have given up what they hold.
+inline gc_status device_alloc(void** p, size_t bytes)
+{
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation)
+    {
+        cudaGetLastError();
+        gc_release_cache();
+        e = cudaMalloc(p, bytes);
+    }
+    if (e != cudaSuccess)
+    {
+        cudaGetLastError();
+        return fail(e == cudaErrorMemoryAllocation ? GC_ERR_OUT_OF_MEMORY : GC_ERR_CUDA,
+                    std::string("cudaMalloc: ") + cudaGetErrorString(e));
+    }
+    return GC_OK;
+}
+
 template <class T>
 struct DevBuf
 {
@@ -94,14 +114,9 @@ struct DevBuf
         reset();
         if (count == 0)
             count = 1;
-        cudaError_t e = cudaMalloc(&p, count * sizeof(T));
-        if (e != cudaSuccess)
-        {
-            cudaGetLastError();
-            p = nullptr;
-            return fail(e == cudaErrorMemoryAllocation ? GC_ERR_OUT_OF_MEMORY : GC_ERR_CUDA,
-                        std::string("cudaMalloc: ") + cudaGetErrorString(e));
-        }
+        void* q = nullptr;
+        GC_TRY(device_alloc(&q, count * sizeof(T)));
+        p = static_cast<T*>(q);
         n = count;
         return GC_OK;
     }
@@ -149,20 +164,8 @@ struct PoolBuf
         void*        q    = pool_take(want, &got);
         if (!q)
         {
-            got           = want;
-            cudaError_t e = cudaMalloc(&q, got);
-            if (e == cudaErrorMemoryAllocation)
-            {
-                cudaGetLastError();
-                gc_release_cache(); // free what idle plans and the pool hold and try once more
-                e = cudaMalloc(&q, got);
-            }
-            if (e != cudaSuccess)
-            {
-                cudaGetLastError();
-                return fail(e == cudaErrorMemoryAllocation ? GC_ERR_OUT_OF_MEMORY : GC_ERR_CUDA,
-                            std::string("cudaMalloc: ") + cudaGetErrorString(e));
-            }
+            got = want;
+            GC_TRY(device_alloc(&q, got));
         }
         p   = static_cast<T*>(q);
         n   = count;

@@ -128,3 +128,30 @@ def test_shared_memory_limits_do_not_depend_on_the_call(fake):
     varying = fake.lib().fake_varying_limits(names, 4096)
     assert fake.lib().fake_limited() > 10
     assert varying == 0, names.value.decode()
+
+
+@pytest.mark.parametrize("name", CALLS)
+def test_kept_memory_makes_way(fake, name):
+    """A call that fits in device memory runs also when what earlier calls left
+    behind (a kept plan, pooled blocks) fills it: those are given up."""
+    L, call = fake.lib(), CALLS[name]
+
+    def fresh():
+        fake.batch_release()
+        fake.release_cache()
+
+    fresh()
+    L.fake_reset(0)
+    base = L.fake_live()
+    call(fake)
+    need = L.fake_peak() - base
+    fresh()
+    fake.te_matrix(_x(60, 1500), 4, 1)
+    filled = L.fake_live() - base
+    assert filled > need
+    L.fake_limit(base + filled)
+    try:
+        call(fake)
+    finally:
+        L.fake_limit(180 << 30)
+        fresh()
