@@ -42,6 +42,8 @@ struct TeTraj
     TeParams desc(int* status, int b) const;
     // The same with the block's rows at the given addresses.
     TeParams desc_rows(int* status, int b, float* SG_, uint16_t* PG_, float* SM_, uint16_t* PM_) const;
+    // Device memory it holds.
+    size_t bytes() const;
     // Bytes of one block's G and M rows (256-byte aligned parts).
     size_t block_row_bytes() const;
     // Transpose and FP32 copy of device coordinates d_xyz, then the counters

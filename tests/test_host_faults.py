@@ -155,3 +155,16 @@ def test_kept_memory_makes_way(fake, name):
     finally:
         L.fake_limit(180 << 30)
         fresh()
+
+
+def test_a_large_te_plan_is_not_kept_whole(fake):
+    """gc_te_matrix keeps its plan for the next call of the shape, but not one of
+    many GB: its blocks serve the next call, of whatever shape, from the pool."""
+    L = fake.lib()
+    fake.release_cache()
+    fake.te_matrix(_x(247, 2000), 100, 1)
+    first = L.fake_live()
+    assert first > 8 << 30  # the sorted rows alone
+    fake.te_matrix(_x(246, 2000), 100, 1)
+    assert L.fake_live() < 1.2 * first
+    fake.release_cache()
