@@ -8,8 +8,9 @@
 namespace gc {
 
 constexpr int kSumThreads = 256;
-constexpr int kSumTerms   = 2048; // terms of a chunk over all sums of the CTA
+constexpr int kSumTerms   = 1024; // terms of a chunk over all sums of the CTA
 constexpr int kSumMost    = 32;   // most sums per CTA
+static_assert(kSumTerms / kSumMost >= 32, "a warp evaluates 32 consecutive terms of a sum");
 
 // Sums per CTA (a power of two): enough CTAs for every SM before the sums of
 // a CTA grow to 32, the width of the adding warp.
@@ -25,12 +26,15 @@ inline int sums_per_cta(long sums, int sms)
 // term(p, f): seven warps evaluate a chunk of terms, 32 consecutive f at a
 // time (so the counts behind them are read coalesced), into shared memory
 // while the lanes of warp 0 add the previous chunk, each its own sum in order
-// of f.  Lane p of
-// warp 0 returns sum p.
+// of f.  Lane p of warp 0 returns sum p.
 //
-// Bound by the chain of dependent FP64 additions (T of them); a thread that
-// also fetched its own terms spent 80-90 ns per term on dependent loads:
-// 247 x 2000 (30,381 sums of 2000) 294 us, one sum of 2000 86 us.
+// Bound by the chain of dependent FP64 additions (T of them), so a second wave
+// of CTAs doubles it: chunks of 1024 terms (17 KB) let eight CTAs share an SM,
+// 2048 six.  All of a KSG run but its neighbour kernels (normalisation, FP32
+// copy and this), a thread per sum that fetches its own terms / chunks of 2048 /
+// of 1024: 30,381 sums of 2000 terms 361 / 471 / 295 us, 11,325 of 4999 799 /
+// 663 / 712, 2016 of 500 77 / 38 / 39, one of 2000 134 / 69 / 67, 124,750 of 300
+// 138 / 170 / 151.
 template <class Term>
 __device__ __forceinline__ double ordered_sums(int P, int live, int T, Term&& term)
 {
