@@ -657,15 +657,18 @@ __global__ void __launch_bounds__(512) ksg_brute_kernel(const double* __restrict
                 const double* x   = side == 0 ? xa : xb;
                 const float   top = qs[q].top[side], e = side == 0 ? e2a : e2b;
                 const float   lo = __fsub_rd(top, e), hi = __fadd_ru(top, e);
+                // the frames to look at: those listed, or all
+                const int     nl = qs[q].nnear[side], frames_end = nl <= kBfNear ? nl : T;
                 double        best = -1.0;
                 int           add  = 0;
 #pragma unroll 1
                 for (int pass = 0; pass < 2; ++pass)
                 {
                     double m = -1.0;
-                    for (int j = lane; j < T; j += 32)
+                    for (int f = lane; f < frames_end; f += 32)
                     {
-                        float dx, dy;
+                        const int j = nl <= kBfNear ? (int)near[(q * 2 + side) * kBfNear + f] : f;
+                        float     dx, dy;
                         dist32(i, j, dx, dy);
                         const float v = side == 0 ? dx : dy;
                         if (j == i || !(v >= lo && v <= hi) || (pass == 0 && !member(q, j, fmaxf(dx, dy))))
