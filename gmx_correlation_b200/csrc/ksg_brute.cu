@@ -31,7 +31,7 @@
 //
 // The exact FP64 kernel evaluates every distance in about seven FP64 passes
 // (radix selection); measured against it on one B200: 28 pairs of 20,001
-// frames, k = 50: 282 -> 28.6 ms; 1128 pairs of 901 frames, k = 20: 20.0 ->
+// frames, k = 50: 282 -> 27.7 ms; 1128 pairs of 901 frames, k = 20: 20.0 ->
 // 4.0 ms; one pair of 2000 frames, k = 100: 764 -> 42 us.
 
 #include "gc_common.cuh"

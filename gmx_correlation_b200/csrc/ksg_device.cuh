@@ -60,8 +60,7 @@ enum
     kReasonRange    = 2, // k-th value beyond the histogram's two octaves
     kReasonBand     = 3, // band larger than kBandCap or inconsistent with the histogram
     kReasonAmbig    = 4, // ambiguous set inconsistent or larger than kAmbCap
-    kReasonScan     = 5, // scan for the maxima or their counts exceeded kScanCap
-    kReasonPrefix   = 6  // (not raised: the finish looks at whole rows)
+    kReasonScan     = 5  // scan for the maxima or their counts exceeded kScanCap
 };
 
 // Walk result of one (pair, query): bucket of the k-th value, the number of

@@ -297,11 +297,15 @@ __device__ __forceinline__ void walk_query_group(const WalkParams& p, long pl, i
             return (unsigned)min(max((int)(__float_as_uint(v) - Lh) >> shift, 0), (int)kTop);
         return min((__float_as_uint(v) - Lh) >> shift, kTop);
     };
-    // Every 16 entries the indices below the current value are final
-    // (later entries have v >= s), so their running sum R decides the stop
-    // value.  The rows end in NaN up to a 4-entry boundary, which the
-    // take test (s <= stop) never passes, so taken entries form a prefix
-    // of each group and a group short of 4 ends the walk.
+    // Every 16 entries the indices below the current value's are final (a later
+    // entry lies in its fine bucket or a later one, so in its index or a later
+    // one), and their running sum R decides the stop value.  The take test
+    // (s <= stop) passes every entry before stop's fine bucket; within that
+    // bucket entries come in any order, but their v lie beyond the k-th value's
+    // bucket, which ends 2 eps below stop.  A group whose last entry fails it
+    // ends the walk, as the NaN behind the row does: m_end is no count of taken
+    // entries, only not before the start of stop's fine bucket, an upper end for
+    // the finish's search for the k-th value's.
     const float4* Sg = reinterpret_cast<const float4*>(u.rw.S); // 4-entry groups of this lane's row
     const uint2*  Pg = reinterpret_cast<const uint2*>(u.rw.P);
     const size_t  gs = (size_t)p.Qp << p.run;                  // groups from a run to the next

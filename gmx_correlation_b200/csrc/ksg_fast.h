@@ -14,7 +14,8 @@ constexpr int kWalkWarps   = 32;       // most warps per walk CTA
 // what the band entries leave of an SM's 256 KB.  20 warps with 14-byte
 // entries leave about 60 KB: 30.6 ms at 247 x 2000 k=100 and 44.1 at 151 x
 // 4999 (24 such warps leave 28 KB: 43.8 and 68.7 ms); with 10-byte entries 20
-// warps take 29.4 and 41.2 ms, 24 28.1 and 39.4, 25 (72 registers) 27.4 and 38.7.
+// warps take 29.4 and 41.2 ms, 24 28.1 and 39.4, 25 (72 registers, 136 bytes
+// spilled) 27.4 and 38.7; with the rows in runs (row_run) 27.0 and 36.5.
 constexpr int kFinishWarps = GC_FINISH_WARPS;
 constexpr int kWalkBuckets = 128;      // per-lane histogram buckets
 #ifndef GC_BAND_CAP

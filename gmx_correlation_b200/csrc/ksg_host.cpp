@@ -29,9 +29,14 @@ int ksg_block_queries(int natoms, int T, double budget, int quantum, double extr
     return (int)q;
 }
 
-// The row walk holds 32 pairs of one atom in a warp: below 24 atoms most of
-// its lanes are idle; its window index 0 counts up to k - 1 entries in a byte;
-// its tile and a few warps' histograms have to fit in shared memory.
+// The row walk holds 32 pairs of one atom in a warp: with few atoms most of its
+// lanes are idle.  All neighbour kernels with the lane walk / the row walk, us:
+// 500 frames, k = 10: 16 atoms 163 / 169, 24 208 / 212, 28 250 / 239, 40 365 / 345;
+// 2000, k = 100: 16 991 / 1140, 24 1546 / 1607, 28 1930 / 1831, 40 3144 / 2963; TE
+// (the same line): 500: 16 252 / 240, 24 414 / 371; 2000: 16 2484 / 2930, 20 3220 /
+// 3286, 24 4234 / 3971, 40 10030 / 8116.  Its window index 0 counts up to k - 1
+// entries in a byte; its tile and a few warps' histograms have to fit in shared
+// memory.
 static bool row_walk_fits(int natoms, int T, int k)
 {
     int ctas = 0;

@@ -28,13 +28,15 @@ namespace gc {
 // That is all the walks need (their own buckets are whole fine ones); the
 // finish and count kernels look at a value's whole fine bucket.
 //
-// Bound by shared-memory atomics and issue slots.  The full sort it replaces
-// (range, coarse distribution, histogram, scan, scatter and one thread's
-// insertion sort per bucket, over eight barriers) took 10.7 ms for the rows of
-// 247 atoms x 2000 frames, 51.8 ms for 151 x 4999 and 289 us for 64 x 500;
-// this one 6.55 ms, 28.2 ms and 134 us.  Fine buckets of 2^15 ulps make it 2%
-// faster and the finish 3% slower, 2^13 the rows 8% slower; putting the
-// entries of each bucket in order as well costs as much as the full sort.
+// Bound by shared memory (L1 97% busy at 247 x 2000, issue slots 68%): the
+// atomics and the scatter.  The full sort it replaces (range, coarse
+// distribution, histogram, scan, scatter and one thread's insertion sort per
+// bucket, over eight barriers) took 10.7 ms for the rows of 247 atoms x 2000
+// frames, 51.8 ms for 151 x 4999 and 289 us for 64 x 500; this one 6.55 ms, 28.2
+// ms and 134 us written in single groups, 3.93, 16.3 and .099 in the runs that
+// row_run gives.  Fine buckets of 2^15 ulps make it 2% faster and the finish 3%
+// slower, 2^13 the rows 8% slower; putting the entries of each bucket in order as
+// well costs as much as the full sort (all these in single groups).
 
 constexpr int kRowBins  = 4096;
 constexpr int kRowFine  = 14; // log2 of a fine bucket's width in float ulps
@@ -320,7 +322,7 @@ __device__ __forceinline__ float row_top(float eps_atom) { return eps_atom * 419
 // Shared memory of one row of N entries; *threads and *regs pick the sort_row
 // instantiation (threads per row, distances per thread kept in registers).
 // The passes are short, so what counts is how little a barrier holds up:
-// few threads a row, many rows an SM.  64 x 500: 209 us by 256 threads, 169
+// few threads a row, many rows an SM.  In single groups, 64 x 500: 209 us by 256 threads, 169
 // by 256 with 4 distances, 142 by 128, 134 by 64; 247 x 2000: 6.78 ms by 256,
 // 6.55 by 128; 150 x 3000: 11.2 ms by 512, 9.7 by 256; 151 x 4999: 29.8 ms by
 // 512 (two rows an SM), 28.2 (three), 30.3 by 256 with 32 distances.

@@ -65,8 +65,7 @@ enum
 {
     kTeReasonRange  = 2, // k-th value beyond the histogram's range
     kTeReasonBand   = 3, // band larger than kTeBandCap or inconsistent with the histogram
-    kTeReasonAmbig  = 4, // more than kTeAmbCap values within the error bound of the k-th
-    kTeReasonPrefix = 6  // (not raised: the finish looks at whole rows)
+    kTeReasonAmbig  = 4  // more than kTeAmbCap values within the error bound of the k-th
 };
 __device__ __forceinline__ unsigned long long te_pack_walk(int bstar, int prefix, int m_end, int reason)
 {

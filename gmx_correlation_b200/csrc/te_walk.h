@@ -22,8 +22,9 @@ constexpr int kTeBandCap = 24; // band entries kept per lane in the finish kerne
 #ifndef GC_TE_FINISH_WARPS
 #define GC_TE_FINISH_WARPS 28 // a build-time setting for timing other finish CTA shapes
 #endif
-// Warps per TE finish CTA: 24 take 68.3 ms at 247 x 2000 k=100, 28 66.5, 30 67.2;
-// up to 28 the band entries leave L1 the same 124 KB.
+// Warps per TE finish CTA: 24 take 68.3 ms at 247 x 2000 k=100, 28 (72 registers,
+// 60 bytes spilled) 66.5, 30 67.2; up to 28 the band entries leave L1 the same 124
+// KB.  With both rows gathered alike and in runs 28 take 60.4.
 constexpr int kTeFinishWarps = GC_TE_FINISH_WARPS;
 
 // One query block of one trajectory.  Entry m of the G row of (atom a,

@@ -124,7 +124,7 @@ gc_status gc_ksg_matrix_prepared(const double* X, const double* psi, int natoms,
 /* gc_ksg_matrix keeps the device workspace of its last call on each device
  * (a few GB at 247 atoms x 2000 frames) and reuses it when the next call has
  * the same shape (atoms, frames, k, path, pair range); explicit pair lists are
- * not kept.  gc_te_matrix keeps its last plan in the same way.  gc_release_cache
+ * not kept.  gc_te_matrix keeps its last plan of up to 4 GiB in the same way.  gc_release_cache
  * frees every kept workspace and the device blocks kept for later calls. */
 void gc_release_cache(void);
 
