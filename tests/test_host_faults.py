@@ -50,6 +50,11 @@ def _plan(gc, make):
         p.close()
 
 
+def _milca(N, k):
+    from gmx_correlation_b200.milca import milca
+    return milca("mi_xnynK", np.random.default_rng(1).exponential(1.0, (4, N)), k, dimx=2, dimy=2)
+
+
 CALLS = {
     "ksg": lambda gc: gc.kraskov_corrmatrix(_x(5, 60), 4),
     "ksg rows": lambda gc: gc.kraskov_corrmatrix(_x(30, 60), 4),
@@ -68,6 +73,7 @@ CALLS = {
     "te batch": lambda gc: gc.te_batch([_x(5, 60), _x(3, 50)], 4, 1),
     "gcmi batch": lambda gc: gc.gcmi_batch([_x(5, 60), _x(3, 50)]),
     "features": lambda gc: gc.screen_features(_x(4, 60), 4),
+    "milca": lambda gc: _milca(60, 5),
 }
 
 
@@ -119,6 +125,8 @@ def test_shared_memory_limits_do_not_depend_on_the_call(fake):
         fake.kraskov_wrap(np.ones((6, T)), np.ones(T + 1), 1, 0, k)
         if T <= 16384:
             fake.screen_features(x, k)
+    for N, k in ((300, 250), (900, 800)):  # more than the default limit, and more again
+        _milca(N, k)
     for T in (300, 2500, 900):
         fake.ksg_batch([_x(30, T), _x(5, T // 2)], 5)
         fake.te_batch([_x(30, T), _x(5, T // 2)], 5, 1)
