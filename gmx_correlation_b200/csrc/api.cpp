@@ -324,7 +324,7 @@ gc_status gc_ksg_plan_create(int natoms, int nframes, int k, const gc_opts* opts
     if (!p->fast && o.path != GC_PATH_EXACT_FP64)
         GC_TRY(p->brute.alloc(gc::ksg_brute_scratch(natoms) / sizeof(double) + 1));
     const std::vector<double> psi = digamma_table(nframes);
-    GC_TRY_CUDA(cudaMemcpy(p->psi.p, psi.data(), sizeof(double) * psi.size(), cudaMemcpyHostToDevice));
+    GC_TRY_CUDA(upload(p->psi.p, psi.data(), sizeof(double) * psi.size()));
     if (o.pair_list && pc > 0)
     {
         std::vector<int2> ab((size_t)pc);
@@ -335,7 +335,7 @@ gc_status gc_ksg_plan_create(int natoms, int nframes, int k, const gc_opts* opts
             ab[(size_t)q] = make_int2(a1, a2);
         }
         GC_TRY(p->pair_ab.alloc((size_t)pc));
-        GC_TRY_CUDA(cudaMemcpy(p->pair_ab.p, ab.data(), sizeof(int2) * ab.size(), cudaMemcpyHostToDevice));
+        GC_TRY_CUDA(upload(p->pair_ab.p, ab.data(), sizeof(int2) * ab.size()));
     }
     if (p->fast)
     {

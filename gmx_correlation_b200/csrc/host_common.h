@@ -209,6 +209,16 @@ inline gc_status check_view(const gc_traj_view* v)
     return GC_OK;
 }
 
+// Copies a table to the device and waits until it is there.  cudaMemcpy from
+// pageable memory returns once the bytes are staged; the transfer may still be
+// on its way in the legacy stream, for which the library's non-blocking streams
+// do not wait, and a pooled block still holds what its last owner wrote.
+inline cudaError_t upload(void* d, const void* h, size_t bytes)
+{
+    const cudaError_t e = cudaMemcpy(d, h, bytes, cudaMemcpyHostToDevice);
+    return e == cudaSuccess ? cudaStreamSynchronize(cudaStreamLegacy) : e;
+}
+
 // Waits for what is ordered on s, so that device blocks and caller's arrays in
 // use there are free: on the way out of a call that failed in the middle.  A
 // stream under capture has nothing in flight and is left alone.

@@ -279,7 +279,7 @@ gc_status create_plan(const gc_traj_view* trajs, const int* ks, int ntraj, int d
         GC_TRY(b->mi.alloc((size_t)b->pairs));
         GC_TRY(b->cnt.alloc((size_t)b->T * b->pairs));
         const std::vector<double> psi = digamma_table(b->T);
-        GC_TRY_CUDA(cudaMemcpy(b->psi.p, psi.data(), sizeof(double) * psi.size(), cudaMemcpyHostToDevice));
+        GC_TRY_CUDA(upload(b->psi.p, psi.data(), sizeof(double) * psi.size()));
         bp->key.insert(bp->key.end(), {b->natoms, b->T, b->K});
         bp->t.push_back(std::move(b));
     }

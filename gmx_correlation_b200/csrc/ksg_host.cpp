@@ -119,7 +119,7 @@ gc_status KsgTraj::set_pair_tile(int tile)
         order[(size_t)q] = (int)(key[(size_t)q] & 0xFFFFFFFFll);
     if (!pair_order.p)
         GC_TRY(pair_order.alloc((size_t)pair_count));
-    GC_TRY_CUDA(cudaMemcpy(pair_order.p, order.data(), sizeof(int) * order.size(), cudaMemcpyHostToDevice));
+    GC_TRY_CUDA(upload(pair_order.p, order.data(), sizeof(int) * order.size()));
     pair_tile = tile;
     return GC_OK;
 }
@@ -234,8 +234,8 @@ gc_status KsgLaunch::build(const std::vector<std::vector<WalkParams>>& wave_desc
     GC_TRY(descs.alloc(all.size()));
     GC_TRY(prefix.alloc(pre.size()));
     GC_TRY(counters.alloc(2 * wave_descs.size() + 1));
-    GC_TRY_CUDA(cudaMemcpy(descs.p, all.data(), sizeof(WalkParams) * all.size(), cudaMemcpyHostToDevice));
-    GC_TRY_CUDA(cudaMemcpy(prefix.p, pre.data(), sizeof(long long) * pre.size(), cudaMemcpyHostToDevice));
+    GC_TRY_CUDA(upload(descs.p, all.data(), sizeof(WalkParams) * all.size()));
+    GC_TRY_CUDA(upload(prefix.p, pre.data(), sizeof(long long) * pre.size()));
     waves.clear();
     wave_rows.clear();
     wave_queries.clear();

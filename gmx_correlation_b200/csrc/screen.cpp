@@ -357,7 +357,7 @@ gc_status gc_screen_model_create(int members, uint64_t seed, int device, gc_scre
             for (long i = 0; i < sg.count; ++i)
                 h[(size_t)z * gc::kMlpStride + sg.off + i] = u(rng);
         }
-    cudaError_t e = cudaMemcpy(m->params.p, h.data(), n * sizeof(float), cudaMemcpyHostToDevice);
+    cudaError_t e = upload(m->params.p, h.data(), n * sizeof(float));
     if (e == cudaSuccess)
         e = cudaMemset(m->grad.p, 0, n * sizeof(float));
     if (e == cudaSuccess)
@@ -403,7 +403,7 @@ gc_status gc_screen_model_set_params(gc_screen_model* m, const float* params)
     DeviceScope dev(m->device);
     GC_TRY(dev.st);
     const size_t n = (size_t)m->members * gc::kMlpStride;
-    GC_TRY_CUDA(cudaMemcpy(m->params.p, params, sizeof(float) * n, cudaMemcpyHostToDevice));
+    GC_TRY_CUDA(upload(m->params.p, params, sizeof(float) * n));
     GC_TRY_CUDA(cudaMemset(m->adam_m.p, 0, sizeof(float) * n));
     GC_TRY_CUDA(cudaMemset(m->adam_v.p, 0, sizeof(float) * n));
     GC_TRY_CUDA(cudaMemset(m->counters.p, 0, 2 * sizeof(int)));
@@ -421,10 +421,10 @@ gc_status gc_screen_model_set_input(gc_screen_model* m, const float* feat_mean, 
             return fail(GC_ERR_INVALID, "feature standard deviations must be finite and positive");
     DeviceScope dev(m->device);
     GC_TRY(dev.st);
-    GC_TRY_CUDA(cudaMemcpy(m->feat_mean.p, feat_mean, sizeof(float) * gc::kScreenIn, cudaMemcpyHostToDevice));
-    GC_TRY_CUDA(cudaMemcpy(m->feat_sd.p, feat_sd, sizeof(float) * gc::kScreenIn, cudaMemcpyHostToDevice));
-    GC_TRY_CUDA(cudaMemcpy(m->pca.p, pca_mean, sizeof(float) * 64, cudaMemcpyHostToDevice));
-    GC_TRY_CUDA(cudaMemcpy(m->pca.p + 64, pca_comp, sizeof(float) * 64 * gc::kScreenComp, cudaMemcpyHostToDevice));
+    GC_TRY_CUDA(upload(m->feat_mean.p, feat_mean, sizeof(float) * gc::kScreenIn));
+    GC_TRY_CUDA(upload(m->feat_sd.p, feat_sd, sizeof(float) * gc::kScreenIn));
+    GC_TRY_CUDA(upload(m->pca.p, pca_mean, sizeof(float) * 64));
+    GC_TRY_CUDA(upload(m->pca.p + 64, pca_comp, sizeof(float) * 64 * gc::kScreenComp));
     m->has_input = true;
     return GC_OK;
 }

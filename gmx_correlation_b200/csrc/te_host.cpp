@@ -81,7 +81,7 @@ gc_status TeTraj::create(int n, int nframes, int k, int lg, int q, bool own_rows
     GC_TRY(eps.alloc((size_t)n));
     GC_TRY(cnt.alloc((size_t)Nv * npairs));
     const std::vector<double> tab = digamma_table(Nv + 1);
-    GC_TRY_CUDA(cudaMemcpy(psi.p, tab.data(), sizeof(double) * tab.size(), cudaMemcpyHostToDevice));
+    GC_TRY_CUDA(upload(psi.p, tab.data(), sizeof(double) * tab.size()));
     Q = q;
     if (Q <= 0)
         return GC_OK;
@@ -111,7 +111,7 @@ gc_status TeTraj::create(int n, int nframes, int k, int lg, int q, bool own_rows
     GC_TRY(reasons.alloc(8));
     const std::vector<int> order = te_tile_order(n);
     GC_TRY(pair_order.alloc(order.size()));
-    GC_TRY_CUDA(cudaMemcpy(pair_order.p, order.data(), sizeof(int) * order.size(), cudaMemcpyHostToDevice));
+    GC_TRY_CUDA(upload(pair_order.p, order.data(), sizeof(int) * order.size()));
     return GC_OK;
 }
 
@@ -236,8 +236,8 @@ gc_status TeLaunch::build(const std::vector<std::vector<TeParams>>& wave_descs, 
     GC_TRY(descs.alloc(all.size()));
     GC_TRY(prefix.alloc(pre.size()));
     GC_TRY(counters.alloc(2 * wave_descs.size() + 1));
-    GC_TRY_CUDA(cudaMemcpy(descs.p, all.data(), sizeof(TeParams) * all.size(), cudaMemcpyHostToDevice));
-    GC_TRY_CUDA(cudaMemcpy(prefix.p, pre.data(), sizeof(long long) * pre.size(), cudaMemcpyHostToDevice));
+    GC_TRY_CUDA(upload(descs.p, all.data(), sizeof(TeParams) * all.size()));
+    GC_TRY_CUDA(upload(prefix.p, pre.data(), sizeof(long long) * pre.size()));
     waves.clear();
     wave_rows.clear();
     wave_queries.clear();

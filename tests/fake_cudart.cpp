@@ -1,7 +1,8 @@
 // A CUDA runtime without a GPU, for tests of the library's host code: linked
 // with the library's own objects in place of the CUDA runtime.  Device memory
 // is host memory, kernels do nothing, streams only count what was ordered on
-// them.  It keeps what the tests ask for: work pending on a stream, bytes
+// them.  It keeps what the tests ask for: work pending on a stream, kernels
+// launched while an upload of the legacy stream may be on its way, bytes
 // allocated, the dynamic shared memory limit of every kernel, and it can fail
 // the n-th call that may fail.
 #include <cuda_runtime_api.h>
@@ -41,6 +42,7 @@ std::map<const void*, std::set<int>> g_limits; // every dynamic shared memory li
 std::map<const void*, int>         g_limit_now;
 long                               g_calls = 0, g_fail_at = 0;
 int                                g_bad = 0; // streams destroyed with work pending
+int                                g_early = 0; // launches while an upload may be on its way
 cudaError_t                        g_last = cudaSuccess;
 
 using Lock = std::lock_guard<std::recursive_mutex>;
@@ -55,11 +57,22 @@ cudaError_t err(cudaError_t e)
 // Counts a call that may fail; true when this one is to.
 bool fails() { return ++g_calls == g_fail_at; }
 
+CUstream_st& stream_of(cudaStream_t s) { return s && s != cudaStreamLegacy ? *s : g_legacy; }
+
 void order(cudaStream_t s)
 {
-    CUstream_st& st = s ? *s : g_legacy;
+    CUstream_st& st = stream_of(s);
     if (!st.capturing)
         ++st.ordered;
+}
+
+// A kernel or graph launch: the library's streams do not wait for the legacy one.
+void launch(cudaStream_t s)
+{
+    CUstream_st& st = stream_of(s);
+    if (&st != &g_legacy && !st.capturing)
+        g_early += g_legacy.ordered > g_legacy.done;
+    order(s);
 }
 
 struct Config
@@ -81,6 +94,7 @@ void fake_reset(long fail_at)
     g_calls   = 0;
     g_fail_at = fail_at;
     g_bad     = 0;
+    g_early   = 0;
     g_peak    = g_live;
     g_last    = cudaSuccess;
 }
@@ -98,6 +112,7 @@ int fake_pending()
     return n;
 }
 int    fake_bad() { return g_bad; }
+int    fake_early() { return g_early; }
 size_t fake_live() { return g_live; }
 size_t fake_peak() { return g_peak; }
 void   fake_limit(size_t bytes) { g_limit = bytes; }
@@ -177,6 +192,7 @@ cudaError_t cudaFree(void* p)
     Lock l(g_mutex);
     for (cudaStream_t s : g_streams) // waits for the device
         s->done = s->ordered;
+    g_legacy.done = g_legacy.ordered;
     auto it = g_blocks.find((char*)p);
     if (it == g_blocks.end())
         return p ? err(cudaErrorInvalidValue) : cudaSuccess;
@@ -196,12 +212,15 @@ cudaError_t cudaGetSymbolAddress(void** p, const void* symbol)
     *p = const_cast<void*>(symbol);
     return cudaSuccess;
 }
-cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind)
+cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind kind)
 {
     Lock l(g_mutex);
     if (fails())
         return err(cudaErrorUnknown);
     std::memcpy(d, s, n);
+    g_legacy.done = g_legacy.ordered; // the stream is synchronised before the copy
+    if (kind == cudaMemcpyHostToDevice)
+        ++g_legacy.ordered; // from pageable memory: on its way when the call returns
     return cudaSuccess;
 }
 cudaError_t cudaMemcpy2D(void* d, size_t dp, const void* s, size_t sp, size_t w, size_t h, cudaMemcpyKind)
@@ -253,7 +272,7 @@ cudaError_t cudaStreamDestroy(cudaStream_t s)
 cudaError_t cudaStreamSynchronize(cudaStream_t s)
 {
     Lock         l(g_mutex);
-    CUstream_st& st = s ? *s : g_legacy;
+    CUstream_st& st = stream_of(s);
     if (st.capturing)
         return err(cudaErrorStreamCaptureUnsupported);
     st.done = st.ordered;
@@ -290,7 +309,7 @@ cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t s)
     Lock l(g_mutex);
     if (fails())
         return err(cudaErrorUnknown);
-    order(s);
+    launch(s);
     return cudaSuccess;
 }
 cudaError_t cudaEventCreate(cudaEvent_t* e)
@@ -352,7 +371,7 @@ cudaError_t cudaLaunchKernel(const void* f, dim3 g, dim3 b, void**, size_t smem,
     const int limit = it == g_limit_now.end() ? 48 * 1024 : it->second;
     if (fails() || g.x == 0 || g.y == 0 || b.x == 0 || b.x > 1024 || smem > (size_t)limit)
         return err(cudaErrorInvalidValue);
-    order(s);
+    launch(s);
     return cudaSuccess;
 }
 unsigned __cudaPushCallConfiguration(dim3 g, dim3 b, size_t smem, struct CUstream_st* s)

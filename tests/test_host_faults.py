@@ -112,6 +112,25 @@ def test_failed_call_leaves_no_work_pending(fake, name, kept):
     fake.release_cache()
 
 
+def _screened(gc):
+    from gmx_correlation_b200.screen import TrainedScreen
+    m = TrainedScreen.load().model
+    gc.ksg_screened(_x(12, 80), 4, m, sigma_max=float("inf"), margin=0.0)
+
+
+@pytest.mark.parametrize("name", [*CALLS, "screened"])
+def test_no_kernel_before_its_tables_are_there(fake, name):
+    """Uploads by cudaMemcpy from pageable memory may still be on their way in the
+    legacy stream when it returns; the library's own streams do not wait for it."""
+    call = CALLS.get(name, _screened)
+    for _ in range(2):  # a new plan, a kept one
+        fake.lib().fake_reset(0)
+        call(fake)
+        assert fake.lib().fake_early() == 0
+    fake.batch_release()
+    fake.release_cache()
+
+
 def test_shared_memory_limits_do_not_depend_on_the_call(fake):
     """A kernel's dynamic shared memory limit belongs to the function on its
     device: a value of one call's own could lower it between another thread's
