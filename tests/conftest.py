@@ -1,4 +1,5 @@
 """Shared fixtures.  `-m "not gpu"` runs everywhere; `-m gpu` needs a B200."""
+import inspect
 import sys
 from pathlib import Path
 
@@ -13,6 +14,15 @@ sys.path.insert(0, str(ROOT))
 def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs an NVIDIA B200 (sm_100a) and the built CUDA library")
     config.addinivalue_line("markers", "slow: long-running case")
+
+
+def pytest_collection_modifyitems(items):
+    """Where the reference's own library is not built, the GPU tests that need it
+    come last: a run that ends at the first failure has then run the others."""
+    from oracle import REF_SO
+    if not REF_SO.exists():
+        items.sort(key=lambda it: it.get_closest_marker("gpu") is not None
+                   and ("ref" in it.fixturenames or "Reference()" in inspect.getsource(it.function)))
 
 
 @pytest.fixture(scope="session")
